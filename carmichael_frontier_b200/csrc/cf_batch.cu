@@ -512,20 +512,21 @@ __global__ void __launch_bounds__(128)
 k_batch_check(const CfBatchMod* __restrict__ mods, const CfPair* __restrict__ pairs, const u32* __restrict__ pmod,
               const u32* __restrict__ npairs, u32 max_pairs, CfPairResult* __restrict__ res) {
   const u32 np = min(*npairs, max_pairs);
-  for (u32 t = blockIdx.x * blockDim.x + threadIdx.x; t < np; t += gridDim.x * blockDim.x) {
+  const int lane = threadIdx.x & 31;
+  for (u32 t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < np; t += (gridDim.x * blockDim.x) >> 5) {
     const CfBatchMod& md = mods[pmod[t]];
     CfPairResult o;
     switch (md.r) {
-      case 1: o = cf_check_one<1>(md.poolD, md.poolI, md.screen, pairs[t]); break;
-      case 2: o = cf_check_one<2>(md.poolD, md.poolI, md.screen, pairs[t]); break;
-      case 3: o = cf_check_one<3>(md.poolD, md.poolI, md.screen, pairs[t]); break;
-      case 4: o = cf_check_one<4>(md.poolD, md.poolI, md.screen, pairs[t]); break;
-      case 5: o = cf_check_one<5>(md.poolD, md.poolI, md.screen, pairs[t]); break;
-      case 6: o = cf_check_one<6>(md.poolD, md.poolI, md.screen, pairs[t]); break;
-      case 7: o = cf_check_one<7>(md.poolD, md.poolI, md.screen, pairs[t]); break;
-      default: o = cf_check_one<8>(md.poolD, md.poolI, md.screen, pairs[t]); break;
+      case 1: o = cf_check_warp<1>(md.poolD, md.poolI, md.screen, pairs[t], lane); break;
+      case 2: o = cf_check_warp<2>(md.poolD, md.poolI, md.screen, pairs[t], lane); break;
+      case 3: o = cf_check_warp<3>(md.poolD, md.poolI, md.screen, pairs[t], lane); break;
+      case 4: o = cf_check_warp<4>(md.poolD, md.poolI, md.screen, pairs[t], lane); break;
+      case 5: o = cf_check_warp<5>(md.poolD, md.poolI, md.screen, pairs[t], lane); break;
+      case 6: o = cf_check_warp<6>(md.poolD, md.poolI, md.screen, pairs[t], lane); break;
+      case 7: o = cf_check_warp<7>(md.poolD, md.poolI, md.screen, pairs[t], lane); break;
+      default: o = cf_check_warp<8>(md.poolD, md.poolI, md.screen, pairs[t], lane); break;
     }
-    res[t] = o;
+    if (lane == 0) res[t] = o;
   }
 }
 
@@ -561,8 +562,8 @@ extern "C" int cf_batch_run(int mode, const void* mods, const u64* tstart, u32 n
   const cudaStream_t st = (cudaStream_t)stream;
   if (mode == 2) {
     if (max_pairs == 0) return CF_OK;
-    const u32 g = (max_pairs + 127) / 128;
-    k_batch_check<<<g < 1024u ? g : 1024u, 128, 0, st>>>((const CfBatchMod*)mods, (const CfPair*)pairs, pmod, npairs,
+    const u32 g = (max_pairs + 3) / 4;
+    k_batch_check<<<g < 148u * 8u ? g : 148u * 8u, 128, 0, st>>>((const CfBatchMod*)mods, (const CfPair*)pairs, pmod, npairs,
                                                           max_pairs, (CfPairResult*)results);
     CF_LAUNCH_CHECK("cf_batch_run(check)");
     return CF_OK;

@@ -20,15 +20,18 @@ k_check_pairs(const u64* __restrict__ poolD, const u64* __restrict__ poolI, cons
               CfPairResult* __restrict__ res, u32* __restrict__ err) {
   (void)err;
   const u32 np = min(*npairs, max_pairs);
-  for (u32 t = blockIdx.x * blockDim.x + threadIdx.x; t < np; t += gridDim.x * blockDim.x)
-    res[t] = cf_check_one<R>(poolD, poolI, scr, pairs[t]);
+  const int lane = threadIdx.x & 31;
+  for (u32 t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < np; t += (gridDim.x * blockDim.x) >> 5) {
+    const CfPairResult o = cf_check_warp<R>(poolD, poolI, scr, pairs[t], lane);
+    if (lane == 0) res[t] = o;
+  }
 }
 
 template <int R>
 void launch_check(const u64* poolD, const u64* poolI, const CfScreen* scr, const CfPair* pairs, const u32* npairs,
                   u32 max_pairs, CfPairResult* res, u32* err, cudaStream_t st) {
-  const u32 grid = max_pairs ? (u32)((max_pairs + 127) / 128) : 1u;
-  k_check_pairs<R><<<grid < 1024u ? grid : 1024u, 128, 0, st>>>(poolD, poolI, scr, pairs, npairs, max_pairs, res,
+  const u32 grid = max_pairs ? (u32)((max_pairs + 3) / 4) : 1u;
+  k_check_pairs<R><<<grid < 148u * 8u ? grid : 148u * 8u, 128, 0, st>>>(poolD, poolI, scr, pairs, npairs, max_pairs, res,
                                                                 err);
 }
 

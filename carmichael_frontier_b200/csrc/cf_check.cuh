@@ -1,13 +1,59 @@
 // cf_check.cuh -- exact check of one candidate (D, I) pair of one modulus
-// (shared by the single-modulus and the batched pair-check kernels).
+// (shared by the single-modulus and the batched pair-check kernels), one warp per pair.
+//
+// A pair that passes the size screen costs (n + R)^2 modular products (Korselt) and a 2048-bit
+// product of n + R primes; on one thread that is 20 us at 64 primes and 5 ms of a join whose bound
+// lets many pairs through (k = 90, r = 5).  Over a warp the Korselt moduli go to the lanes, and the
+// product keeps two 32-bit limbs per lane with the carries one step behind (a carry out of a lane is
+// added to the next lane's limb before the next factor multiplies it), so a factor is one shuffle.
 #pragma once
 #include "cf_abi_internal.h"
 #include "cf_enum.cuh"
 
-// Check one candidate pair (lexicographic ranks) of one modulus.
+// Limbs 2 * lane and 2 * lane + 1 of a number below 2^2048, with a carry pending on each.
+struct CfWarpBig {
+  u32 l0, l1, c0, c1;
+  bool over;               // lane 31: something carried out of the top
+};
+__device__ __forceinline__ void cf_big_settle(CfWarpBig& b, int lane) {
+  while (__any_sync(0xffffffffu, (b.c0 | b.c1) != 0u)) {
+    const u64 s0 = (u64)b.l0 + b.c0;
+    const u64 s1 = (u64)b.l1 + b.c1 + (s0 >> 32);
+    b.l0 = (u32)s0;
+    b.l1 = (u32)s1;
+    const u32 out = (u32)(s1 >> 32);
+    const u32 in = __shfl_up_sync(0xffffffffu, out, 1);
+    b.over |= lane == 31 && out != 0u;
+    b.c0 = lane ? in : 0u;
+    b.c1 = 0u;
+  }
+}
+__device__ __forceinline__ void cf_big_mul(CfWarpBig& b, u32 q, int lane) {
+  if (q >> 31) cf_big_settle(b, lane);            // (limb + carry) * q stays below 2^64 for q < 2^31
+  const u64 t0 = ((u64)b.l0 + b.c0) * q, t1 = ((u64)b.l1 + b.c1) * q;
+  const u32 out = (u32)(t1 >> 32);
+  const u32 in = __shfl_up_sync(0xffffffffu, out, 1);
+  b.over |= lane == 31 && out != 0u;
+  b.l0 = (u32)t0;
+  b.l1 = (u32)t1;
+  b.c0 = lane ? in : 0u;
+  b.c1 = (u32)(t0 >> 32);
+}
+
+// x-th prime of S = (B0 without the primes at di) and the primes at ii, x < nD; false: deleted.
 template <int R>
-__device__ __forceinline__ CfPairResult cf_check_one(const u64* __restrict__ poolD, const u64* __restrict__ poolI,
-                                     const CfScreen* __restrict__ scr, CfPair pr) {
+__device__ __forceinline__ bool cf_in_base(const int (&di)[R], int x) {
+  bool in = true;
+#pragma unroll
+  for (int j = 0; j < R; ++j) in &= di[j] != x;
+  return in;
+}
+
+// Check one candidate pair (lexicographic ranks) of one modulus; the whole warp calls it with the
+// same pair and every lane gets the result.
+template <int R>
+__device__ __forceinline__ CfPairResult cf_check_warp(const u64* __restrict__ poolD, const u64* __restrict__ poolI,
+                                     const CfScreen* __restrict__ scr, CfPair pr, int lane) {
   const CfPoolHdr* hD = (const CfPoolHdr*)poolD;
   const CfPoolHdr* hI = (const CfPoolHdr*)poolI;
   const int nD = (int)hD->n, nI = (int)hI->n;
@@ -62,70 +108,48 @@ __device__ __forceinline__ CfPairResult cf_check_one(const u64* __restrict__ poo
     bool distinct = true;
     for (int j = 0; j < R; ++j) {
       const u64 q = pI[ii[j]];
-      for (int x = 0; x < nD; ++x) distinct &= (pD[x] != q);
+      for (int x = lane; x < nD; x += 32) distinct &= (pD[x] != q);
       for (int y = 0; y < j; ++y) distinct &= (pI[ii[y]] != q);
     }
-    if (distinct) out.flags |= CF_HIT_DISJOINT;
+    if (__all_sync(0xffffffffu, distinct)) out.flags |= CF_HIT_DISJOINT;
     // --- exact size: n = prod(S) in 32-bit limbs against B
-    u32 limb[CF_SCREEN_MAX_LIMBS];
-    const int L = CF_SCREEN_MAX_LIMBS;
-    for (int l = 0; l < L; ++l) limb[l] = 0;
-    limb[0] = 1;
-    bool over = false;
-    int dpos = 0;
+    CfWarpBig n;
+    n.l0 = lane == 0 ? 1u : 0u;
+    n.l1 = n.c0 = n.c1 = 0u;
+    n.over = false;
     for (int x = 0; x < nD + R; ++x) {
-      u64 q;
-      if (x < nD) {
-        if (dpos < R && di[dpos] == x) { ++dpos; continue; }
-        q = pD[x];
-      } else {
-        q = pI[ii[x - nD]];
-      }
-      if (q >> 32) { over = true; continue; }
-      u64 carry = 0;
-      for (int l = 0; l < L; ++l) {
-        const u64 v = (u64)limb[l] * q + carry;
-        limb[l] = (u32)v;
-        carry = v >> 32;
-      }
-      if (carry) over = true;
+      if (x < nD && !cf_in_base<R>(di, x)) continue;
+      const u64 q = x < nD ? pD[x] : pI[ii[x - nD]];
+      if (q >> 32) { n.over = true; continue; }
+      cf_big_mul(n, (u32)q, lane);
     }
-    if (!over) {
-      int cmp = 0;   // -1 n<B, 0 equal, 1 n>B
-      for (int l = L - 1; l >= 0 && cmp == 0; --l) {
-        const u32 b = (l < (int)scr->nlimbs) ? scr->limbsB[l] : 0u;
-        if (limb[l] != b) cmp = (limb[l] < b) ? -1 : 1;
-      }
-      if (cmp <= 0) out.flags |= CF_HIT_SIZE_EXACT;
+    cf_big_settle(n, lane);
+    if (!__any_sync(0xffffffffu, n.over)) {
+      const u32 b0 = 2 * lane < (int)scr->nlimbs ? scr->limbsB[2 * lane] : 0u;
+      const u32 b1 = 2 * lane + 1 < (int)scr->nlimbs ? scr->limbsB[2 * lane + 1] : 0u;
+      const u64 v = ((u64)n.l1 << 32) | n.l0, w = ((u64)b1 << 32) | b0;
+      const u32 gt = __ballot_sync(0xffffffffu, v > w), lt = __ballot_sync(0xffffffffu, v < w);
+      if (gt <= lt) out.flags |= CF_HIT_SIZE_EXACT;   // the highest differing limbs decide
     }
-    // --- Korselt: prod(S) == 1 mod (p-1) for every p in S
+    // --- Korselt: prod(S) == 1 mod (p-1) for every p in S, a prime per lane
     bool korselt = true;
-    int dp1 = 0;
-    for (int x = 0; x < nD + R && korselt; ++x) {
-      u64 p;
-      if (x < nD) {
-        if (dp1 < R && di[dp1] == x) { ++dp1; continue; }
-        p = pD[x];
-      } else {
-        p = pI[ii[x - nD]];
-      }
-      const u64 mod = p - 1;
-      if (mod == 0) { korselt = false; break; }
+    for (int x0 = 0; x0 < nD + R; x0 += 32) {
+      const int x = x0 + lane;
+      const bool mine = x < nD + R && (x >= nD || cf_in_base<R>(di, x));
+      const u64 mod = mine ? (x < nD ? pD[x] : pI[ii[x - nD]]) - 1 : 1;
+      if (mod == 0) korselt = false;
+      if (!__all_sync(0xffffffffu, korselt)) break;
       u64 prod = 1 % mod;
-      int dq = 0;
       for (int y = 0; y < nD + R; ++y) {
-        u64 q;
-        if (y < nD) {
-          if (dq < R && di[dq] == y) { ++dq; continue; }
-          q = pD[y];
-        } else {
-          q = pI[ii[y - nD]];
-        }
-        prod = (u64)(((unsigned __int128)prod * (q % mod)) % mod);
+        if (y < nD && !cf_in_base<R>(di, y)) continue;
+        const u64 q = y < nD ? pD[y] : pI[ii[y - nD]];
+        prod = ((mod | q) >> 32) == 0 ? prod * ((u32)q % (u32)mod) % mod
+                                      : (u64)(((unsigned __int128)prod * (q % mod)) % mod);
       }
-      korselt = (prod == 1 % mod);
+      korselt = prod == 1 % mod;
+      if (!__all_sync(0xffffffffu, korselt)) break;
     }
-    if (korselt) out.flags |= CF_HIT_KORSELT;
+    if (__all_sync(0xffffffffu, korselt)) out.flags |= CF_HIT_KORSELT;
   }
   return out;
 }
