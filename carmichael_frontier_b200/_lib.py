@@ -77,6 +77,9 @@ SIGNATURES = [
     ("cf_fused_probe3", C.c_int, [vp, vp, C.c_int, C.c_int, u64, u64, vp, C.c_int, C.c_int, C.c_int, u64, C.c_int,
                                   vp, u32, vp, vp, u32, vp]),
     ("cf_fused_probe", C.c_int, [vp, vp, C.c_int, C.c_int, u64, u64, vp, C.c_int, u64, vp, u32, vp, vp, u32, vp]),
+    ("cf_class_plan_bytes", sz, []),
+    ("cf_class_plan", C.c_int, [u64, C.c_int, C.c_int, C.c_int, u64, u64, C.c_int, vp, sz]),
+    ("cf_class_join", C.c_int, [vp, vp, vp, u32, u32, vp, sz, vp, u32, vp, vp, vp, vp]),
     ("cf_pair_result_bytes", sz, []),
     ("cf_check_pairs", C.c_int, [vp, vp, vp, C.c_int, vp, vp, u32, vp, vp, vp]),
     ("cf_scan_tmp_bytes", sz, [u64]),

@@ -200,6 +200,24 @@ int cf_fused_probe(const void* pool_dev, const void* tail, int n, int r, uint64_
                    const void* tab, int bbits, uint64_t d_rank0, void* pairs, uint32_t max_pairs,
                    uint32_t* npairs, uint32_t* err, uint32_t grid, void* stream);
 
+/* Class join (csrc/cf_class.cu): the same pair set as cf_dtab_build + cf_fused_probe, one residue
+ * class modulo a small divisor of the odd part m of M at a time, each class's filter in shared
+ * memory.  cf_class_plan (host only) fills a plan of cf_class_plan_bytes() bytes for the D side
+ * C(nD, r) against the I ranks [i_lo, i_lo + i_n) (swap: the I window is the smaller side); its
+ * first fields are {u64 magic; u32 ok, d, mp, phi; u64 ws_bytes}, and ok = 0 means that the class
+ * join does not apply to this instance (join it with the fused probe).  cf_class_join runs it:
+ * poolD / poolI are device pool tables (D with a multiplier whose residues mod plan.mp and plan.d
+ * are multD_m and multD_d, I with multiplier 1), ws is plan.ws_bytes of 256-byte aligned device
+ * memory, pairs / npairs / err as for cf_fused_probe; CF_ERR_PART_OVERFLOW in *err: a survivor
+ * list ran out, join the instance with the fused probe instead.  ev_built: null, or a CUDA event
+ * recorded between the filter build and the probe. */
+size_t cf_class_plan_bytes(void);
+int cf_class_plan(uint64_t m, int nD, int nI, int r, uint64_t i_lo, uint64_t i_n, int swap, void* plan,
+                  size_t plan_bytes);
+int cf_class_join(const void* plan, const void* poolD, const void* poolI, uint32_t multD_m, uint32_t multD_d,
+                  void* ws, size_t ws_bytes, void* pairs, uint32_t max_pairs, uint32_t* npairs, uint32_t* err,
+                  void* ev_built, void* stream);
+
 /* Exact check of candidate pairs (lexicographic-rank ids): recomputed residues,
  * conservative fp64 log-size screen, exact size n <= B, Korselt, distinctness.
  * results[t] (cf_pair_result_bytes() each) for t < min(*npairs, max_pairs).
