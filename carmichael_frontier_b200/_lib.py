@@ -109,6 +109,8 @@ SIGNATURES = [
     ("cf_sort_pairs", C.c_int, [vp, vp, u64, C.c_int, vp, sz, vp]),
     ("cf_sort_digits_tmp_bytes", sz, [u64, C.c_int, C.c_int]),
     ("cf_sort_pairs_digits", C.c_int, [vp, vp, u64, C.c_int, C.c_int, vp, sz, vp]),
+    ("cf_sort_to_tmp_bytes", sz, [u64]),
+    ("cf_sort_pairs_to", C.c_int, [vp, vp, vp, vp, u64, C.c_int, vp, sz, vp]),
     ("cf_sort_pairs_noalloc_max", u64, []),
     ("cf_sort_pairs_noalloc", C.c_int, [vp, vp, u64, C.c_int, vp]),
     ("cf_join_tmp_bytes", sz, [u64]),

@@ -19,6 +19,7 @@
 // every I row with at least one equal D key is appended as (row, first D
 // position, count) to a compact run list (pairs are rare).  The host expands
 // runs into pairs in I-row order, which is join_sorted's output order.
+#include <string.h>
 #include <type_traits>
 #include <vector>
 #include "cf_abi_internal.h"
@@ -179,10 +180,11 @@ struct PassLayout {
 // the start (every pointer 16-byte aligned), so the id load overlaps the ranking;
 // otherwise by plain coalesced loads.  Each item's digit (DB + 1 bits, R = no
 // item) rides in the top bits of its local offset.
-template <int DB, bool BULK, typename SW>
+// MSD: the digit is taken from the scaled key mulhi(key, *scale) instead of the key.
+template <int DB, bool BULK, typename SW, bool MSD>
 __global__ void __launch_bounds__(kSortBlock, 2)
 k_sort_pass(const u64* __restrict__ kin, const u64* __restrict__ iin, u64* __restrict__ kout,
-            u64* __restrict__ iout, u64 n, int shift, const u64* __restrict__ gexcl /*[R]*/,
+            u64* __restrict__ iout, u64 n, int shift, const u64* __restrict__ scale, const u64* __restrict__ gexcl /*[R]*/,
             SW* __restrict__ status /*[tiles][R]*/, u32* __restrict__ ticket, u32* __restrict__ err) {
   using St = Status<SW>;
   using L = PassLayout<DB>;
@@ -216,6 +218,7 @@ k_sort_pass(const u64* __restrict__ kin, const u64* __restrict__ iin, u64* __res
     }
   }
   __syncthreads();
+  const u64 sc = MSD ? *scale : 0ull;
   const u32 tile = s_tile;
   const u64 base = (u64)tile * kSortTile;
   const u64 left = n - base;
@@ -273,7 +276,8 @@ k_sort_pass(const u64* __restrict__ kin, const u64* __restrict__ iin, u64* __res
 #pragma unroll
   for (int it = 0; it < kSortItems; ++it) {
     const int e = wid * 32 * kSortItems + it * 32 + lane;
-    const u32 d = e < tr ? (u32)((key[it] >> shift) & (u64)(R - 1)) : kNone;
+    const u64 kd = MSD ? __umul64hi(key[it], sc) : key[it];
+    const u32 d = e < tr ? (u32)((kd >> shift) & (u64)(R - 1)) : kNone;
     const bool valid = d < kNone;
     if (valid) atomicOr(&mm[d], 1u << lane);
     __syncwarp();
@@ -415,6 +419,276 @@ k_sort_pass(const u64* __restrict__ kin, const u64* __restrict__ iin, u64* __res
 }
 
 // ---------------------------------------------------------------------------
+// Segment sort: the sort of sides whose keys spread over their range (residues do).
+//
+// An LSD sort moves every record once per digit, 7 or 8 times.  Here the scaled key
+//     f = mulhi(key, S),  S = floor(2^(64 + T + L) / (max key + 1))
+// (monotone in the key, below 2^(T + L), even over the range whatever the largest key) is sorted by
+// its top T bits only, in one or two onesweep passes, which leaves 2^T segments of 1,500 to 3,000
+// records in order; each is then sorted in shared memory by one CTA: the next L bits of f are its
+// bin (about one record per bin), one atomic per record gives bin sizes and slots, and a record's
+// place is its bin's start plus the records of the bin before it in (key, position) order.  A
+// record moves 32 bytes per onesweep pass and 32 in the segment sort.
+//
+// A segment above kSegCap records (few distinct keys, or keys far from even) leaves the records as
+// the passes left them, a stable reordering, and the caller runs the LSD sort on that.
+// ---------------------------------------------------------------------------
+constexpr int kSegBlock = 512;
+constexpr int kSegItems = 8;
+constexpr int kSegCap = kSegBlock * kSegItems;         // 4096 records
+constexpr int kSegBits = 12;                           // L: bins of a segment, log2
+constexpr int kSegBins = 1 << kSegBits;
+constexpr int kSegBinMax = 32;                         // larger bins: the segment goes to the bitonic sort
+constexpr size_t kSegSmem = (size_t)kSegCap * 8 + kSegCap * 2 + (size_t)kSegBins * 4;
+
+struct SegCtl {            // zeroed before the sort
+  u64 max_key, scale;
+  u32 blocks_done, max_seg, tickets[2];
+};
+
+__device__ __forceinline__ u64 seg_scale(u64 max_key, int bits) {   // floor(2^(64 + bits) / (max + 1)), at most 2^64 - 1
+  const u64 d = max_key + 1;
+  if (d == 0) return 1ull << bits;                     // max = 2^64 - 1
+  if (d <= (1ull << bits)) return ~0ull;
+  const unsigned __int128 num = (unsigned __int128)1 << (64 + bits);
+  return (u64)(num / d);
+}
+
+__global__ void __launch_bounds__(512) k_seg_max(const u64* __restrict__ keys, u64 n, int bits, SegCtl* ctl) {
+  __shared__ u64 s_m[16];
+  u64 m = 0;
+  for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64)gridDim.x * blockDim.x) {
+    const u64 k = keys[i];
+    m = k > m ? k : m;
+  }
+#pragma unroll
+  for (int o = 16; o; o >>= 1) {
+    const u64 x = __shfl_xor_sync(0xffffffffu, m, o);
+    m = x > m ? x : m;
+  }
+  if ((threadIdx.x & 31) == 0) s_m[threadIdx.x >> 5] = m;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 16; ++w) m = s_m[w] > m ? s_m[w] : m;
+    atomicMax((unsigned long long*)&ctl->max_key, (unsigned long long)m);
+    __threadfence();
+    if (atomicAdd(&ctl->blocks_done, 1u) == gridDim.x - 1) {
+      __threadfence();
+      ctl->scale = seg_scale(*(volatile u64*)&ctl->max_key, bits);
+    }
+  }
+}
+
+// Histograms of the one or two digits of the scaled key: bits [kSegBits + p * db, ...) of f, p < np.
+__global__ void __launch_bounds__(512)
+k_seg_hist(const u64* __restrict__ keys, u64 n, const SegCtl* __restrict__ ctl, u64* __restrict__ hist, int np, int db) {
+  __shared__ u32 s_h[2 << 9];
+  const int bins = np << db;
+  const u32 mask = (1u << db) - 1u;
+  for (int i = threadIdx.x; i < bins; i += blockDim.x) s_h[i] = 0;
+  const u64 sc = ctl->scale;
+  __syncthreads();
+  for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64)gridDim.x * blockDim.x) {
+    const u32 v = (u32)(__umul64hi(keys[i], sc) >> kSegBits);
+    atomicAdd(&s_h[v & mask], 1u);
+    if (np > 1) atomicAdd(&s_h[(1u << db) + (v >> db)], 1u);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < bins; i += blockDim.x)
+    if (s_h[i]) atomicAdd((unsigned long long*)&hist[i], (unsigned long long)s_h[i]);
+}
+
+// First record of each of the 2^T segments (records ordered by f >> kSegBits), and the largest segment.
+__global__ void __launch_bounds__(256)
+k_seg_bounds(const u64* __restrict__ keys, u32 n, int T, SegCtl* __restrict__ ctl, u32* __restrict__ starts) {
+  const u32 s = blockIdx.x * blockDim.x + threadIdx.x, ns = 1u << T;
+  const u64 sc = ctl->scale;
+  u32 len = 0;
+  if (s <= ns) {
+    u32 at[2];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {                      // lower bounds of segments s and s + 1
+      u32 lo = 0, hi = n;
+      if (s + e >= ns) lo = n;
+      while (lo < hi) {
+        const u32 mid = (lo + hi) >> 1;
+        if ((u32)(__umul64hi(keys[mid], sc) >> kSegBits) < s + e) lo = mid + 1; else hi = mid;
+      }
+      at[e] = lo;
+    }
+    starts[s] = at[0];
+    len = at[1] - at[0];
+  }
+#pragma unroll
+  for (int o = 16; o; o >>= 1) len = max(len, __shfl_xor_sync(0xffffffffu, len, o));
+  if ((threadIdx.x & 31) == 0 && len) atomicMax(&ctl->max_seg, len);
+}
+
+// Sort one segment by (key, position).  Two CTAs of 512 threads per SM (57 KB, 64 registers): while
+// one loads or stores, the other ranks.  starts == nullptr: the whole array is one segment (n <=
+// kSegCap) and its largest key is found here.
+__global__ void __launch_bounds__(kSegBlock, 2)
+k_seg_sort(const u64* kin, const u64* iin, u64* kout, u64* iout, u32 n, const SegCtl* __restrict__ ctl,
+           const u32* __restrict__ starts) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  u64* s_key = (u64*)smem;                             // [kSegCap]
+  u16* s_pos = (u16*)(s_key + kSegCap);                // [kSegCap]
+  u32* s_bin = (u32*)(s_pos + kSegCap);                // [kSegBins] sizes, then starts
+  __shared__ u32 s_w[kSegBlock / 32];
+  __shared__ u64 s_m[kSegBlock / 32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  if (starts && ctl->max_seg > (u32)kSegCap) return;   // uniform: the caller takes the LSD sort
+  const u32 first = starts ? starts[blockIdx.x] : 0u;
+  const u32 m = starts ? starts[blockIdx.x + 1] - first : n;
+  if (m == 0) return;
+  u64 key[kSegItems], id[kSegItems];
+#pragma unroll
+  for (int k = 0; k < kSegItems; ++k) {
+    const u32 j = threadIdx.x + k * kSegBlock;
+    key[k] = j < m ? kin[first + j] : 0ull;
+    id[k] = j < m ? iin[first + j] : 0ull;
+  }
+  for (int i = threadIdx.x; i < kSegBins; i += kSegBlock) s_bin[i] = 0;
+  u64 sc;
+  if (starts) {
+    sc = ctl->scale;
+    __syncthreads();
+  } else {
+    u64 mx = 0;
+#pragma unroll
+    for (int k = 0; k < kSegItems; ++k) mx = key[k] > mx ? key[k] : mx;
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+      const u64 x = __shfl_xor_sync(0xffffffffu, mx, o);
+      mx = x > mx ? x : mx;
+    }
+    if (lane == 0) s_m[wid] = mx;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int w = 1; w < kSegBlock / 32; ++w) mx = s_m[w] > mx ? s_m[w] : mx;
+      s_m[0] = seg_scale(mx, kSegBits);
+    }
+    __syncthreads();
+    sc = s_m[0];
+  }
+  u32 bs[kSegItems];                                   // bin << 16 | slot in the bin
+#pragma unroll
+  for (int k = 0; k < kSegItems; ++k) {
+    const u32 j = threadIdx.x + k * kSegBlock;
+    const u32 b = (u32)__umul64hi(key[k], sc) & (kSegBins - 1u);
+    bs[k] = j < m ? (b << 16) | atomicAdd(&s_bin[b], 1u) : 0u;
+  }
+  __syncthreads();
+  // exclusive scan of the bin sizes, 8 bins per thread
+  constexpr int kPer = kSegBins / kSegBlock;
+  u32 c[kPer], sum = 0, big = 0;
+#pragma unroll
+  for (int q = 0; q < kPer; ++q) {
+    c[q] = s_bin[threadIdx.x * kPer + q];
+    big = max(big, c[q]);
+    sum += c[q];
+  }
+  u32 incl = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const u32 x = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += x;
+  }
+  if (lane == 31) s_w[wid] = incl;
+  const bool heavy = __syncthreads_or(big > (u32)kSegBinMax) != 0;
+  u32 run = incl - sum;
+  for (int w = 0; w < wid; ++w) run += s_w[w];
+#pragma unroll
+  for (int q = 0; q < kPer; ++q) {
+    s_bin[threadIdx.x * kPer + q] = run;
+    run += c[q];
+  }
+  __syncthreads();
+  if (!heavy) {
+    u32 at[kSegItems];
+#pragma unroll
+    for (int k = 0; k < kSegItems; ++k) {
+      const u32 j = threadIdx.x + k * kSegBlock;
+      at[k] = s_bin[bs[k] >> 16];
+      if (j < m) {
+        s_key[at[k] + (bs[k] & 0xffffu)] = key[k];
+        s_pos[at[k] + (bs[k] & 0xffffu)] = (u16)j;
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kSegItems; ++k) {
+      const u32 j = threadIdx.x + k * kSegBlock;
+      if (j >= m) continue;
+      const u32 b = bs[k] >> 16, lo = at[k], hi = b + 1 < (u32)kSegBins ? s_bin[b + 1] : m;
+      u32 r = 0;
+      if (hi - lo > 1)
+        for (u32 q = lo; q < hi; ++q) {
+          const u64 o = s_key[q];
+          r += (o < key[k] || (o == key[k] && s_pos[q] < j)) ? 1u : 0u;
+        }
+      at[k] = lo + r;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kSegItems; ++k)
+      if (threadIdx.x + k * kSegBlock < m) s_key[at[k]] = key[k];
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kSegItems; ++k) {
+      const u32 j = threadIdx.x + k * kSegBlock;
+      if (j < m) kout[first + j] = s_key[j];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kSegItems; ++k)
+      if (threadIdx.x + k * kSegBlock < m) s_key[at[k]] = id[k];
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kSegItems; ++k) {
+      const u32 j = threadIdx.x + k * kSegBlock;
+      if (j < m) iout[first + j] = s_key[j];
+    }
+    return;
+  }
+  // many records in one bin: bitonic sort of (key, position); the padding (~0, 0xffff) stays last
+  u32 p2 = 2;
+  while (p2 < m) p2 <<= 1;
+#pragma unroll
+  for (int k = 0; k < kSegItems; ++k) {
+    const u32 j = threadIdx.x + k * kSegBlock;
+    if (j < p2) {
+      s_key[j] = j < m ? key[k] : ~0ull;
+      s_pos[j] = j < m ? (u16)j : (u16)0xffff;
+    }
+  }
+  __syncthreads();
+  for (u32 w = 2; w <= p2; w <<= 1)
+    for (u32 h = w >> 1; h; h >>= 1) {
+      for (u32 t = threadIdx.x; t < p2 / 2; t += kSegBlock) {
+        const u32 x = 2 * t - (t & (h - 1)), y = x + h;
+        const u64 ka = s_key[x], kb = s_key[y];
+        const u16 pa = s_pos[x], pb = s_pos[y];
+        const bool gt = ka > kb || (ka == kb && pa > pb);
+        if (gt == ((x & w) == 0)) {
+          s_key[x] = kb; s_key[y] = ka;
+          s_pos[x] = pb; s_pos[y] = pa;
+        }
+      }
+      __syncthreads();
+    }
+  for (u32 j = threadIdx.x; j < m; j += kSegBlock) kout[first + j] = s_key[j];
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < kSegItems; ++k) {
+    const u32 j = threadIdx.x + k * kSegBlock;
+    if (j < m) s_key[j] = id[k];
+  }
+  __syncthreads();
+  for (u32 j = threadIdx.x; j < m; j += kSegBlock) iout[first + j] = s_key[s_pos[j]];
+}
+
+// ---------------------------------------------------------------------------
 // Merge join of two sorted key arrays.
 // ---------------------------------------------------------------------------
 constexpr int kMergeBlock = 256;
@@ -479,29 +753,30 @@ static size_t sort_tmp_bytes(u64 n, int np, int db) {
 
 static int sort_passes(int key_bits, int db) { return (key_bits + db - 1) / db; }
 
-template <int DB, typename SW>
+template <int DB, typename SW, bool MSD>
 static cudaError_t sort_pass_attrs() {
-  cudaError_t e = cudaFuncSetAttribute(k_sort_pass<DB, true, SW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  cudaError_t e = cudaFuncSetAttribute(k_sort_pass<DB, true, SW, MSD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)PassLayout<DB>::kSmem);
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_sort_pass<DB, false, SW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    e = cudaFuncSetAttribute(k_sort_pass<DB, false, SW, MSD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)PassLayout<DB>::kSmem);
   return e;
 }
 
-template <int DB, typename SW>
+template <int DB, typename SW, bool MSD = false>
 static void sort_pass_launch(bool bulk, unsigned tiles, cudaStream_t st, const u64* ka, const u64* ia, u64* kb,
-                             u64* ib, u64 n, int shift, const u64* excl, SW* status, u32* ticket, u32* errw) {
+                             u64* ib, u64 n, int shift, const u64* excl, SW* status, u32* ticket, u32* errw,
+                             const u64* scale = nullptr) {
   if (bulk)
-    k_sort_pass<DB, true, SW><<<tiles, kSortBlock, PassLayout<DB>::kSmem, st>>>(ka, ia, kb, ib, n, shift, excl,
-                                                                              status, ticket, errw);
+    k_sort_pass<DB, true, SW, MSD><<<tiles, kSortBlock, PassLayout<DB>::kSmem, st>>>(ka, ia, kb, ib, n, shift, scale,
+                                                                                     excl, status, ticket, errw);
   else
-    k_sort_pass<DB, false, SW><<<tiles, kSortBlock, PassLayout<DB>::kSmem, st>>>(ka, ia, kb, ib, n, shift, excl,
-                                                                               status, ticket, errw);
+    k_sort_pass<DB, false, SW, MSD><<<tiles, kSortBlock, PassLayout<DB>::kSmem, st>>>(ka, ia, kb, ib, n, shift, scale,
+                                                                                      excl, status, ticket, errw);
 }
 
 template <typename SW>
-static cudaError_t sort_passes_attrs(int db) { return db == 8 ? sort_pass_attrs<8, SW>() : sort_pass_attrs<9, SW>(); }
+static cudaError_t sort_passes_attrs(int db) { return db == 8 ? sort_pass_attrs<8, SW, false>() : sort_pass_attrs<9, SW, false>(); }
 
 // The sort behind cf_sort_pairs and cf_sort_pairs_digits: np = ceil(key_bits / db)
 // passes of db-bit digits (8 or 9), passes whose digit is constant skipped.
@@ -613,6 +888,103 @@ extern "C" int cf_sort_pairs_digits(u64* keys, u64* ids, u64 n, int key_bits, in
   if (rc != CF_OK) return rc;
   return sort_pairs(keys, ids, n, key_bits, digit_bits, tmp, tmp_bytes,
                     cf_sort_digits_tmp_bytes(n, key_bits, digit_bits), (cudaStream_t)stream);
+}
+
+// Bits T of the scaled key that the onesweep passes sort: segments of 1,500 to 3,000 records.
+static int seg_bits(u64 n) {
+  int T = 0;
+  while (T < 18 && (n >> T) > 3000) ++T;
+  return T;
+}
+constexpr u64 kSegMaxN = 3000ull << 18;                // 7.9e8: two 9-bit digits
+
+// Workspace of cf_sort_pairs_to for n records.
+extern "C" size_t cf_sort_to_tmp_bytes(u64 n) {
+  const size_t lsd = sort_tmp_bytes(n, kMaxPasses, 8), lsd9 = sort_tmp_bytes(n, sort_passes(64, 9), 9);
+  return (lsd > lsd9 ? lsd : lsd9) + ((size_t)8 << 18) + 65536;
+}
+
+// Stable sort of (kin, iin)[n] by key into (kout, iout), which must not overlap the inputs; the
+// inputs are left as they are.  digit_bits (8 or 9): the digit width of the LSD sort that takes the
+// sides the segment sort does not (above 7.9e8 records, or a segment above 4096 records).
+// Synchronises the stream once at the end (twice where the LSD sort runs).
+extern "C" int cf_sort_pairs_to(const u64* kin, const u64* iin, u64* kout, u64* iout, u64 n, int digit_bits, void* tmp,
+                                size_t tmp_bytes, void* stream) {
+  if (digit_bits != 8 && digit_bits != 9) {
+    cf_set_error("cf_sort_pairs_to: digit_bits must be 8 or 9%s", "");
+    return CF_EBADARG;
+  }
+  if (n == 0) return CF_OK;
+  if (!kin || !iin || !kout || !iout || !tmp) { cf_set_error("cf_sort_pairs_to: null buffer%s", ""); return CF_EBADARG; }
+  if (n > (1ull << 40)) { cf_set_error("cf_sort_pairs_to: n too large%s", ""); return CF_EBADARG; }
+  if (tmp_bytes < cf_sort_to_tmp_bytes(n)) { cf_set_error("cf_sort_pairs_to: workspace too small%s", ""); return CF_ENOMEM; }
+  const cudaStream_t st = (cudaStream_t)stream;
+  cudaError_t e = cudaFuncSetAttribute(k_seg_sort, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSegSmem);
+  if (e != cudaSuccess) return cf_cuda_status(e, "cf_sort_pairs_to: smem attribute");
+  if (n <= (u64)kSegCap) {                             // one segment: one launch
+    k_seg_sort<<<1, kSegBlock, kSegSmem, st>>>(kin, iin, kout, iout, (u32)n, nullptr, nullptr);
+    CF_LAUNCH_CHECK("cf_sort_pairs_to: one segment");
+    return cf_cuda_status(cudaStreamSynchronize(st), "cf_sort_pairs_to");
+  }
+  const u64 *src_k = kin, *src_i = iin;
+  u32 max_seg = ~0u, herr = 0;
+  if (n <= kSegMaxN) {
+    const int T = seg_bits(n), np = T <= 9 ? 1 : 2;
+    const int db = (np == 1 ? T : (T + 1) / 2) <= 8 ? 8 : 9, bins = 1 << db;
+    const u64 tiles = (n + kSortTile - 1) / kSortTile;
+    // workspace: second buffers, then the zeroed control words, histograms and status words
+    unsigned char* w = (unsigned char*)tmp;
+    const size_t side = (size_t)(n + (n & 1)) * 8;     // 16-byte aligned ids for the bulk copies
+    u64* k2 = (u64*)w; w += side;
+    u64* i2 = (u64*)w; w += side;
+    SegCtl* ctl = (SegCtl*)w; w += 256;
+    u32* errw = (u32*)(ctl + 1);
+    u64* hist = (u64*)w; w += (size_t)np * bins * 8;
+    u32* status = (u32*)w; w += (size_t)np * tiles * bins * 4;
+    const size_t zeroed = (size_t)(w - (unsigned char*)ctl);
+    u64* excl = (u64*)(((uintptr_t)w + 7) & ~(uintptr_t)7); w = (unsigned char*)(excl + (size_t)np * bins);
+    u32* starts = (u32*)w; w += ((size_t)4 << T) + 4;
+    if ((size_t)(w - (unsigned char*)tmp) > tmp_bytes) { cf_set_error("cf_sort_pairs_to: workspace too small%s", ""); return CF_ENOMEM; }
+    e = db == 8 ? sort_pass_attrs<8, u32, true>() : sort_pass_attrs<9, u32, true>();
+    if (e == cudaSuccess) e = cudaMemsetAsync(ctl, 0, zeroed, st);
+    if (e != cudaSuccess) return cf_cuda_status(e, "cf_sort_pairs_to: set-up");
+    const unsigned g = (unsigned)((n + 4095) / 4096), gm = g < 148 * 4 ? g : 148 * 4;
+    k_seg_max<<<gm, 512, 0, st>>>(kin, n, T + kSegBits, ctl);
+    k_seg_hist<<<gm, 512, 0, st>>>(kin, n, ctl, hist, np, db);
+    k_sort_hist_scan<<<1, 32 * np, 0, st>>>(hist, excl, db);
+    for (int p = 0; p < np; ++p) {
+      const u64 *ka = p ? k2 : kin, *ia = p ? i2 : iin;
+      u64 *kb = p + 1 == np ? kout : k2, *ib = p + 1 == np ? iout : i2;
+      const bool bulk = ((((uintptr_t)ka) | ((uintptr_t)ia)) & 15u) == 0;
+      const int shift = kSegBits + p * db;
+      u32* pst = status + (size_t)p * tiles * bins;
+      if (db == 8)
+        sort_pass_launch<8, u32, true>(bulk, (unsigned)tiles, st, ka, ia, kb, ib, n, shift, excl + p * bins, pst,
+                                       ctl->tickets + p, errw, &ctl->scale);
+      else
+        sort_pass_launch<9, u32, true>(bulk, (unsigned)tiles, st, ka, ia, kb, ib, n, shift, excl + p * bins, pst,
+                                       ctl->tickets + p, errw, &ctl->scale);
+    }
+    k_seg_bounds<<<((1u << T) + 256) / 256, 256, 0, st>>>(kout, (u32)n, T, ctl, starts);
+    k_seg_sort<<<1u << T, kSegBlock, kSegSmem, st>>>(kout, iout, kout, iout, (u32)n, ctl, starts);
+    CF_LAUNCH_CHECK("cf_sort_pairs_to: segments");
+    SegCtl h[2];                                       // control words and, after them, the error word
+    e = cudaMemcpyAsync(h, ctl, sizeof(SegCtl) + 4, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) return cf_cuda_status(e, "cf_sort_pairs_to: control words");
+    max_seg = h[0].max_seg;
+    memcpy(&herr, &h[1], 4);
+    if (herr & CF_ERR_SPIN_LIMIT) { cf_set_error("cf_sort_pairs_to: look-back wait exceeded its limit%s", ""); return CF_ETIMEOUT; }
+    if (max_seg <= (u32)kSegCap) return CF_OK;
+    src_k = kout;                                      // ordered by the top bits, equal keys in input order
+    src_i = iout;
+  }
+  if (src_k == kin) {
+    e = cudaMemcpyAsync(kout, src_k, n * 8, cudaMemcpyDeviceToDevice, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(iout, src_i, n * 8, cudaMemcpyDeviceToDevice, st);
+    if (e != cudaSuccess) return cf_cuda_status(e, "cf_sort_pairs_to: copy");
+  }
+  return sort_pairs(kout, iout, n, 64, digit_bits, tmp, tmp_bytes, sort_tmp_bytes(n, sort_passes(64, digit_bits), digit_bits), st);
 }
 
 extern "C" size_t cf_merge_run_bytes(void) { return sizeof(CfRun); }

@@ -6,7 +6,7 @@ CuPy arrays.  Every function runs hand-written sm_100a kernels through the C ABI
 (``include/cfmitm.h``):
 
   generate    -> cf_gen_subsets   (lexicographic rank ranges, canonical residues)
-  sort_side   -> cf_sort_pairs_digits (stable LSD onesweep radix sort, keys and ids, tuned digit width)
+  sort_side   -> cf_sort_pairs_to (stable; partition by leading bits, segments sorted in shared memory)
   join_sorted -> cf_merge_join_runs + host expansion of the (rare) equal runs
 """
 from __future__ import annotations
@@ -102,22 +102,31 @@ def set_sort_digit_bits(n: int, bits: int | None) -> None:
 
 
 def sort_side(keys, ids, digit_bits: int | None = None):
-    """Sort one side by key (stable LSD radix sort). Returns (sorted_keys, sorted_ids).
-    digit_bits (8 or 9) overrides the tuned radix digit width; the result is the same."""
+    """Sort one side by key (stable). Returns (sorted_keys, sorted_ids).  digit_bits (8 or 9) takes
+    the LSD radix sort of that digit width; the result is the same."""
+    torch = _torch()
     n = keys.numel()
-    ko = keys.contiguous().clone()
-    io = ids.contiguous().clone()
-    if n <= 1:
-        return ko, io
+    ki, ii = keys.contiguous(), ids.contiguous()
     db = sort_digit_bits(n) if digit_bits is None else int(digit_bits)
-    if db not in SORT_DIGIT_WIDTHS:
+    if n > 1 and db not in SORT_DIGIT_WIDTHS:
         raise ValueError(f"digit width {db} not in {SORT_DIGIT_WIDTHS}")
-    dev = ko.device
     lib = _lib.load()
-    nbytes = lib.cf_sort_digits_tmp_bytes(n, 64, db)
-    tmp = _workspace(dev, "sort", nbytes)
-    _lib.check(lib.cf_sort_pairs_digits(_lib.ptr(ko), _lib.ptr(io), n, 64, db, _lib.ptr(tmp), nbytes,
-                                        _lib.stream_handle()), "sort_side")
+    if n <= 1 or digit_bits is not None:       # the LSD sort, in place on copies
+        ko, io = ki.clone(), ii.clone()
+        if n <= 1:
+            return ko, io
+        nbytes = lib.cf_sort_digits_tmp_bytes(n, 64, db)
+        tmp = _workspace(ko.device, "sort", nbytes)
+        _lib.check(lib.cf_sort_pairs_digits(_lib.ptr(ko), _lib.ptr(io), n, 64, db, _lib.ptr(tmp), nbytes,
+                                            _lib.stream_handle()), "sort_side")
+        return ko, io
+    ko, io = torch.empty_like(ki), torch.empty_like(ii)
+    if ii.numel() > n:
+        io.view(-1)[n:] = ii.view(-1)[n:]
+    nbytes = lib.cf_sort_to_tmp_bytes(n)
+    tmp = _workspace(ko.device, "sort", nbytes)
+    _lib.check(lib.cf_sort_pairs_to(_lib.ptr(ki), _lib.ptr(ii), _lib.ptr(ko), _lib.ptr(io), n, db, _lib.ptr(tmp),
+                                    nbytes, _lib.stream_handle()), "sort_side")
     return ko, io
 
 

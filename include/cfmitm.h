@@ -460,6 +460,13 @@ size_t cf_sort_digits_tmp_bytes(uint64_t n, int key_bits, int digit_bits);
 int cf_sort_pairs_digits(uint64_t* keys, uint64_t* ids, uint64_t n, int key_bits, int digit_bits, void* tmp,
                          size_t tmp_bytes, void* stream);
 
+/* The same stable sort into other arrays, the inputs left as they are: one or two partition passes
+ * on the leading bits and a shared-memory sort of each segment, or, for keys that do not spread over
+ * their range, the LSD sort with digit_bits (8 or 9). */
+size_t cf_sort_to_tmp_bytes(uint64_t n);
+int cf_sort_pairs_to(const uint64_t* kin, const uint64_t* iin, uint64_t* kout, uint64_t* iout, uint64_t n,
+                     int digit_bits, void* tmp, size_t tmp_bytes, void* stream);
+
 /* The same sort for callers that cannot allocate device memory (for example
  * when all device memory belongs to another allocator): no workspace argument;
  * the scratch is a fixed array inside this library's own device memory (3 MiB,
