@@ -175,16 +175,32 @@ struct PassLayout {
   static_assert(2 * (kSmem + 1024 + 256) <= 233472, "two CTAs per SM");
 };
 
+// Control words of the segment sort (below) and its scaled key.
+struct SegCtl {            // zeroed before the sort
+  u64 scale;
+  u32 top;                 // 2^L NS - 1
+  u32 blocks_done, max_seg, tickets[2], pad;
+  u64 max_key;
+};
+struct SegScale {
+  u64 s;
+  u32 top;
+  __device__ __forceinline__ u32 operator()(u64 key) const {
+    const u64 f = __umul64hi(key, s);
+    return f < top ? (u32)f : top;
+  }
+};
+
 // One onesweep pass over the DB-bit digit at bit `shift`.  Two CTAs per SM.  BULK:
 // the tile's keys and ids are brought into shared memory by two bulk copies at
 // the start (every pointer 16-byte aligned), so the id load overlaps the ranking;
 // otherwise by plain coalesced loads.  Each item's digit (DB + 1 bits, R = no
 // item) rides in the top bits of its local offset.
-// MSD: the digit is taken from the scaled key mulhi(key, *scale) instead of the key.
+// MSD: the digit is taken from the scaled key (SegScale) instead of the key.
 template <int DB, bool BULK, typename SW, bool MSD>
 __global__ void __launch_bounds__(kSortBlock, 2)
 k_sort_pass(const u64* __restrict__ kin, const u64* __restrict__ iin, u64* __restrict__ kout,
-            u64* __restrict__ iout, u64 n, int shift, const u64* __restrict__ scale, const u64* __restrict__ gexcl /*[R]*/,
+            u64* __restrict__ iout, u64 n, int shift, const SegCtl* __restrict__ scale, const u64* __restrict__ gexcl /*[R]*/,
             SW* __restrict__ status /*[tiles][R]*/, u32* __restrict__ ticket, u32* __restrict__ err) {
   using St = Status<SW>;
   using L = PassLayout<DB>;
@@ -218,7 +234,7 @@ k_sort_pass(const u64* __restrict__ kin, const u64* __restrict__ iin, u64* __res
     }
   }
   __syncthreads();
-  const u64 sc = MSD ? *scale : 0ull;
+  const SegScale sc = MSD ? SegScale{scale->scale, scale->top} : SegScale{0, 0};
   const u32 tile = s_tile;
   const u64 base = (u64)tile * kSortTile;
   const u64 left = n - base;
@@ -276,7 +292,7 @@ k_sort_pass(const u64* __restrict__ kin, const u64* __restrict__ iin, u64* __res
 #pragma unroll
   for (int it = 0; it < kSortItems; ++it) {
     const int e = wid * 32 * kSortItems + it * 32 + lane;
-    const u64 kd = MSD ? __umul64hi(key[it], sc) : key[it];
+    const u64 kd = MSD ? (u64)sc(key[it]) : key[it];
     const u32 d = e < tr ? (u32)((kd >> shift) & (u64)(R - 1)) : kNone;
     const bool valid = d < kNone;
     if (valid) atomicOr(&mm[d], 1u << lane);
@@ -422,13 +438,14 @@ k_sort_pass(const u64* __restrict__ kin, const u64* __restrict__ iin, u64* __res
 // Segment sort: the sort of sides whose keys spread over their range (residues do).
 //
 // An LSD sort moves every record once per digit, 7 or 8 times.  Here the scaled key
-//     f = mulhi(key, S),  S = floor(2^(64 + T + L) / (max key + 1))
-// (monotone in the key, below 2^(T + L), even over the range whatever the largest key) is sorted by
-// its top T bits only, in one or two onesweep passes, which leaves 2^T segments of 1,500 to 3,000
-// records in order; each is then sorted in shared memory by one CTA: the next L bits of f are its
-// bin (about one record per bin), one atomic per record gives bin sizes and slots, and a record's
-// place is its bin's start plus the records of the bin before it in (key, position) order.  A
-// record moves 32 bytes per onesweep pass and 32 in the segment sort.
+//     f = min(mulhi(key, S), 2^L NS - 1),  S = floor(2^(64 + L) NS / (m + 1))
+// (monotone in the key, even over the range for m the largest key, whatever its size) is sorted by
+// f >> L only, in one or two onesweep passes, which leaves NS segments of about 3,400 records in
+// order; each is then sorted in shared memory by one CTA: the low L bits of f are its bin (about
+// one record per bin), one atomic per record gives bin sizes and slots, and a record's place is its
+// bin's start plus the records of the bin before it in (key, position) order.  A record moves 32
+// bytes per onesweep pass and 32 in the segment sort.  m is the largest of a sample of the keys; the
+// few above it share the last bin.
 //
 // A segment above kSegCap records (few distinct keys, or keys far from even) leaves the records as
 // the passes left them, a stable reordering, and the caller runs the LSD sort on that.
@@ -436,31 +453,25 @@ k_sort_pass(const u64* __restrict__ kin, const u64* __restrict__ iin, u64* __res
 constexpr int kSegBlock = 512;
 constexpr int kSegItems = 8;
 constexpr int kSegCap = kSegBlock * kSegItems;         // 4096 records
+constexpr u64 kSegMean = 3400;                         // records per segment: 12 sigma below the capacity
 constexpr int kSegBits = 12;                           // L: bins of a segment, log2
 constexpr int kSegBins = 1 << kSegBits;
 constexpr int kSegBinMax = 32;                         // larger bins: the segment goes to the bitonic sort
-constexpr size_t kSegSmem = (size_t)kSegCap * 8 + kSegCap * 2 + (size_t)kSegBins * 4;
+constexpr size_t kSegSmem = (size_t)kSegCap * 18 + (size_t)kSegBins * 4;
+constexpr u32 kSegFrontMax = 1u << 16;                 // up to here one CTA samples, counts and scans
+constexpr u64 kSegMaxN = kSegMean << 18;               // 8.9e8: two 9-bit digits
 
-struct SegCtl {            // zeroed before the sort
-  u64 max_key, scale;
-  u32 blocks_done, max_seg, tickets[2];
-};
-
-__device__ __forceinline__ u64 seg_scale(u64 max_key, int bits) {   // floor(2^(64 + bits) / (max + 1)), at most 2^64 - 1
-  const u64 d = max_key + 1;
-  if (d == 0) return 1ull << bits;                     // max = 2^64 - 1
-  if (d <= (1ull << bits)) return ~0ull;
-  const unsigned __int128 num = (unsigned __int128)1 << (64 + bits);
-  return (u64)(num / d);
+__device__ __forceinline__ SegScale seg_scale(u64 max_key, u32 segs) {
+  const u64 d = max_key + 1, range = (u64)segs << kSegBits;
+  SegScale r;
+  r.top = (u32)(range - 1);
+  if (d == 0) r.s = range;                             // max = 2^64 - 1
+  else if (d <= range) r.s = ~0ull;                    // f = key - 1: below the range already
+  else r.s = (u64)(((unsigned __int128)range << 64) / d);
+  return r;
 }
 
-__global__ void __launch_bounds__(512) k_seg_max(const u64* __restrict__ keys, u64 n, int bits, SegCtl* ctl) {
-  __shared__ u64 s_m[16];
-  u64 m = 0;
-  for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64)gridDim.x * blockDim.x) {
-    const u64 k = keys[i];
-    m = k > m ? k : m;
-  }
+__device__ __forceinline__ u64 block_max(u64 m, u64* s_m) {
 #pragma unroll
   for (int o = 16; o; o >>= 1) {
     const u64 x = __shfl_xor_sync(0xffffffffu, m, o);
@@ -468,28 +479,47 @@ __global__ void __launch_bounds__(512) k_seg_max(const u64* __restrict__ keys, u
   }
   if ((threadIdx.x & 31) == 0) s_m[threadIdx.x >> 5] = m;
   __syncthreads();
+  m = s_m[0];
+  for (u32 w = 1; w < blockDim.x / 32; ++w) m = s_m[w] > m ? s_m[w] : m;
+  __syncthreads();
+  return m;
+}
+
+// Sampled maximum: one run of 32 keys of every 32 * step.
+__global__ void __launch_bounds__(512) k_seg_max(const u64* __restrict__ keys, u64 n, u32 step, u32 segs, SegCtl* ctl) {
+  __shared__ u64 s_m[16];
+  u64 m = 0;
+  const u64 lanes = (u64)gridDim.x * blockDim.x;
+  for (u64 t = (u64)blockIdx.x * blockDim.x + threadIdx.x;; t += lanes) {
+    const u64 i = (t >> 5) * 32 * step + (t & 31);
+    if (i >= n) break;
+    const u64 k = keys[i];
+    m = k > m ? k : m;
+  }
+  m = block_max(m, s_m);
   if (threadIdx.x == 0) {
-    for (int w = 1; w < 16; ++w) m = s_m[w] > m ? s_m[w] : m;
     atomicMax((unsigned long long*)&ctl->max_key, (unsigned long long)m);
     __threadfence();
     if (atomicAdd(&ctl->blocks_done, 1u) == gridDim.x - 1) {
       __threadfence();
-      ctl->scale = seg_scale(*(volatile u64*)&ctl->max_key, bits);
+      const SegScale sc = seg_scale(*(volatile u64*)&ctl->max_key, segs);
+      ctl->scale = sc.s;
+      ctl->top = sc.top;
     }
   }
 }
 
-// Histograms of the one or two digits of the scaled key: bits [kSegBits + p * db, ...) of f, p < np.
+// Histograms of the one or two digits of f >> L: db low bits, then the rest.
 __global__ void __launch_bounds__(512)
 k_seg_hist(const u64* __restrict__ keys, u64 n, const SegCtl* __restrict__ ctl, u64* __restrict__ hist, int np, int db) {
   __shared__ u32 s_h[2 << 9];
   const int bins = np << db;
   const u32 mask = (1u << db) - 1u;
   for (int i = threadIdx.x; i < bins; i += blockDim.x) s_h[i] = 0;
-  const u64 sc = ctl->scale;
+  const SegScale sc{ctl->scale, ctl->top};
   __syncthreads();
   for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64)gridDim.x * blockDim.x) {
-    const u32 v = (u32)(__umul64hi(keys[i], sc) >> kSegBits);
+    const u32 v = sc(keys[i]) >> kSegBits;
     atomicAdd(&s_h[v & mask], 1u);
     if (np > 1) atomicAdd(&s_h[(1u << db) + (v >> db)], 1u);
   }
@@ -498,41 +528,88 @@ k_seg_hist(const u64* __restrict__ keys, u64 n, const SegCtl* __restrict__ ctl, 
     if (s_h[i]) atomicAdd((unsigned long long*)&hist[i], (unsigned long long)s_h[i]);
 }
 
-// First record of each of the 2^T segments (records ordered by f >> kSegBits), and the largest segment.
-__global__ void __launch_bounds__(256)
-k_seg_bounds(const u64* __restrict__ keys, u32 n, int T, SegCtl* __restrict__ ctl, u32* __restrict__ starts) {
-  const u32 s = blockIdx.x * blockDim.x + threadIdx.x, ns = 1u << T;
-  const u64 sc = ctl->scale;
-  u32 len = 0;
-  if (s <= ns) {
-    u32 at[2];
+// Up to kSegFrontMax records, one digit (segs <= 256): maximum, counts, offsets and starts in one CTA.
+__global__ void __launch_bounds__(1024)
+k_seg_front(const u64* __restrict__ keys, u32 n, u32 segs, SegCtl* __restrict__ ctl, u64* __restrict__ excl,
+            u32* __restrict__ starts) {
+  __shared__ u64 s_m[32];
+  __shared__ u32 s_h[256], s_w[8];
+  u64 m = 0;
+  for (u32 i = threadIdx.x; i < n; i += 4096)          // a quarter of the keys
+    m = keys[i] > m ? keys[i] : m;
+  if (threadIdx.x < 256) s_h[threadIdx.x] = 0;
+  m = block_max(m, s_m);
+  if (threadIdx.x == 0) {
+    const SegScale sc = seg_scale(m, segs);
+    ctl->scale = s_m[0] = sc.s;
+    ctl->top = sc.top;
+  }
+  __syncthreads();
+  const SegScale sc{s_m[0], (segs << kSegBits) - 1u};
+#pragma unroll 8
+  for (u32 i = threadIdx.x; i < n; i += 1024) atomicAdd(&s_h[sc(keys[i]) >> kSegBits], 1u);
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  u32 v = 0, incl = 0;
+  if (threadIdx.x < 256) {
+    v = incl = s_h[threadIdx.x];
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {                      // lower bounds of segments s and s + 1
-      u32 lo = 0, hi = n;
-      if (s + e >= ns) lo = n;
-      while (lo < hi) {
-        const u32 mid = (lo + hi) >> 1;
-        if ((u32)(__umul64hi(keys[mid], sc) >> kSegBits) < s + e) lo = mid + 1; else hi = mid;
-      }
-      at[e] = lo;
+    for (int o = 1; o < 32; o <<= 1) {
+      const u32 x = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += x;
     }
-    starts[s] = at[0];
-    len = at[1] - at[0];
+    if (lane == 31) s_w[threadIdx.x >> 5] = incl;
+    atomicMax(&ctl->max_seg, v);
+  }
+  __syncthreads();
+  if (threadIdx.x < 256) {
+    u32 add = 0;
+    for (u32 w = 0; w < threadIdx.x >> 5; ++w) add += s_w[w];
+    excl[threadIdx.x] = add + incl - v;
+    if (threadIdx.x <= segs) starts[threadIdx.x] = add + incl - v;
+    if (threadIdx.x == 255 && segs == 256) starts[256] = add + incl;
+  }
+}
+
+// First record of each segment (records ordered by f >> L), and the largest segment.
+__global__ void __launch_bounds__(256)
+k_seg_bounds(const u64* __restrict__ keys, u32 n, u32 segs, SegCtl* __restrict__ ctl, u32* __restrict__ starts) {
+  const u32 s = blockIdx.x * blockDim.x + threadIdx.x;
+  const SegScale sc{ctl->scale, ctl->top};
+  u32 lo = 0, hi = s < segs ? n : 0u, len = 0;
+  while (lo < hi) {                                    // lower bound of segment s
+    const u32 mid = (lo + hi) >> 1;
+    if ((sc(keys[mid]) >> kSegBits) < s) lo = mid + 1; else hi = mid;
+  }
+  if (s >= segs) lo = n;
+  if (s <= segs) starts[s] = lo;
+  const u32 next = __shfl_down_sync(0xffffffffu, lo, 1);
+  if ((threadIdx.x & 31) < 31) len = next - lo;
+  else if (s < segs) {                                 // the next warp's first segment
+    u32 l2 = lo, h2 = s + 1 < segs ? n : lo;
+    while (l2 < h2) {
+      const u32 mid = (l2 + h2) >> 1;
+      if ((sc(keys[mid]) >> kSegBits) < s + 1) l2 = mid + 1; else h2 = mid;
+    }
+    len = (s + 1 < segs ? l2 : n) - lo;
   }
 #pragma unroll
   for (int o = 16; o; o >>= 1) len = max(len, __shfl_xor_sync(0xffffffffu, len, o));
   if ((threadIdx.x & 31) == 0 && len) atomicMax(&ctl->max_seg, len);
 }
 
-// Sort one segment by (key, position).  Two CTAs of 512 threads per SM (57 KB, 64 registers): while
-// one loads or stores, the other ranks.  starts == nullptr: the whole array is one segment (n <=
-// kSegCap) and its largest key is found here.
+// Sort one segment by (key, position).  Bound by its chain of shared-memory phases (issue slots 45%
+// busy, L1 61%, DRAM a third): 2^26 records in 1.02 ms, 2.1 TB/s; the onesweep pass takes 0.71 ms for
+// the same records and the whole sort 2.67 ms (6.28 ms as eight LSD passes).  Two CTAs of 512 threads per SM (88 KB of shared memory, 64
+// registers): while one loads or stores, the other ranks.  starts == nullptr: the whole array is one
+// segment (n <= kSegCap) and its largest key is found here.
 __global__ void __launch_bounds__(kSegBlock, 2)
 k_seg_sort(const u64* kin, const u64* iin, u64* kout, u64* iout, u32 n, const SegCtl* __restrict__ ctl,
            const u32* __restrict__ starts) {
   extern __shared__ __align__(16) unsigned char smem[];
-  u64* s_key = (u64*)smem;                             // [kSegCap]
-  u16* s_pos = (u16*)(s_key + kSegCap);                // [kSegCap]
+  u64* s_key = (u64*)smem;                             // [kSegCap] in bin order
+  u64* s_id = s_key + kSegCap;                         // [kSegCap] ids in input order
+  u16* s_pos = (u16*)(s_id + kSegCap);                 // [kSegCap] input position of s_key's record
   u32* s_bin = (u32*)(s_pos + kSegCap);                // [kSegBins] sizes, then starts
   __shared__ u32 s_w[kSegBlock / 32];
   __shared__ u64 s_m[kSegBlock / 32];
@@ -541,41 +618,38 @@ k_seg_sort(const u64* kin, const u64* iin, u64* kout, u64* iout, u32 n, const Se
   const u32 first = starts ? starts[blockIdx.x] : 0u;
   const u32 m = starts ? starts[blockIdx.x + 1] - first : n;
   if (m == 0) return;
-  u64 key[kSegItems], id[kSegItems];
+  u64 key[kSegItems];
 #pragma unroll
   for (int k = 0; k < kSegItems; ++k) {
     const u32 j = threadIdx.x + k * kSegBlock;
     key[k] = j < m ? kin[first + j] : 0ull;
-    id[k] = j < m ? iin[first + j] : 0ull;
+  }
+#pragma unroll
+  for (int k = 0; k < kSegItems; ++k) {
+    const u32 j = threadIdx.x + k * kSegBlock;
+    if (j < m) s_id[j] = iin[first + j];
   }
   for (int i = threadIdx.x; i < kSegBins; i += kSegBlock) s_bin[i] = 0;
-  u64 sc;
+  SegScale sc;
   if (starts) {
-    sc = ctl->scale;
+    sc.s = ctl->scale;
+    sc.top = ctl->top;
     __syncthreads();
   } else {
     u64 mx = 0;
 #pragma unroll
     for (int k = 0; k < kSegItems; ++k) mx = key[k] > mx ? key[k] : mx;
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-      const u64 x = __shfl_xor_sync(0xffffffffu, mx, o);
-      mx = x > mx ? x : mx;
-    }
-    if (lane == 0) s_m[wid] = mx;
+    mx = block_max(mx, s_m);
+    if (threadIdx.x == 0) s_m[0] = seg_scale(mx, 1u).s;
     __syncthreads();
-    if (threadIdx.x == 0) {
-      for (int w = 1; w < kSegBlock / 32; ++w) mx = s_m[w] > mx ? s_m[w] : mx;
-      s_m[0] = seg_scale(mx, kSegBits);
-    }
-    __syncthreads();
-    sc = s_m[0];
+    sc.s = s_m[0];
+    sc.top = kSegBins - 1u;
   }
   u32 bs[kSegItems];                                   // bin << 16 | slot in the bin
 #pragma unroll
   for (int k = 0; k < kSegItems; ++k) {
     const u32 j = threadIdx.x + k * kSegBlock;
-    const u32 b = (u32)__umul64hi(key[k], sc) & (kSegBins - 1u);
+    const u32 b = sc(key[k]) & (kSegBins - 1u);
     bs[k] = j < m ? (b << 16) | atomicAdd(&s_bin[b], 1u) : 0u;
   }
   __syncthreads();
@@ -583,8 +657,12 @@ k_seg_sort(const u64* kin, const u64* iin, u64* kout, u64* iout, u32 n, const Se
   constexpr int kPer = kSegBins / kSegBlock;
   u32 c[kPer], sum = 0, big = 0;
 #pragma unroll
+  for (int q = 0; q < kPer; q += 4) {
+    const uint4 v = *(const uint4*)&s_bin[threadIdx.x * kPer + q];
+    c[q] = v.x; c[q + 1] = v.y; c[q + 2] = v.z; c[q + 3] = v.w;
+  }
+#pragma unroll
   for (int q = 0; q < kPer; ++q) {
-    c[q] = s_bin[threadIdx.x * kPer + q];
     big = max(big, c[q]);
     sum += c[q];
   }
@@ -596,58 +674,50 @@ k_seg_sort(const u64* kin, const u64* iin, u64* kout, u64* iout, u32 n, const Se
   }
   if (lane == 31) s_w[wid] = incl;
   const bool heavy = __syncthreads_or(big > (u32)kSegBinMax) != 0;
-  u32 run = incl - sum;
-  for (int w = 0; w < wid; ++w) run += s_w[w];
-#pragma unroll
-  for (int q = 0; q < kPer; ++q) {
-    s_bin[threadIdx.x * kPer + q] = run;
-    run += c[q];
-  }
-  __syncthreads();
   if (!heavy) {
-    u32 at[kSegItems];
+    u32 run = incl - sum;
+    for (int w = 0; w < wid; ++w) run += s_w[w];
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+      const u32 v = c[q];
+      c[q] = run;
+      run += v;
+    }
+#pragma unroll
+    for (int q = 0; q < kPer; q += 4)
+      *(uint4*)&s_bin[threadIdx.x * kPer + q] = make_uint4(c[q], c[q + 1], c[q + 2], c[q + 3]);
+    __syncthreads();
 #pragma unroll
     for (int k = 0; k < kSegItems; ++k) {
       const u32 j = threadIdx.x + k * kSegBlock;
-      at[k] = s_bin[bs[k] >> 16];
       if (j < m) {
-        s_key[at[k] + (bs[k] & 0xffffu)] = key[k];
-        s_pos[at[k] + (bs[k] & 0xffffu)] = (u16)j;
+        const u32 to = s_bin[bs[k] >> 16] + (bs[k] & 0xffffu);
+        s_key[to] = key[k];
+        s_pos[to] = (u16)j;
       }
     }
     __syncthreads();
+    // place q of the bin order: its record moves within its bin only, by the records of the bin
+    // that come before it
 #pragma unroll
     for (int k = 0; k < kSegItems; ++k) {
-      const u32 j = threadIdx.x + k * kSegBlock;
-      if (j >= m) continue;
-      const u32 b = bs[k] >> 16, lo = at[k], hi = b + 1 < (u32)kSegBins ? s_bin[b + 1] : m;
-      u32 r = 0;
-      if (hi - lo > 1)
-        for (u32 q = lo; q < hi; ++q) {
-          const u64 o = s_key[q];
-          r += (o < key[k] || (o == key[k] && s_pos[q] < j)) ? 1u : 0u;
-        }
-      at[k] = lo + r;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < kSegItems; ++k)
-      if (threadIdx.x + k * kSegBlock < m) s_key[at[k]] = key[k];
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < kSegItems; ++k) {
-      const u32 j = threadIdx.x + k * kSegBlock;
-      if (j < m) kout[first + j] = s_key[j];
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < kSegItems; ++k)
-      if (threadIdx.x + k * kSegBlock < m) s_key[at[k]] = id[k];
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < kSegItems; ++k) {
-      const u32 j = threadIdx.x + k * kSegBlock;
-      if (j < m) iout[first + j] = s_key[j];
+      const u32 q = threadIdx.x + k * kSegBlock;
+      if (q >= m) continue;
+      const u64 kq = s_key[q];
+      const u32 pq = s_pos[q], f = sc(kq);
+      u32 to = q;
+      for (u32 x = q; x-- > 0;) {
+        const u64 o = s_key[x];
+        if (sc(o) != f) break;
+        to -= (o > kq || (o == kq && s_pos[x] > pq)) ? 1u : 0u;
+      }
+      for (u32 x = q + 1; x < m; ++x) {
+        const u64 o = s_key[x];
+        if (sc(o) != f) break;
+        to += (o < kq || (o == kq && s_pos[x] < pq)) ? 1u : 0u;
+      }
+      kout[first + to] = kq;
+      iout[first + to] = s_id[pq];
     }
     return;
   }
@@ -677,15 +747,10 @@ k_seg_sort(const u64* kin, const u64* iin, u64* kout, u64* iout, u32 n, const Se
       }
       __syncthreads();
     }
-  for (u32 j = threadIdx.x; j < m; j += kSegBlock) kout[first + j] = s_key[j];
-  __syncthreads();
-#pragma unroll
-  for (int k = 0; k < kSegItems; ++k) {
-    const u32 j = threadIdx.x + k * kSegBlock;
-    if (j < m) s_key[j] = id[k];
+  for (u32 j = threadIdx.x; j < m; j += kSegBlock) {
+    kout[first + j] = s_key[j];
+    iout[first + j] = s_id[s_pos[j]];
   }
-  __syncthreads();
-  for (u32 j = threadIdx.x; j < m; j += kSegBlock) iout[first + j] = s_key[s_pos[j]];
 }
 
 // ---------------------------------------------------------------------------
@@ -766,7 +831,7 @@ static cudaError_t sort_pass_attrs() {
 template <int DB, typename SW, bool MSD = false>
 static void sort_pass_launch(bool bulk, unsigned tiles, cudaStream_t st, const u64* ka, const u64* ia, u64* kb,
                              u64* ib, u64 n, int shift, const u64* excl, SW* status, u32* ticket, u32* errw,
-                             const u64* scale = nullptr) {
+                             const SegCtl* scale = nullptr) {
   if (bulk)
     k_sort_pass<DB, true, SW, MSD><<<tiles, kSortBlock, PassLayout<DB>::kSmem, st>>>(ka, ia, kb, ib, n, shift, scale,
                                                                                      excl, status, ticket, errw);
@@ -890,14 +955,6 @@ extern "C" int cf_sort_pairs_digits(u64* keys, u64* ids, u64 n, int key_bits, in
                     cf_sort_digits_tmp_bytes(n, key_bits, digit_bits), (cudaStream_t)stream);
 }
 
-// Bits T of the scaled key that the onesweep passes sort: segments of 1,500 to 3,000 records.
-static int seg_bits(u64 n) {
-  int T = 0;
-  while (T < 18 && (n >> T) > 3000) ++T;
-  return T;
-}
-constexpr u64 kSegMaxN = 3000ull << 18;                // 7.9e8: two 9-bit digits
-
 // Workspace of cf_sort_pairs_to for n records.
 extern "C" size_t cf_sort_to_tmp_bytes(u64 n) {
   const size_t lsd = sort_tmp_bytes(n, kMaxPasses, 8), lsd9 = sort_tmp_bytes(n, sort_passes(64, 9), 9);
@@ -906,7 +963,7 @@ extern "C" size_t cf_sort_to_tmp_bytes(u64 n) {
 
 // Stable sort of (kin, iin)[n] by key into (kout, iout), which must not overlap the inputs; the
 // inputs are left as they are.  digit_bits (8 or 9): the digit width of the LSD sort that takes the
-// sides the segment sort does not (above 7.9e8 records, or a segment above 4096 records).
+// sides the segment sort does not (above 8.9e8 records, or a segment above 4096 records).
 // Synchronises the stream once at the end (twice where the LSD sort runs).
 extern "C" int cf_sort_pairs_to(const u64* kin, const u64* iin, u64* kout, u64* iout, u64 n, int digit_bits, void* tmp,
                                 size_t tmp_bytes, void* stream) {
@@ -929,8 +986,9 @@ extern "C" int cf_sort_pairs_to(const u64* kin, const u64* iin, u64* kout, u64* 
   const u64 *src_k = kin, *src_i = iin;
   u32 max_seg = ~0u, herr = 0;
   if (n <= kSegMaxN) {
-    const int T = seg_bits(n), np = T <= 9 ? 1 : 2;
-    const int db = (np == 1 ? T : (T + 1) / 2) <= 8 ? 8 : 9, bins = 1 << db;
+    const u32 segs = (u32)((n + kSegMean - 1) / kSegMean);
+    const int np = segs <= 512 ? 1 : 2, db = segs <= 256 || (np == 2 && segs <= 65536) ? 8 : 9, bins = 1 << db;
+    const bool front = n <= kSegFrontMax;              // segs <= 20
     const u64 tiles = (n + kSortTile - 1) / kSortTile;
     // workspace: second buffers, then the zeroed control words, histograms and status words
     unsigned char* w = (unsigned char*)tmp;
@@ -943,15 +1001,21 @@ extern "C" int cf_sort_pairs_to(const u64* kin, const u64* iin, u64* kout, u64* 
     u32* status = (u32*)w; w += (size_t)np * tiles * bins * 4;
     const size_t zeroed = (size_t)(w - (unsigned char*)ctl);
     u64* excl = (u64*)(((uintptr_t)w + 7) & ~(uintptr_t)7); w = (unsigned char*)(excl + (size_t)np * bins);
-    u32* starts = (u32*)w; w += ((size_t)4 << T) + 4;
+    u32* starts = (u32*)w; w += (size_t)4 * segs + 4;
     if ((size_t)(w - (unsigned char*)tmp) > tmp_bytes) { cf_set_error("cf_sort_pairs_to: workspace too small%s", ""); return CF_ENOMEM; }
     e = db == 8 ? sort_pass_attrs<8, u32, true>() : sort_pass_attrs<9, u32, true>();
     if (e == cudaSuccess) e = cudaMemsetAsync(ctl, 0, zeroed, st);
     if (e != cudaSuccess) return cf_cuda_status(e, "cf_sort_pairs_to: set-up");
     const unsigned g = (unsigned)((n + 4095) / 4096), gm = g < 148 * 4 ? g : 148 * 4;
-    k_seg_max<<<gm, 512, 0, st>>>(kin, n, T + kSegBits, ctl);
-    k_seg_hist<<<gm, 512, 0, st>>>(kin, n, ctl, hist, np, db);
-    k_sort_hist_scan<<<1, 32 * np, 0, st>>>(hist, excl, db);
+    if (front) {
+      k_seg_front<<<1, 1024, 0, st>>>(kin, (u32)n, segs, ctl, excl, starts);
+    } else {
+      // keys that fit L2 are read whole: the histogram and the first pass then find them there
+      // (7.6e6 records: 403 us against 414 with a sample; 2^26: 2.67 ms with a sample, 2.78 without)
+      k_seg_max<<<gm, 512, 0, st>>>(kin, n, n >= (1u << 23) ? 64 : 1, segs, ctl);
+      k_seg_hist<<<gm, 512, 0, st>>>(kin, n, ctl, hist, np, db);
+      k_sort_hist_scan<<<1, 32 * np, 0, st>>>(hist, excl, db);
+    }
     for (int p = 0; p < np; ++p) {
       const u64 *ka = p ? k2 : kin, *ia = p ? i2 : iin;
       u64 *kb = p + 1 == np ? kout : k2, *ib = p + 1 == np ? iout : i2;
@@ -960,13 +1024,13 @@ extern "C" int cf_sort_pairs_to(const u64* kin, const u64* iin, u64* kout, u64* 
       u32* pst = status + (size_t)p * tiles * bins;
       if (db == 8)
         sort_pass_launch<8, u32, true>(bulk, (unsigned)tiles, st, ka, ia, kb, ib, n, shift, excl + p * bins, pst,
-                                       ctl->tickets + p, errw, &ctl->scale);
+                                       ctl->tickets + p, errw, ctl);
       else
         sort_pass_launch<9, u32, true>(bulk, (unsigned)tiles, st, ka, ia, kb, ib, n, shift, excl + p * bins, pst,
-                                       ctl->tickets + p, errw, &ctl->scale);
+                                       ctl->tickets + p, errw, ctl);
     }
-    k_seg_bounds<<<((1u << T) + 256) / 256, 256, 0, st>>>(kout, (u32)n, T, ctl, starts);
-    k_seg_sort<<<1u << T, kSegBlock, kSegSmem, st>>>(kout, iout, kout, iout, (u32)n, ctl, starts);
+    if (!front) k_seg_bounds<<<segs / 256 + 1, 256, 0, st>>>(kout, (u32)n, segs, ctl, starts);
+    k_seg_sort<<<segs, kSegBlock, kSegSmem, st>>>(kout, iout, kout, iout, (u32)n, ctl, starts);
     CF_LAUNCH_CHECK("cf_sort_pairs_to: segments");
     SegCtl h[2];                                       // control words and, after them, the error word
     e = cudaMemcpyAsync(h, ctl, sizeof(SegCtl) + 4, cudaMemcpyDeviceToHost, st);

@@ -34,7 +34,7 @@ def keys_of(kind, n, rng):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("kind", ["uniform", "full", "small", "equal", "zero", "clusters", "skewed", "descending"])
-@pytest.mark.parametrize("n", [2, 33, CAP - 1, CAP, CAP + 1, 20_003, 3000 * 256 + 1, 3000 * 512, 3000 * 512 + 1, 5_000_011])
+@pytest.mark.parametrize("n", [2, 33, CAP - 1, CAP, CAP + 1, 20_003, 65_536, 65_537, 3400 * 256, 3400 * 256 + 1, 3400 * 512 + 1, 5_000_011])
 def test_sort_side_equals_numpy_stable_sort(cuda, kind, n):
     import torch
     rng = np.random.default_rng(n)
