@@ -147,8 +147,96 @@ class BoundedSolve:
 
     def solve(self, inst, verify: bool = True):
         Icap, Dmin = caps(inst)
-        pairs, nD, nI, plan = self._join(inst, Icap, Dmin, None, None)
+        got = None
+        if self.s.tuning.class_join and 3 <= inst.r <= 8:
+            with self.torch.cuda.stream(self.s._torch_stream()):
+                got = self._join_class(inst, Icap, Dmin)
+        pairs, nD, nI, plan = got or self._join(inst, Icap, Dmin, None, None)
         return self._finish(inst, pairs, nD, nI, plan, verify)
+
+    # The class join takes a record of the unpruned sides in about a tenth of a leaf's time with its share
+    # of the levels (k = 76, r = 6: 16.5 ms for 4.8e9 records against 124 ms for 4.4e9 leaves).
+    CLASS_RATIO = 8
+    CLASS_MIN = 1 << 22           # unpruned records of both sides: below, the level loop is as fast
+
+    def _join_class(self, inst, Icap, Dmin):
+        """The bounded join through the class join of the unpruned sides: every equal-residue pair, those
+        inside the bounds kept, and the exact sizes of the bounded sides counted (cf_bounded_count).
+        Primes that no bounded subset holds leave the pools first.  None where the bounds leave less
+        than 1/CLASS_RATIO of what remains, or the class join does not apply.
+
+    XXMEAS"""
+        from .solve import RESULT_DTYPE, Instance
+        lib, dp, s = self.lib, _lib.ptr, self.s
+        r, M = inst.r, inst.M
+        if Icap <= 1 or Dmin >= U128:
+            return None
+        small, large = math.prod(inst.INS[:r - 1]), math.prod(inst.B0[-(r - 1):])
+        INS = [q for x, q in enumerate(inst.INS) if x < r or q * small < Icap]
+        skip = next((x for x in range(len(inst.B0) - r) if inst.B0[x] * large >= Dmin), len(inst.B0) - r)
+        B0 = inst.B0[skip:]
+        total = math.comb(len(B0), r) + math.comb(len(INS), r)
+        if total < self.CLASS_MIN or math.comb(max(len(B0), len(INS)), r - 3) >> 32:
+            return None
+        sub = Instance(M, list(B0), INS, r, inst.B, inst.P0)
+        nD, nI = math.comb(len(B0), r), math.comb(len(INS), r)
+        plan = s.plan(nD, nI)
+        if min(nD, nI) >= RANK_LIMIT or max(nD, nI) < s.tuning.class_min_probe:
+            return None
+        plan.update(strategy="fused", i_limit=None, i_lo=0)
+        cp = s._class_plan(sub, plan)
+        if cp is None:
+            return None
+        multD = pow(inst.P0, -1, M)
+        poolD, poolI = s.tables.pool(B0, r, M, multD), s.tables.pool(INS, r, M, 1)
+        G = s.tables.get(("bcountG", tuple(B0), r, Dmin), lambda: self._bound_table(lib.cf_ddump_bounds, B0, r, Dmin))
+        H = s.tables.get(("bcountH", tuple(INS), r, Icap), lambda: self._bound_table(lib.cf_igen_bounds, INS, r, Icap))
+        misc = s._buf("bctr", 64)[:64]
+        misc.zero_()
+        sh, base = s._sh(), dp(misc)
+        _lib.check(lib.cf_bounded_count(1, dp(poolD), dp(G), len(B0), r, base + 16, sh), "cf_bounded_count(D)")
+        _lib.check(lib.cf_bounded_count(0, dp(poolI), dp(H), len(INS), r, base + 24, sh), "cf_bounded_count(I)")
+        bD, bI = misc[16:32].cpu().numpy().view(np.uint64).tolist()
+        if (bD + bI) * self.CLASS_RATIO < total:
+            return None
+        out = dict(strategy="bounded", Icap=Icap, Dmin=Dmin, table="class", class_plan=cp)
+        if bD == 0 or bI == 0:
+            return [], bD, bI, out
+        _ok, d, mp, _phi = np.frombuffer(cp, dtype=np.uint32, count=4, offset=8).tolist()
+        ws_bytes = int(np.frombuffer(cp, dtype=np.uint64, count=1, offset=24)[0])
+        ws = s._buf("class", ws_bytes)
+        maxp = max(s.tuning.pair_capacity, min(1 << 22, 1 << (8 * nD * nI // M).bit_length()))
+        screen = s.tables.screen(inst.P0, 1, 1e-6)     # no pair passes: the check only turns ranks into indices
+        while True:
+            pairs = s._buf("pairs", maxp * 16)
+            res = s._buf("res", maxp * s.result_bytes)
+            misc[:8].zero_()
+            _lib.check(lib.cf_class_join(cp, dp(poolD), dp(poolI), multD % mp, multD % d, dp(ws), ws_bytes, dp(pairs),
+                                         maxp, base, base + 4, None, sh), "cf_class_join")
+            _lib.check(lib.cf_check_pairs(dp(poolD), dp(poolI), dp(screen), r, dp(pairs), base, maxp, dp(res),
+                                          base + 4, sh), "cf_check_pairs")
+            self.gen.launches += 10
+            npairs, err = misc[:8].cpu().numpy().view(np.uint32).tolist()
+            if err & _lib.ERR_PART_OVERFLOW:
+                return None                           # a survivor list ran out
+            if err & _lib.ERR_PAIR_OVERFLOW:
+                maxp = max(2 * maxp, npairs + 16)
+                continue
+            if err:
+                raise _lib.CfError(_lib.CF_EBADARG, "bounded", f"class join failed (err {err:#x})")
+            break
+        if npairs == 0:
+            return [], bD, bI, out
+        rows = np.frombuffer(res[: npairs * s.result_bytes].cpu().numpy().tobytes(), dtype=RESULT_DTYPE)
+        di, ii = rows["d_idx"][:, :r].astype(np.int64), rows["i_idx"][:, :r].astype(np.int64)
+        keep = _inside(di, B0, lambda p: p >= Dmin, math.log2(max(Dmin, 1)), 1) \
+            & _inside(ii, INS, lambda p: p < Icap, math.log2(Icap), -1)
+        di, ii = di[keep] + skip, ii[keep]
+        got = list(zip(map(tuple, di.tolist()), map(tuple, ii.tolist())))
+        if wide_modulus(M):                            # keys were compared mod 2^64
+            got = [(x, y) for x, y in got
+                   if (inst.P0 * math.prod(inst.INS[q] for q in y) - math.prod(inst.B0[q] for q in x)) % M == 0]
+        return got, bD, bI, out
 
     def _join(self, inst, Icap, Dmin, split, hmax):
         # the producers launch, fill and upload on the current stream: make it the solver's
@@ -361,6 +449,16 @@ class BoundedSolve:
         pairs_out.sort()
         return SolveResult(hits, nD, nI, len(pairs_out), screened, above, rejected, plan=plan, pairs=pairs_out,
                            launches=self.gen.launches)
+
+
+def _inside(idx, primes, exact, lg_bound: float, sign: int) -> np.ndarray:
+    """Rows of idx whose product of primes is inside a bound: by log2 where the margin is clear (far
+    above the rounding of a sum of 8 logarithms), by exact integers near it."""
+    lg = np.log2(np.asarray(primes, dtype=np.float64))[idx].sum(axis=1) - lg_bound
+    keep = lg * sign > 0
+    for k in np.nonzero(np.abs(lg) < 1e-6)[0].tolist():
+        keep[k] = exact(math.prod(primes[x] for x in idx[k].tolist()))
+    return keep
 
 
 def _confirmed_pairs(dd_all, ii_all, dkeys, INS, P0m: int, M: int) -> list:

@@ -84,6 +84,21 @@ def _dtab_bytes(n: int, tu: Tuning) -> int:
     return (164 << bb) + ((32 << fb) if fb else 0)
 
 
+def _class_bytes(inst: Instance, tu: Tuning) -> int:
+    """Device bytes of the instance's class join (its whole sides), 0 where it does not apply."""
+    import numpy as np
+    from . import _lib
+    from .tables import split_modulus
+    nD, nI = math.comb(len(inst.B0), inst.r), math.comb(len(inst.INS), inst.r)
+    if not tu.class_join or not nD or not nI or max(nD, nI) < tu.class_min_probe:
+        return 0
+    lib = _lib.load()
+    out = np.zeros(lib.cf_class_plan_bytes(), dtype=np.uint8)
+    _lib.check(lib.cf_class_plan(split_modulus(inst.M)[0], len(inst.B0), len(inst.INS), inst.r, 0, min(nI, 2 ** 64 - 1),
+                                 int(nI < nD), out.ctypes.data, out.nbytes), "cf_class_plan")
+    return int(out[24:32].view(np.uint64)[0]) if out[8:12].view(np.uint32)[0] else 0
+
+
 def footprint(inst: Instance, tu: Tuning) -> dict:
     """Upper bound on the device bytes one solve of `inst` holds at once, and the
     strategy it will use ('bounded' or 'fused')."""
@@ -104,10 +119,11 @@ def footprint(inst: Instance, tu: Tuning) -> dict:
         # most min(nI, nD) of them) or on the D records (I leaves probed, never written)
         m = min(nI, nD)
         side = max(16 * m + _dtab_bytes(m, tu), _dtab_bytes(nD, tu))
-        return dict(bytes=fixed + 16 * nD + frontier * 2 + side, strategy="bounded", nD=nD, nI=nI, work=nD + nI)
+        need = max(16 * nD + frontier * 2 + side, _class_bytes(inst, tu))
+        return dict(bytes=fixed + need, strategy="bounded", nD=nD, nI=nI, work=nD + nI)
     small = min(math.comb(nB, r), math.comb(nI_full, r))
     tails = 16 * (math.comb(nB, 2) + math.comb(nI_full, 2))
-    return dict(bytes=fixed + _dtab_bytes(small, tu) + tails, strategy="fused",
+    return dict(bytes=fixed + max(_dtab_bytes(small, tu) + tails, _class_bytes(inst, tu)), strategy="fused",
                 work=math.comb(nB, r) + math.comb(nI_full, r))
 
 

@@ -278,6 +278,11 @@ int cf_igen_count(const void* pool_dev, const void* bounds_dev, uint64_t M, uint
 int cf_igen_write(const void* pool_dev, int n, int r, int split_idx, const void* tmp, const void* state,
                   uint64_t c0, uint64_t cc, uint64_t* keys, uint64_t* ids, void* stream);
 
+/* Exact size of a product-bounded side without its records: *out (device u64, zeroed by the caller)
+ * += the r-subsets with a product below Icap (side 0, a cf_igen_bounds table) or of at least Dmin
+ * (side 1, a cf_ddump_bounds table); 3 <= r <= 16. */
+int cf_bounded_count(int side, const void* pool, const void* bounds, int n, int r, uint64_t* out, void* stream);
+
 /* One product-bounded exchange instance in one call (the device part of the
  * reference driver's run_instance, gpu/mitm_gpu_mstar_driver.py:184-286):
  * cf_ddump_bounds computes the D side's bound table G (exact 128-bit,
