@@ -80,6 +80,10 @@ SIGNATURES = [
     ("cf_class_plan_bytes", sz, []),
     ("cf_class_plan", C.c_int, [u64, C.c_int, C.c_int, C.c_int, u64, u64, C.c_int, vp, sz]),
     ("cf_class_join", C.c_int, [vp, vp, vp, u32, u32, vp, sz, vp, u32, vp, vp, vp, vp]),
+    ("cf_solve_desc_bytes", sz, []),
+    ("cf_solve_table_bytes", sz, [C.c_int, C.c_int, C.c_int]),
+    ("cf_solve_tail_bytes", sz, [C.c_int, C.c_int, C.c_int]),
+    ("cf_solve", C.c_int, [vp, vp]),
     ("cf_pair_result_bytes", sz, []),
     ("cf_check_pairs", C.c_int, [vp, vp, vp, C.c_int, vp, vp, u32, vp, vp, vp]),
     ("cf_scan_tmp_bytes", sz, [u64]),
@@ -130,6 +134,18 @@ SIGNATURES = [
     ("cf_merge_run_bytes", sz, []),
     ("cf_merge_join_runs", C.c_int, [vp, u64, vp, u64, vp, u64, vp, vp, vp, vp]),
 ]
+
+class CfSolve(C.Structure):
+    """One fused solve for cf_solve (include/cfmitm.h)."""
+    _fields_ = [("primesD", vp), ("primesI", vp), ("m", u64), ("multD_odd", u64), ("multD_2", u64), ("n_D", u64),
+                ("i_lo", u64), ("n_I", u64), ("limbsB", vp), ("lgP0", C.c_double), ("lgB", C.c_double),
+                ("eps", C.c_double), ("class_plan", vp), ("stage", vp), ("tables", vp), ("tails", vp), ("ws", vp),
+                ("tails_bytes", u64), ("ws_bytes", u64), ("pairs", vp), ("results", vp), ("misc", vp),
+                ("readback", vp), ("events", vp * 4), ("multD_mp", u32), ("multD_d", u32), ("max_pairs", u32),
+                ("rows", u32), ("fused_grid", u32), ("nlimbs", C.c_int), ("nD", C.c_int), ("nI", C.c_int),
+                ("r", C.c_int), ("a", C.c_int), ("swap", C.c_int), ("bbits", C.c_int), ("fbits", C.c_int),
+                ("side_format", C.c_int)]
+
 
 class CfBatchQueue(C.Structure):
     """include/cfmitm.h CfBatchQueue: one prepared batch for cf_solve_batch."""

@@ -21,6 +21,7 @@ certification of every hit by ``certify.verify_certificate``.
 """
 from __future__ import annotations
 
+import ctypes as C
 import math
 from dataclasses import dataclass, field
 
@@ -243,6 +244,8 @@ def finish_rows(inst: Instance, res: np.ndarray, nD: int, nI: int, plan: dict, v
 class Solver:
     """Reusable device state for repeated solves on one device and stream."""
 
+    READBACK_ROWS = 256
+
     def __init__(self, device=None, stream=None, tuning: Tuning | None = None):
         import torch
         self.torch = torch
@@ -254,6 +257,7 @@ class Solver:
         self.tuning = tuning or Tuning()
         self.tables = DeviceTables(self.device, stream=stream, async_upload=True)
         self._bufs: dict[str, object] = {}
+        self._rows = self.READBACK_ROWS  # checked rows that come back with a solve's counters
         self._bufset = 0                 # which of two buffer sets the next enqueue uses (solve_many)
         self.d2h_bytes = 0               # bytes read back from the device by collect()
         self._pinned: dict = {}
@@ -266,6 +270,8 @@ class Solver:
         key = (name, self._bufset)
         t = self._bufs.get(key)
         if t is None or t.numel() < nbytes:
+            if t is not None:                  # a growing buffer grows by half at least: few reallocations in a list
+                nbytes = max(nbytes, t.numel() * 3 // 2)
             t = self.torch.empty(max(nbytes, 16), dtype=self.torch.uint8, device=self.device)
             self._bufs[key] = t
         return t
@@ -314,9 +320,9 @@ class Solver:
         """Queue the whole device pipeline for `inst` on the stream (no host sync).
         `marks` (optional list) receives (tag, CUDA event) pairs around every kernel."""
         if plan.get("strategy", "fused") == "fused":
-            if plan.get("class_plan"):
-                return self._enqueue_class(inst, plan, marks)
-            return self._enqueue_fused(inst, plan, marks)
+            pshape = self._part_shape(inst, plan)
+            return self._enqueue_solve(inst, plan, marks) if pshape is None \
+                else self._enqueue_fused(inst, plan, pshape, marks)
         return self._enqueue_partition(inst, plan, marks)
 
     def _side_tables(self, inst: Instance, side: str):
@@ -332,8 +338,72 @@ class Solver:
         screen = self.tables.screen(inst.P0, inst.B, 1e-6)
         return poolD, poolI, tailD, tailI, screen
 
-    def _enqueue_fused(self, inst: Instance, plan: dict, marks: list | None):
-        """D table build, fused generate-and-probe of the I side, pair check."""
+    def _part_shape(self, inst: Instance, plan: dict) -> tuple | None:
+        """(bucket ranges, range capacity) of a table join with the partitioned build, else None."""
+        tu, lib = self.tuning, self.lib
+        nb = 1 << plan["bbits"]
+        if plan.get("class_plan") or not tu.part_build or plan.get("no_part") or nb < tu.part_min_buckets \
+                or inst.r > lib.cf_batch_max_r():
+            return None
+        nD, nIt = ncomb(len(inst.B0), inst.r), _i_window(inst, plan)
+        return part_shape(nIt if plan.get("swap") and nIt < nD else nD, plan["bbits"], tu.part_lb, tu.part_sigma,
+                          lib.cf_batch_part_max_ranges())
+
+    def _enqueue_solve(self, inst: Instance, plan: dict, marks: list | None):
+        """Class join, or table build in place and generate-and-probe, with tables, check and
+        read-back: one cf_solve call.  Table by table from Python, k = 29, r = 2 took 235 us a
+        solve against 184, and 24 portfolio moduli (11.0 ms against 8.3)"""
+        lib, dp = self.lib, _lib.ptr
+        r, M = inst.r, inst.M
+        if inst.B < 1 or inst.B.bit_length() > 2048:
+            raise ValueError("size bound B must be below 2^2048")
+        nD, nIt = ncomb(len(inst.B0), r), _i_window(inst, plan)
+        m, a = split_modulus(M)
+        multD = pow(inst.P0, -1, M)
+        cp = plan.get("class_plan")
+        pD, pI = np.array(inst.B0, dtype=np.uint64), np.array(inst.INS, dtype=np.uint64)
+        lb = np.frombuffer(inst.B.to_bytes((inst.B.bit_length() + 31) // 32 * 4, "little"), dtype=np.uint32)
+        q = _lib.CfSolve(primesD=pD.ctypes.data, primesI=pI.ctypes.data, m=m, multD_odd=multD % m,
+                         multD_2=multD & ((1 << a) - 1), n_D=nD, i_lo=_i_lo(plan), n_I=nIt, limbsB=lb.ctypes.data,
+                         nlimbs=len(lb), lgP0=math.log2(inst.P0), lgB=math.log2(inst.B), eps=1e-6, nD=len(pD),
+                         nI=len(pI), r=r, a=a, swap=int(bool(plan.get("swap")) and nIt < nD), bbits=plan["bbits"],
+                         fbits=plan.get("fbits", 0), fused_grid=self.tuning.fused_grid)
+        # in-place builds of tables of at most 2^20 buckets use compact side words (half the side area,
+        # L2-resident while built); larger tables the wide entries
+        q.side_format = 1 if q.bbits <= 20 else 0
+        tb = lib.cf_solve_table_bytes(len(pD), len(pI), r)
+        stage, tabs = self._pinned_buf("stage", tb), self._buf("tables", tb)
+        if cp:
+            _ok, d, mp, _phi = np.frombuffer(cp, dtype=np.uint32, count=4, offset=8).tolist()
+            q.class_plan = C.cast(C.c_char_p(cp), C.c_void_p)
+            q.multD_mp, q.multD_d = multD % mp, multD % d
+            q.ws_bytes = int(np.frombuffer(cp, dtype=np.uint64, count=1, offset=24)[0])
+            ws = self._buf("class", q.ws_bytes)
+        else:
+            q.ws_bytes = lib.cf_dtab_bytes2(q.bbits, q.fbits)
+            ws = self._buf("dtab", q.ws_bytes)
+            q.tails_bytes = lib.cf_solve_tail_bytes(len(pD), len(pI), r)
+            q.tails = dp(self._buf("tails", q.tails_bytes))
+        maxp = plan["pairs"]
+        rb = self.result_bytes
+        rows = max(0, min(self._rows, maxp))
+        pairs, res, ctr = self._buf("pairs", maxp * 16), self._buf("res", maxp * rb), self._buf("ctr", 64)
+        hm = self._pinned_buf("readback", 8 + rows * rb)
+        q.stage, q.tables, q.ws, q.pairs, q.results, q.misc = \
+            stage.data_ptr(), dp(tabs), dp(ws), dp(pairs), dp(res), dp(ctr)
+        q.max_pairs, q.rows, q.readback = maxp, rows, hm.data_ptr()
+        if marks is not None:
+            for j, tag in enumerate(("start", "gen_D", "probe", "check")):
+                self._mark(marks, tag)             # makes the event; cf_solve records it again in its place
+                q.events[j] = marks[-1][1].cuda_event
+        _lib.check(lib.cf_solve(C.byref(q), self._sh()), "cf_solve")
+        ev = self.torch.cuda.Event()
+        ev.record(self._torch_stream())
+        return dict(misc=ctr[:64].view(self.torch.int32), dcnt=None, icnt=None, res=res, nD=nD, nI=nIt, plan=plan,
+                    launches=9 if cp else 5, ev=ev, hread=hm, hrows=rows)
+
+    def _enqueue_fused(self, inst: Instance, plan: dict, pshape: tuple, marks: list | None):
+        """Table join with the partitioned build: D table, fused generate-and-probe, pair check."""
         torch, lib = self.torch, self.lib
         r = inst.r
         nD, nIt = ncomb(len(inst.B0), r), _i_window(inst, plan)
@@ -354,34 +424,17 @@ class Solver:
         tab[160 * nb: tbytes].zero_()              # fill counters and Bloom filter
         # build on the smaller side (swap: the table holds the I window and the D side probes)
         swap = bool(plan.get("swap")) and nIt < nD
-        bside, pside = ("I", "D") if swap else ("D", "I")
-        bn, bcount = (len(inst.INS), nIt) if swap else (len(inst.B0), nD)
+        pside = "D" if swap else "I"
         pn, pcount = (len(inst.B0), nD) if swap else (len(inst.INS), nIt)
-        tu = self.tuning
-        pshape = None
-        if tu.part_build and not plan.get("no_part") and nb >= tu.part_min_buckets and r <= lib.cf_batch_max_r():
-            pshape = part_shape(bcount, bbits, tu.part_lb, tu.part_sigma, lib.cf_batch_part_max_ranges())
-        # in-place builds of tables of at most 2^20 buckets use compact side words (half the side area,
-        # L2-resident while built); partitioned builds and larger tables the wide entries
-        side_format = 1 if pshape is None and bbits <= 20 else 0
         self._mark(marks, "start")
         ilo = _i_lo(plan)                          # first I rank of the window
-        if pshape is not None:
-            tables = self._tables_for(inst)
-            self._part_build(inst, plan, pshape, tables, tab, nD, nIt, swap, misc)
-            poolD, poolI, tailD, tailI, screen = tables
-            ppool, ptail = (poolD, tailD) if pside == "D" else (poolI, tailI)
-        else:
-            # the build side's tables first: the table build runs while the host prepares the other side
-            bpool, btail = self._side_tables(inst, bside)
-            ck(lib.cf_dtab_build3(dp(bpool), dp(btail), bn, r, ilo if swap else 0, bcount, dp(tab), bbits, fbits,
-                                  side_format, dp(misc) + 4, sh), "cf_dtab_build")
-            ppool, ptail = self._side_tables(inst, pside)
-            screen = self.tables.screen(inst.P0, inst.B, 1e-6)
-            poolD, poolI = (bpool, ppool) if bside == "D" else (ppool, bpool)
+        tables = self._tables_for(inst)
+        self._part_build(inst, plan, pshape, tables, tab, nD, nIt, swap, misc)
+        poolD, poolI, tailD, tailI, screen = tables
+        ppool, ptail = (poolD, tailD) if pside == "D" else (poolI, tailI)
         ppool, ptail = dp(ppool), dp(ptail)
         self._mark(marks, "gen_D")
-        ck(lib.cf_fused_probe3(ppool, ptail, pn, r, 0 if swap else ilo, pcount, dp(tab), bbits, fbits, side_format,
+        ck(lib.cf_fused_probe3(ppool, ptail, pn, r, 0 if swap else ilo, pcount, dp(tab), bbits, fbits, 0,
                                ilo if swap else 0, int(swap), dp(pairs), maxp, dp(misc), dp(misc) + 4,
                                self.tuning.fused_grid, sh), "cf_fused_probe")
         self._mark(marks, "probe")
@@ -398,43 +451,12 @@ class Solver:
         against 323; r = 4, 1.4e7 0.15 against 0.23."""
         tu, lib = self.tuning, self.lib
         nD, nI = ncomb(len(inst.B0), inst.r), _i_window(inst, plan)
-        if not tu.class_join or plan.get("no_class") or max(nD, nI) < tu.class_min_probe:
-            return None
+        if not tu.class_join or plan.get("no_class") or max(nD, nI) < tu.class_min_probe or not tu.l2_table_bytes:
+            return None                       # (no L2 for tables: the caller wants the table join's filter level)
         out = np.zeros(lib.cf_class_plan_bytes(), dtype=np.uint8)
         _lib.check(lib.cf_class_plan(split_modulus(inst.M)[0], len(inst.B0), len(inst.INS), inst.r, _i_lo(plan), nI,
                                      int(bool(plan.get("swap"))), out.ctypes.data, out.nbytes), "cf_class_plan")
         return out.tobytes() if out[8:12].view(np.uint32)[0] else None
-
-    def _enqueue_class(self, inst: Instance, plan: dict, marks: list | None):
-        """Class join (filters, probe, survivors resolved to equal-residue pairs), pair check."""
-        torch, lib = self.torch, self.lib
-        r = inst.r
-        cp = plan["class_plan"]
-        _ok, d, mp, _phi = np.frombuffer(cp, dtype=np.uint32, count=4, offset=8).tolist()
-        ws_bytes = int(np.frombuffer(cp, dtype=np.uint64, count=1, offset=24)[0])
-        ws = self._buf("class", ws_bytes)
-        ctr = self._buf("ctr", 64)
-        misc = ctr[:64].view(torch.int32)
-        maxp = plan["pairs"]
-        pairs = self._buf("pairs", maxp * 16)
-        res = self._buf("res", maxp * self.result_bytes)
-        sh, dp, ck = self._sh(), _lib.ptr, _lib.check
-        misc.zero_()
-        multD = pow(inst.P0, -1, inst.M)
-        poolD = self.tables.pool(inst.B0, r, inst.M, multD)
-        poolI = self.tables.pool(inst.INS, r, inst.M, 1)
-        screen = self.tables.screen(inst.P0, inst.B, 1e-6)
-        self._mark(marks, "start")
-        self._mark(marks, "gen_D")                 # recorded again by the join, after its filter build
-        built = marks[-1][1].cuda_event if marks is not None else None
-        ck(lib.cf_class_join(cp, dp(poolD), dp(poolI), multD % mp, multD % d, dp(ws), ws_bytes, dp(pairs), maxp,
-                             dp(misc), dp(misc) + 4, built, sh), "cf_class_join")
-        self._mark(marks, "probe")
-        ck(lib.cf_check_pairs(dp(poolD), dp(poolI), dp(screen), r, dp(pairs), dp(misc), maxp, dp(res),
-                              dp(misc) + 4, sh), "cf_check_pairs")
-        self._mark(marks, "check")
-        return dict(misc=misc, dcnt=None, icnt=None, res=res, nD=ncomb(len(inst.B0), r), nI=_i_window(inst, plan),
-                    plan=plan, launches=9)
 
     def _part_build(self, inst: Instance, plan: dict, pshape: tuple, tables: tuple, tab, nD: int, nIt: int,
                     swap: bool, misc):
@@ -587,9 +609,10 @@ class Solver:
     def _finish(self, inst: Instance, h: dict, res: np.ndarray, verify: bool) -> SolveResult:
         return finish_rows(inst, res, h["nD"], h["nI"], h["plan"], verify)
 
-    def _direct_plan(self, inst: Instance, i_limit: int | None, i_lo: int = 0) -> dict | None:
+    def _direct_plan(self, inst: Instance, i_limit: int | None, i_lo: int = 0, cp: bytes | None = None) -> dict | None:
         """The device plan of a fused or partition join of inst over the I ranks [i_lo, i_limit), or
-        None when inst takes another path (radius 0, the bounded strategy, an empty window)."""
+        None when inst takes another path (radius 0, the bounded strategy, an empty window).  cp: the
+        class plan of this instance and window where the caller has it."""
         if inst.r == 0:
             return None
         st = self.tuning.strategy
@@ -607,7 +630,7 @@ class Solver:
         if min(nD, nI) >= 1 << 32:        # ranks in the fused table are 32-bit
             plan["strategy"] = "partition"
         if plan["strategy"] == "fused":
-            plan["class_plan"] = self._class_plan(inst, plan)
+            plan["class_plan"] = cp or self._class_plan(inst, plan)
             if plan["class_plan"]:            # room for the pairs a modulus with few units has (8 nD nI / M)
                 plan["pairs"] = max(plan["pairs"], min(1 << 22, _pow2ceil(8 * nD * nI // inst.M)))
         return plan
@@ -674,6 +697,8 @@ class Solver:
         """Queue, behind a solve's kernels, the copy of its counters and of its first `rows`
         checked rows into page-locked memory, and an event after them: collect() then waits
         for this solve alone, not for work queued after it."""
+        if h.get("ev") is not None:                # cf_solve has queued it
+            return
         torch = self.torch
         rb = self.result_bytes
         rows = max(0, min(int(rows), int(h["plan"]["pairs"])))
@@ -689,14 +714,14 @@ class Solver:
 
     def solve_many(self, insts: list, verify: bool = True, marks_list: list | None = None,
                    i_limit: int | None = None, readback_rows: int = 256, streams: int = 2,
-                   i_lo: int = 0) -> list[SolveResult]:
+                   i_lo: int = 0, class_plans: list | None = None) -> list[SolveResult]:
         """Solve instances one after another, each with its own build, probe and check, while
         the host collects and certifies each one as the device runs the next: two buffer sets
         alternate, and every solve's counters and first checked rows come back behind its own
         kernels.  With streams = 2 the two buffer sets also have a CUDA stream each, so one
         solve's table build can run beside the previous solve's probe.  The results equal
         solve_instance's on each instance (i_lo, i_limit: the same I-rank window for every
-        instance).  marks_list (optional list) receives one marks list per instance (see
+        instance; class_plans: their class plans where the caller has them).  marks_list (optional list) receives one marks list per instance (see
         enqueue)."""
         torch = self.torch
         out: list = [None] * len(insts)
@@ -717,6 +742,7 @@ class Solver:
             return torch.cuda.stream(st)
 
         pending = None
+        self._rows = int(readback_rows)
         try:
             for i in range(len(insts) + 1):
                 cur = None
@@ -727,7 +753,7 @@ class Solver:
                         marks = []
                         marks_list.append(marks)
                     with use(i):                   # the set (and stream) the solve in flight does not use
-                        plan = self._direct_plan(inst, i_limit, i_lo)
+                        plan = self._direct_plan(inst, i_limit, i_lo, class_plans[i] if class_plans else None)
                         if plan is None:
                             out[i] = self.solve_instance(inst, verify=verify, marks=marks, i_limit=i_limit,
                                                          i_lo=i_lo)
@@ -747,6 +773,7 @@ class Solver:
                 pending = cur
         finally:
             self._bufset = 0
+            self._rows = self.READBACK_ROWS
             self.stream, self.tables.stream = saved
             for st in sts:
                 if st is not base:

@@ -218,6 +218,28 @@ int cf_class_join(const void* plan, const void* poolD, const void* poolI, uint32
                   void* ws, size_t ws_bytes, void* pairs, uint32_t max_pairs, uint32_t* npairs, uint32_t* err,
                   void* ev_built, void* stream);
 
+/* One fused solve in one call (csrc/cf_solve.cu): tables prepared into page-locked memory, uploaded,
+ * the table join (class_plan null: ws is the D table of bbits / fbits) or the class join (ws: its
+ * workspace) queued, the pairs checked, {npairs, err} and the first `rows` results copied to
+ * readback.  Nothing is waited for. */
+typedef struct CfSolve {
+  const uint64_t *primesD, *primesI;
+  uint64_t m, multD_odd, multD_2, n_D, i_lo, n_I;
+  const uint32_t* limbsB;
+  double lgP0, lgB, eps;
+  const void* class_plan;
+  void *stage, *tables, *tails, *ws;
+  uint64_t tails_bytes, ws_bytes;
+  void *pairs, *results, *misc, *readback;
+  void* events[4];
+  uint32_t multD_mp, multD_d, max_pairs, rows, fused_grid;
+  int nlimbs, nD, nI, r, a, swap, bbits, fbits, side_format;
+} CfSolve;
+size_t cf_solve_desc_bytes(void);
+size_t cf_solve_table_bytes(int nD, int nI, int r);
+size_t cf_solve_tail_bytes(int nD, int nI, int r);
+int cf_solve(const CfSolve* s, void* stream);
+
 /* Exact check of candidate pairs (lexicographic-rank ids): recomputed residues,
  * conservative fp64 log-size screen, exact size n <= B, Korselt, distinctness.
  * results[t] (cf_pair_result_bytes() each) for t < min(*npairs, max_pairs).
