@@ -112,3 +112,17 @@ def test_scaled_residues_of_equal_records_differ_by_at_most_one():
                 vs.append(((w >> 32) * s + ((w & 0xffffffff) * s >> 32)) & 0xffffffff)
             exact = (x << 32) // mp
             assert all(v in (exact, exact - 1) for v in vs), (mp, x, vs)
+
+
+@pytest.mark.gpu
+def test_portfolio_sends_moduli_to_the_class_join(cuda):
+    from carmichael_frontier_b200.portfolio import BatchSolver, BatchTuning
+    insts = [instance("2^46", 64, 100, 4), instance("2^51", 64, 40, 5), instance("2^43", 20, 30, 3), instance("2^46", 64, 90, 5)]
+    lim = 1 << 20
+    dt = Tuning(class_min_probe=1 << 18)
+    bs = BatchSolver(cuda, tuning=BatchTuning(dtab=dt))
+    prep = bs.prepare(insts, i_limit=lim)
+    assert sorted(prep.single) == [0, 1, 3] and [b.idx for b in prep.batches] == [[2]]
+    ref = [summary(x) for x in BatchSolver(cuda, tuning=BatchTuning(class_join=False)).solve(insts, i_limit=lim)]
+    for graphs in (False, True, True):
+        assert [summary(x) for x in bs.run(prep, graphs=graphs)] == ref
