@@ -165,7 +165,8 @@ class BoundedSolve:
         Primes that no bounded subset holds leave the pools first.  None where the bounds leave less
         than 1/CLASS_RATIO of what remains, or the class join does not apply.
 
-    XXMEAS"""
+        k = 76, r = 6, 1.4e8 D records, 4.3e9 I leaves: 124 ms as a level loop with leaf probes, 16.5 ms on
+        the device here (1.4 of it the counts); k = 78, r = 4, 1.4e6 and 2.6e7: 0.89 against 0.64 ms in all."""
         from .solve import RESULT_DTYPE, Instance
         lib, dp, s = self.lib, _lib.ptr, self.s
         r, M = inst.r, inst.M

@@ -149,7 +149,7 @@ k_bgen_expand(int d, int r, int n, u64 F, const u64* __restrict__ pool, const u6
   if (LEAF) {
     // wide: the packed residue (x mod m in Montgomery form) << a | x mod 2^a, taken mod 2^64
     okey[k] = wide ? (kk << md.a) | ((hd->x20 * (alo[p] * prime)) & md.mask2)
-                   : cf_key_to_canon(kk, md, hd->inv2a, hd->inv2aR);
+                   : cf_key_to_canon(kk, md);
     oid[k] = nid;
   } else {
     U128 A;

@@ -42,7 +42,7 @@ k_bgen_probe(int r, int n, u64 F, const u64* __restrict__ pool, const u64* __res
     while (p + 1 < F && offs[p + 1] <= c) ++p;  // consecutive leaves share or follow their parent
     const int x = (int)(xs[p] + (c - offs[p]));
     const u64 kk = cf_mul_key(key[p], pkey[x], md);
-    const u64 X = KEYFORM ? kk : cf_key_to_canon(kk, md, hd->inv2a, hd->inv2aR);
+    const u64 X = KEYFORM ? kk : cf_key_to_canon(kk, md);
     const u64 iid = id[p] + binom[(size_t)x * (r + 1) + r];      // colex: + C(x, r)
     if (tab.bloom) {
       const CfBloomKey bk = cf_bloom_key(X, 0u, tab.fbits);

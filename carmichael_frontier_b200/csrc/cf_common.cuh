@@ -171,15 +171,13 @@ CF_HD CfMod cf_mod_from_hdr(const CfPoolHdr* h) {
   return md;
 }
 
-// key -> canonical residue in [0, M) (Chinese remaindering of the Montgomery
-// odd part and the 2-adic part).
-CF_HD u64 cf_key_to_canon(u64 k, const CfMod& md, u64 inv2a, u64 inv2aR) {
-  const u64 X = k >> md.a;
-  const u64 x2 = k & md.mask2;
-  const u64 t = cf_redc_mul(X, inv2a, md.m, md.minv);    // x_m * 2^-a
-  const u64 s = cf_redc_mul(x2, inv2aR, md.m, md.minv);  // x_2 * 2^-a
-  const u64 q = (t >= s) ? (t - s) : (t + md.m - s);     // (x_m - x_2) * 2^-a mod m
-  return x2 + (q << md.a);
+// Canonical residue in [0, M) from x mod m (xm) and x mod 2^a (x2): x = xm + k m with k = (x2 - xm)
+// m^-1 mod 2^a, two low-word multiplies (M below 2^64, so k m + xm < M does not wrap).
+CF_HD u64 cf_crt(u64 xm, u64 x2, u64 m, u64 minv, u64 mask2) { return xm + (((x2 - xm) * minv) & mask2) * m; }
+
+// key (odd part in Montgomery form) -> canonical residue in [0, M).
+CF_HD u64 cf_key_to_canon(u64 k, const CfMod& md) {
+  return cf_crt(cf_redc_mul(k >> md.a, 1, md.m, md.minv), k & md.mask2, md.m, md.minv, md.mask2);
 }
 
 // Tail table entry: the product of one b-subset (b <= 3) of the pool, lexicographic

@@ -190,9 +190,7 @@ extern "C" u64 cf_canon_of(u64 M, u64 k) {
   if (host_mod_init(M, &h) != CF_OK) return ~0ull;
   CfMod md;
   md.m = h.m; md.minv = h.minv; md.mask2 = h.mask2; md.a = h.a;
-  const u64 inv2a = mod_pow((h.m + 1) / 2, (u64)h.a, h.m);
-  const u64 inv2aR = (u64)((u128)inv2a * h.Rm % h.m);
-  return cf_key_to_canon(k, md, inv2a, inv2aR);
+  return cf_key_to_canon(k, md);
 }
 
 extern "C" u64 cf_key_mul(u64 M, u64 kx, u64 ky) {

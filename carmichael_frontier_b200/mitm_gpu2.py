@@ -54,6 +54,9 @@ def _workspace(dev, name: str, nbytes: int):
     return t
 
 
+GEN_TAIL_MIN = 1 << 17        # records from which generate uses the pool's suffix table (a launch of 6 us to make)
+
+
 def generate(primes, r: int, M: int, mult: int = 1, bits: int = 10, lo: int = 0, hi=None, device=None):
     """Residue records for the r-combinations of `primes` with CNS rank in [lo, hi).
     Returns torch uint64 (keys, ids); ids pack r indices of `bits` bits each."""
@@ -76,8 +79,13 @@ def generate(primes, r: int, M: int, mult: int = 1, bits: int = 10, lo: int = 0,
         raise ValueError("M must be at least 2")
     pool = _dtables(dev).pool(primes, r, M, mult)
     lib = _lib.load()
-    _lib.check(lib.cf_gen_subsets(_lib.ptr(pool), n, r, lo, count, 0, bits, 1, _lib.ptr(keys), _lib.ptr(ids),
-                                  _lib.stream_handle()), "generate")
+    if r >= 3 and count >= GEN_TAIL_MIN and max(primes) < 1 << 31 and M % (1 << 33):
+        tail = _dtables(dev).tail(primes, r, M, mult, pool)
+        _lib.check(lib.cf_gen_subsets_tail(_lib.ptr(pool), _lib.ptr(tail), n, r, lo, count, 0, bits, 1, _lib.ptr(keys),
+                                           _lib.ptr(ids), _lib.stream_handle()), "generate")
+    else:
+        _lib.check(lib.cf_gen_subsets(_lib.ptr(pool), n, r, lo, count, 0, bits, 1, _lib.ptr(keys), _lib.ptr(ids),
+                                      _lib.stream_handle()), "generate")
     return keys, ids
 
 
