@@ -176,20 +176,44 @@ struct PassLayout {
 };
 
 // Control words of the segment sort (below) and its scaled key.
-struct SegCtl {            // zeroed before the sort
-  u64 scale;
+constexpr int kSegLog = 64 * 32;   // pieces of the logarithmic map: 32 per power of two
+struct SegCtl {            // zeroed before the sort, except where noted
+  u64 scale, max_key;
   u32 top;                 // 2^L NS - 1
-  u32 blocks_done, max_seg, tickets[2], pad;
-  u64 max_key;
+  u32 linear;              // 1: f = mulhi(key, scale); 0: f from the piecewise map
+  u32 blocks_done, max_seg, err, pad, tickets[2];
+  u32 hist[kSegLog];       // sampled keys per piece
+  u32 cdf[kSegLog + 1];    // (not zeroed) f at the start of each piece
 };
+// Piece of a key and its place in the piece, 20 bits.
+__device__ __forceinline__ u32 seg_piece(u64 key, u32& frac) {
+  const int z = __clzll((long long)(key | 1ull));
+  const u32 h = (u32)(((key | 1ull) << z) >> 32);
+  frac = (h >> 6) & 0xfffffu;
+  return ((u32)(63 - z) << 5) | ((h >> 26) & 31u);
+}
 struct SegScale {
   u64 s;
-  u32 top;
+  u32 top, linear;
+  const u32* cdf;
   __device__ __forceinline__ u32 operator()(u64 key) const {
-    const u64 f = __umul64hi(key, s);
-    return f < top ? (u32)f : top;
+    if (linear) {                                      // uniform over the launch
+      const u64 f = __umul64hi(key, s);
+      return f < top ? (u32)f : top;
+    }
+    u32 frac;
+    const u32 i = seg_piece(key, frac), c0 = __ldg(cdf + i), c1 = __ldg(cdf + i + 1);
+    return min(c0 + (u32)(((u64)(c1 - c0) * frac) >> 20), top);
   }
 };
+__device__ __forceinline__ SegScale seg_map(const SegCtl* c) {
+  SegScale r;
+  r.s = c->scale;
+  r.top = c->top;
+  r.linear = c->linear;
+  r.cdf = c->cdf;
+  return r;
+}
 
 // One onesweep pass over the DB-bit digit at bit `shift`.  Two CTAs per SM.  BULK:
 // the tile's keys and ids are brought into shared memory by two bulk copies at
@@ -234,7 +258,8 @@ k_sort_pass(const u64* __restrict__ kin, const u64* __restrict__ iin, u64* __res
     }
   }
   __syncthreads();
-  const SegScale sc = MSD ? SegScale{scale->scale, scale->top} : SegScale{0, 0};
+  SegScale sc{};
+  if constexpr (MSD) sc = seg_map(scale);
   const u32 tile = s_tile;
   const u64 base = (u64)tile * kSortTile;
   const u64 left = n - base;
@@ -442,35 +467,36 @@ k_sort_pass(const u64* __restrict__ kin, const u64* __restrict__ iin, u64* __res
 // (monotone in the key, even over the range for m the largest key, whatever its size) is sorted by
 // f >> L only, in one or two onesweep passes, which leaves NS segments of about 3,400 records in
 // order; each is then sorted in shared memory by one CTA: the low L bits of f are its bin (about
-// one record per bin), one atomic per record gives bin sizes and slots, and a record's place is its
+// 0.4 records per bin), one atomic per record gives bin sizes and slots, and a record's place is its
 // bin's start plus the records of the bin before it in (key, position) order.  A record moves 32
-// bytes per onesweep pass and 32 in the segment sort.  m is the largest of a sample of the keys; the
-// few above it share the last bin.
+// bytes per onesweep pass and 32 in the segment sort.
 //
-// A segment above kSegCap records (few distinct keys, or keys far from even) leaves the records as
+// Residues are even over [0, M) once products wrap; the D side's are not (products of few small
+// primes stay below M).  The keys are sampled by pieces of their logarithm (32 per power of two),
+// and where the sample is not even f runs through each piece by the piece's share of it.
+//
+// A segment above kSegCap records (few distinct keys, clusters) leaves the records as
 // the passes left them, a stable reordering, and the caller runs the LSD sort on that.
 // ---------------------------------------------------------------------------
 constexpr int kSegBlock = 512;
 constexpr int kSegItems = 8;
 constexpr int kSegCap = kSegBlock * kSegItems;         // 4096 records
 constexpr u64 kSegMean = 3400;                         // records per segment: 12 sigma below the capacity
-constexpr int kSegBits = 12;                           // L: bins of a segment, log2
+constexpr int kSegBits = 13;                           // L: bins of a segment, log2
 constexpr int kSegBins = 1 << kSegBits;
 constexpr int kSegBinMax = 32;                         // larger bins: the segment goes to the bitonic sort
-constexpr size_t kSegSmem = (size_t)kSegCap * 18 + (size_t)kSegBins * 4;
+constexpr size_t kSegSmem = (size_t)kSegCap * 20 + (size_t)kSegBins * 2;
 constexpr u32 kSegFrontMax = 1u << 16;                 // up to here one CTA samples, counts and scans
 constexpr u64 kSegMaxN = kSegMean << 18;               // 8.9e8: two 9-bit digits
 
-__device__ __forceinline__ SegScale seg_scale(u64 max_key, u32 segs) {
+__device__ __forceinline__ u64 seg_scale(u64 max_key, u32 segs) {   // S of the linear map
   const u64 d = max_key + 1, range = (u64)segs << kSegBits;
-  SegScale r;
-  r.top = (u32)(range - 1);
-  if (d == 0) r.s = range;                             // max = 2^64 - 1
-  else if (d <= range) r.s = ~0ull;                    // f = key - 1: below the range already
-  else r.s = (u64)(((unsigned __int128)range << 64) / d);
-  return r;
+  if (d == 0) return range;                            // max = 2^64 - 1
+  if (d <= range) return ~0ull;                        // f = key - 1: below the range already
+  return (u64)(((unsigned __int128)range << 64) / d);
 }
 
+template <int T>
 __device__ __forceinline__ u64 block_max(u64 m, u64* s_m) {
 #pragma unroll
   for (int o = 16; o; o >>= 1) {
@@ -480,33 +506,85 @@ __device__ __forceinline__ u64 block_max(u64 m, u64* s_m) {
   if ((threadIdx.x & 31) == 0) s_m[threadIdx.x >> 5] = m;
   __syncthreads();
   m = s_m[0];
-  for (u32 w = 1; w < blockDim.x / 32; ++w) m = s_m[w] > m ? s_m[w] : m;
+  for (u32 w = 1; w < T / 32; ++w) m = s_m[w] > m ? s_m[w] : m;
   __syncthreads();
   return m;
 }
 
-// Sampled maximum: one run of 32 keys of every 32 * step.
-__global__ void __launch_bounds__(512) k_seg_max(const u64* __restrict__ keys, u64 n, u32 step, u32 segs, SegCtl* ctl) {
+// The map of the sampled keys counted in h (shared memory, kSegLog pieces), by one CTA of T threads:
+// linear when every piece holds what even keys below the maximum would (within six deviations and a
+// twentieth), else piecewise, f rising by a piece's share of the sample over the piece.
+template <int T>
+__device__ __forceinline__ void seg_make_map(const u32* h, u64 max_key, u32 segs, SegCtl* ctl, u32* s_w) {
+  constexpr int P = kSegLog / T;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  u32 c[P], sum = 0;
+#pragma unroll
+  for (int q = 0; q < P; ++q) sum += c[q] = h[threadIdx.x * P + q];
+  u32 incl = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const u32 x = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += x;
+  }
+  if (lane == 31) s_w[wid] = incl;
+  __syncthreads();
+  u32 run = incl - sum, total = 0;
+  for (int w = 0; w < T / 32; ++w) {
+    if (w < wid) run += s_w[w];
+    total += s_w[w];
+  }
+  const u64 range = (u64)segs << kSegBits;
+  const float per = (float)total / ((float)max_key + 1.0f);
+  bool even = true;
+#pragma unroll
+  for (int q = 0; q < P; ++q) {
+    const u32 i = threadIdx.x * P + q;
+    ctl->cdf[i] = (u32)((u64)run * range / (total ? total : 1u));
+    run += c[q];
+    // keys [2^e (1 + j/32), 2^e (1 + (j+1)/32)) cut at the maximum
+    const float lo = ldexpf(1.0f + (float)(i & 31u) / 32.0f, (int)(i >> 5)), w = ldexpf(1.0f / 32.0f, (int)(i >> 5));
+    const float e = per * fminf(w, fmaxf(0.0f, (float)max_key + 1.0f - lo));
+    even = even && fabsf((float)c[q] - e) <= 0.05f * e + 6.0f * sqrtf(e) + 16.0f;
+  }
+  if (threadIdx.x == T - 1) ctl->cdf[kSegLog] = (u32)range;
+  const int lin = __syncthreads_and(even);
+  if (threadIdx.x == 0) {
+    ctl->scale = seg_scale(max_key, segs);
+    ctl->top = (u32)(range - 1);
+    ctl->linear = (u32)lin;
+  }
+}
+
+// Sampled keys (one run of 32 of every 32 * step): their maximum and pieces; the last CTA makes the map.
+__global__ void __launch_bounds__(512) k_seg_sample(const u64* __restrict__ keys, u64 n, u32 step, u32 segs, SegCtl* ctl) {
   __shared__ u64 s_m[16];
+  __shared__ u32 s_h[kSegLog], s_w[16], s_last;
+  for (int i = threadIdx.x; i < kSegLog; i += 512) s_h[i] = 0;
+  __syncthreads();
   u64 m = 0;
-  const u64 lanes = (u64)gridDim.x * blockDim.x;
-  for (u64 t = (u64)blockIdx.x * blockDim.x + threadIdx.x;; t += lanes) {
+  const u64 lanes = (u64)gridDim.x * 512;
+  for (u64 t = (u64)blockIdx.x * 512 + threadIdx.x;; t += lanes) {
     const u64 i = (t >> 5) * 32 * step + (t & 31);
     if (i >= n) break;
     const u64 k = keys[i];
     m = k > m ? k : m;
+    u32 frac;
+    atomicAdd(&s_h[seg_piece(k, frac)], 1u);
   }
-  m = block_max(m, s_m);
-  if (threadIdx.x == 0) {
-    atomicMax((unsigned long long*)&ctl->max_key, (unsigned long long)m);
-    __threadfence();
-    if (atomicAdd(&ctl->blocks_done, 1u) == gridDim.x - 1) {
-      __threadfence();
-      const SegScale sc = seg_scale(*(volatile u64*)&ctl->max_key, segs);
-      ctl->scale = sc.s;
-      ctl->top = sc.top;
-    }
-  }
+  m = block_max<512>(m, s_m);
+  for (int i = threadIdx.x; i < kSegLog; i += 512)
+    if (s_h[i]) atomicAdd(&ctl->hist[i], s_h[i]);
+  if (threadIdx.x == 0) atomicMax((unsigned long long*)&ctl->max_key, (unsigned long long)m);
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(&ctl->blocks_done, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  for (int i = threadIdx.x; i < kSegLog; i += 512) s_h[i] = __ldcg(&ctl->hist[i]);
+  __syncthreads();
+  seg_make_map<512>(s_h, __ldcg(&ctl->max_key), segs, ctl, s_w);
 }
 
 // Histograms of the one or two digits of f >> L: db low bits, then the rest.
@@ -516,7 +594,7 @@ k_seg_hist(const u64* __restrict__ keys, u64 n, const SegCtl* __restrict__ ctl, 
   const int bins = np << db;
   const u32 mask = (1u << db) - 1u;
   for (int i = threadIdx.x; i < bins; i += blockDim.x) s_h[i] = 0;
-  const SegScale sc{ctl->scale, ctl->top};
+  const SegScale sc = seg_map(ctl);
   __syncthreads();
   for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64)gridDim.x * blockDim.x) {
     const u32 v = sc(keys[i]) >> kSegBits;
@@ -528,26 +606,51 @@ k_seg_hist(const u64* __restrict__ keys, u64 n, const SegCtl* __restrict__ ctl, 
     if (s_h[i]) atomicAdd((unsigned long long*)&hist[i], (unsigned long long)s_h[i]);
 }
 
-// Up to kSegFrontMax records, one digit (segs <= 256): maximum, counts, offsets and starts in one CTA.
+// Up to kSegFrontMax records, one digit (segs <= 256): map, counts, offsets and starts in one CTA.
 __global__ void __launch_bounds__(1024)
 k_seg_front(const u64* __restrict__ keys, u32 n, u32 segs, SegCtl* __restrict__ ctl, u64* __restrict__ excl,
             u32* __restrict__ starts) {
   __shared__ u64 s_m[32];
-  __shared__ u32 s_h[256], s_w[8];
-  u64 m = 0;
-  for (u32 i = threadIdx.x; i < n; i += 4096)          // a quarter of the keys
-    m = keys[i] > m ? keys[i] : m;
+  __shared__ u32 s_l[kSegLog], s_h[256], s_w[32];
+  for (int i = threadIdx.x; i < kSegLog; i += 1024) s_l[i] = 0;
   if (threadIdx.x < 256) s_h[threadIdx.x] = 0;
-  m = block_max(m, s_m);
-  if (threadIdx.x == 0) {
-    const SegScale sc = seg_scale(m, segs);
-    ctl->scale = s_m[0] = sc.s;
-    ctl->top = sc.top;
+  __syncthreads();
+  u64 m = 0;
+#pragma unroll 8
+  for (u32 i = threadIdx.x; i < n; i += 1024) {
+    const u64 k = keys[i];
+    m = k > m ? k : m;
+    u32 frac;
+    atomicAdd(&s_l[seg_piece(k, frac)], 1u);
+  }
+  m = block_max<1024>(m, s_m);
+  seg_make_map<1024>(s_l, m, segs, ctl, s_w);
+  __threadfence_block();
+  __syncthreads();
+  SegScale sc{};
+  sc.s = *(volatile u64*)&ctl->scale;
+  sc.top = *(volatile u32*)&ctl->top;
+  sc.linear = *(volatile u32*)&ctl->linear;
+  for (int i = threadIdx.x; i <= kSegLog; i += 1024) {   // the pieces' starts, in shared memory
+    const u32 v = *(volatile u32*)&ctl->cdf[i];
+    if (i < kSegLog) s_l[i] = v;
   }
   __syncthreads();
-  const SegScale sc{s_m[0], (segs << kSegBits) - 1u};
+  const u32 end = (segs << kSegBits);
 #pragma unroll 8
-  for (u32 i = threadIdx.x; i < n; i += 1024) atomicAdd(&s_h[sc(keys[i]) >> kSegBits], 1u);
+  for (u32 i = threadIdx.x; i < n; i += 1024) {
+    const u64 k = keys[i];
+    u32 f;
+    if (sc.linear) {
+      const u64 g = __umul64hi(k, sc.s);
+      f = g < sc.top ? (u32)g : sc.top;
+    } else {
+      u32 frac;
+      const u32 q = seg_piece(k, frac), c0 = s_l[q], c1 = q + 1 < (u32)kSegLog ? s_l[q + 1] : end;
+      f = min(c0 + (u32)(((u64)(c1 - c0) * frac) >> 20), sc.top);
+    }
+    atomicAdd(&s_h[f >> kSegBits], 1u);
+  }
   __syncthreads();
   const int lane = threadIdx.x & 31;
   u32 v = 0, incl = 0;
@@ -575,7 +678,7 @@ k_seg_front(const u64* __restrict__ keys, u32 n, u32 segs, SegCtl* __restrict__ 
 __global__ void __launch_bounds__(256)
 k_seg_bounds(const u64* __restrict__ keys, u32 n, u32 segs, SegCtl* __restrict__ ctl, u32* __restrict__ starts) {
   const u32 s = blockIdx.x * blockDim.x + threadIdx.x;
-  const SegScale sc{ctl->scale, ctl->top};
+  const SegScale sc = seg_map(ctl);
   u32 lo = 0, hi = s < segs ? n : 0u, len = 0;
   while (lo < hi) {                                    // lower bound of segment s
     const u32 mid = (lo + hi) >> 1;
@@ -598,9 +701,10 @@ k_seg_bounds(const u64* __restrict__ keys, u32 n, u32 segs, SegCtl* __restrict__
   if ((threadIdx.x & 31) == 0 && len) atomicMax(&ctl->max_seg, len);
 }
 
-// Sort one segment by (key, position).  Bound by its chain of shared-memory phases (issue slots 45%
-// busy, L1 61%, DRAM a third): 2^26 records in 1.02 ms, 2.1 TB/s; the onesweep pass takes 0.71 ms for
-// the same records and the whole sort 2.67 ms (6.28 ms as eight LSD passes).  Two CTAs of 512 threads per SM (88 KB of shared memory, 64
+// Sort one segment by (key, position).  Bound by its chain of shared-memory phases, the neighbours'
+// comparisons above all: 2^26 records in 0.85 ms, 2.5 TB/s (0.95 ms with half the bins, 1.02 with the
+// bins recomputed from the keys); the onesweep pass takes 0.71 ms for the same records and the whole
+// sort 2.5 ms (6.28 ms as eight LSD passes).  Two CTAs of 512 threads per SM (98 KB of shared memory, 64
 // registers): while one loads or stores, the other ranks.  starts == nullptr: the whole array is one
 // segment (n <= kSegCap) and its largest key is found here.
 __global__ void __launch_bounds__(kSegBlock, 2)
@@ -610,7 +714,9 @@ k_seg_sort(const u64* kin, const u64* iin, u64* kout, u64* iout, u32 n, const Se
   u64* s_key = (u64*)smem;                             // [kSegCap] in bin order
   u64* s_id = s_key + kSegCap;                         // [kSegCap] ids in input order
   u16* s_pos = (u16*)(s_id + kSegCap);                 // [kSegCap] input position of s_key's record
-  u32* s_bin = (u32*)(s_pos + kSegCap);                // [kSegBins] sizes, then starts
+  u16* s_bid = s_pos + kSegCap;                        // [kSegCap] bin of s_key's record
+  u32* s_bin = (u32*)(s_bid + kSegCap);                // [kSegBins] sizes, then starts, two 16-bit halves a word
+  const u16* s_start = (const u16*)s_bin;
   __shared__ u32 s_w[kSegBlock / 32];
   __shared__ u64 s_m[kSegBlock / 32];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -629,32 +735,33 @@ k_seg_sort(const u64* kin, const u64* iin, u64* kout, u64* iout, u32 n, const Se
     const u32 j = threadIdx.x + k * kSegBlock;
     if (j < m) s_id[j] = iin[first + j];
   }
-  for (int i = threadIdx.x; i < kSegBins; i += kSegBlock) s_bin[i] = 0;
-  SegScale sc;
+  for (int i = threadIdx.x; i < kSegBins / 2; i += kSegBlock) s_bin[i] = 0;
+  SegScale sc{};
   if (starts) {
-    sc.s = ctl->scale;
-    sc.top = ctl->top;
+    sc = seg_map(ctl);
     __syncthreads();
   } else {
     u64 mx = 0;
 #pragma unroll
     for (int k = 0; k < kSegItems; ++k) mx = key[k] > mx ? key[k] : mx;
-    mx = block_max(mx, s_m);
-    if (threadIdx.x == 0) s_m[0] = seg_scale(mx, 1u).s;
+    mx = block_max<kSegBlock>(mx, s_m);
+    if (threadIdx.x == 0) s_m[0] = seg_scale(mx, 1u);
     __syncthreads();
     sc.s = s_m[0];
     sc.top = kSegBins - 1u;
+    sc.linear = 1;
   }
   u32 bs[kSegItems];                                   // bin << 16 | slot in the bin
 #pragma unroll
   for (int k = 0; k < kSegItems; ++k) {
     const u32 j = threadIdx.x + k * kSegBlock;
     const u32 b = sc(key[k]) & (kSegBins - 1u);
-    bs[k] = j < m ? (b << 16) | atomicAdd(&s_bin[b], 1u) : 0u;
+    const u32 sh = 16 * (b & 1u);
+    bs[k] = j < m ? (b << 16) | ((atomicAdd(&s_bin[b >> 1], 1u << sh) >> sh) & 0xffffu) : 0u;
   }
   __syncthreads();
-  // exclusive scan of the bin sizes, 8 bins per thread
-  constexpr int kPer = kSegBins / kSegBlock;
+  // exclusive scan of the bin sizes, 16 bins (8 words) per thread
+  constexpr int kPer = kSegBins / 2 / kSegBlock;
   u32 c[kPer], sum = 0, big = 0;
 #pragma unroll
   for (int q = 0; q < kPer; q += 4) {
@@ -663,8 +770,9 @@ k_seg_sort(const u64* kin, const u64* iin, u64* kout, u64* iout, u32 n, const Se
   }
 #pragma unroll
   for (int q = 0; q < kPer; ++q) {
-    big = max(big, c[q]);
-    sum += c[q];
+    const u32 lo = c[q] & 0xffffu, hi = c[q] >> 16;
+    big = max(big, max(lo, hi));
+    sum += lo + hi;
   }
   u32 incl = sum;
 #pragma unroll
@@ -679,9 +787,9 @@ k_seg_sort(const u64* kin, const u64* iin, u64* kout, u64* iout, u32 n, const Se
     for (int w = 0; w < wid; ++w) run += s_w[w];
 #pragma unroll
     for (int q = 0; q < kPer; ++q) {
-      const u32 v = c[q];
-      c[q] = run;
-      run += v;
+      const u32 lo = c[q] & 0xffffu, hi = c[q] >> 16;
+      c[q] = run | ((run + lo) << 16);
+      run += lo + hi;
     }
 #pragma unroll
     for (int q = 0; q < kPer; q += 4)
@@ -691,9 +799,10 @@ k_seg_sort(const u64* kin, const u64* iin, u64* kout, u64* iout, u32 n, const Se
     for (int k = 0; k < kSegItems; ++k) {
       const u32 j = threadIdx.x + k * kSegBlock;
       if (j < m) {
-        const u32 to = s_bin[bs[k] >> 16] + (bs[k] & 0xffffu);
+        const u32 to = s_start[bs[k] >> 16] + (bs[k] & 0xffffu);
         s_key[to] = key[k];
         s_pos[to] = (u16)j;
+        s_bid[to] = (u16)(bs[k] >> 16);
       }
     }
     __syncthreads();
@@ -704,16 +813,16 @@ k_seg_sort(const u64* kin, const u64* iin, u64* kout, u64* iout, u32 n, const Se
       const u32 q = threadIdx.x + k * kSegBlock;
       if (q >= m) continue;
       const u64 kq = s_key[q];
-      const u32 pq = s_pos[q], f = sc(kq);
+      const u32 pq = s_pos[q], f = s_bid[q];
       u32 to = q;
       for (u32 x = q; x-- > 0;) {
+        if (s_bid[x] != f) break;
         const u64 o = s_key[x];
-        if (sc(o) != f) break;
         to -= (o > kq || (o == kq && s_pos[x] > pq)) ? 1u : 0u;
       }
       for (u32 x = q + 1; x < m; ++x) {
+        if (s_bid[x] != f) break;
         const u64 o = s_key[x];
-        if (sc(o) != f) break;
         to += (o < kq || (o == kq && s_pos[x] < pq)) ? 1u : 0u;
       }
       kout[first + to] = kq;
@@ -1046,8 +1155,8 @@ extern "C" int cf_sort_pairs_to(const u64* kin, const u64* iin, u64* kout, u64* 
     const size_t side = (size_t)(n + (n & 1)) * 8;     // 16-byte aligned ids for the bulk copies
     u64* k2 = (u64*)w; w += side;
     u64* i2 = (u64*)w; w += side;
-    SegCtl* ctl = (SegCtl*)w; w += 256;
-    u32* errw = (u32*)(ctl + 1);
+    SegCtl* ctl = (SegCtl*)w; w += (sizeof(SegCtl) + 255) & ~(size_t)255;
+    u32* errw = &ctl->err;
     u64* hist = (u64*)w; w += (size_t)np * bins * 8;
     u32* status = (u32*)w; w += (size_t)np * tiles * bins * 4;
     const size_t zeroed = (size_t)(w - (unsigned char*)ctl);
@@ -1061,9 +1170,7 @@ extern "C" int cf_sort_pairs_to(const u64* kin, const u64* iin, u64* kout, u64* 
     if (front) {
       k_seg_front<<<1, 1024, 0, st>>>(kin, (u32)n, segs, ctl, excl, starts);
     } else {
-      // keys that fit L2 are read whole: the histogram and the first pass then find them there
-      // (7.6e6 records: 403 us against 414 with a sample; 2^26: 2.67 ms with a sample, 2.78 without)
-      k_seg_max<<<gm, 512, 0, st>>>(kin, n, n >= (1u << 23) ? 64 : 1, segs, ctl);
+      k_seg_sample<<<gm, 512, 0, st>>>(kin, n, n >= (1u << 23) ? 64 : n >= (1u << 18) ? 8 : 1, segs, ctl);
       k_seg_hist<<<gm, 512, 0, st>>>(kin, n, ctl, hist, np, db);
       k_sort_hist_scan<<<1, 32 * np, 0, st>>>(hist, excl, db);
     }
@@ -1083,12 +1190,13 @@ extern "C" int cf_sort_pairs_to(const u64* kin, const u64* iin, u64* kout, u64* 
     if (!front) k_seg_bounds<<<segs / 256 + 1, 256, 0, st>>>(kout, (u32)n, segs, ctl, starts);
     k_seg_sort<<<segs, kSegBlock, kSegSmem, st>>>(kout, iout, kout, iout, (u32)n, ctl, starts);
     CF_LAUNCH_CHECK("cf_sort_pairs_to: segments");
-    SegCtl h[2];                                       // control words and, after them, the error word
-    e = cudaMemcpyAsync(h, ctl, sizeof(SegCtl) + 4, cudaMemcpyDeviceToHost, st);
+    u32 h[2];                                          // largest segment, error word
+    static_assert(offsetof(SegCtl, err) == offsetof(SegCtl, max_seg) + 4, "read together");
+    e = cudaMemcpyAsync(h, &ctl->max_seg, 8, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return cf_cuda_status(e, "cf_sort_pairs_to: control words");
-    max_seg = h[0].max_seg;
-    memcpy(&herr, &h[1], 4);
+    max_seg = h[0];
+    herr = h[1];
     if (herr & CF_ERR_SPIN_LIMIT) { cf_set_error("cf_sort_pairs_to: look-back wait exceeded its limit%s", ""); return CF_ETIMEOUT; }
     if (max_seg <= (u32)kSegCap) return CF_OK;
     src_k = kout;                                      // ordered by the top bits, equal keys in input order

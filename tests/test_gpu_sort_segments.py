@@ -27,13 +27,16 @@ def keys_of(kind, n, rng):
         k = rng.integers(0, 1 << 20, n, dtype=np.uint64)
         k[0] = 1 << 62
         return k
+    if kind == "products":                   # products of a few primes: spread over many powers of two
+        return np.prod(rng.choice(np.array([3, 11, 29, 101, 331, 1009, 3001], dtype=np.uint64), (4, n)) +
+                       2 * rng.integers(0, 500, (4, n), dtype=np.uint64), axis=0)
     if kind == "descending":
         return np.arange(n, 0, -1, dtype=np.uint64) << np.uint64(7)
     raise ValueError(kind)
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("kind", ["uniform", "full", "small", "equal", "zero", "clusters", "skewed", "descending"])
+@pytest.mark.parametrize("kind", ["uniform", "full", "small", "equal", "zero", "clusters", "skewed", "products", "descending"])
 @pytest.mark.parametrize("n", [2, 33, CAP - 1, CAP, CAP + 1, 20_003, 65_536, 65_537, 3400 * 256, 3400 * 256 + 1, 3400 * 512 + 1, 5_000_011])
 def test_sort_side_equals_numpy_stable_sort(cuda, kind, n):
     import torch
