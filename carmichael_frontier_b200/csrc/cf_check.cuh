@@ -40,6 +40,28 @@ __device__ __forceinline__ void cf_big_mul(CfWarpBig& b, u32 q, int lane) {
   b.c1 = (u32)(t0 >> 32);
 }
 
+// cf_unrank_lex by a warp: 32 candidates of a position at a time.
+template <int R>
+__device__ __forceinline__ void cf_unrank_warp(u64 rank, int n, const u64* __restrict__ binom, int (&idx)[R], int lane) {
+  int start = 0;
+#pragma unroll
+  for (int pos = 0; pos < R - 1; ++pos) {
+    const int rem = R - pos - 1;
+    const u64 total = cf_binom(binom, R, n - start, rem + 1), Y = total - rank;
+    int lo = start;                               // largest c with C(n-c, rem+1) >= Y
+    for (int base = start; base <= n - 1 - rem; base += 32) {
+      const int c = base + lane;
+      const int k = __popc(__ballot_sync(0xffffffffu, c <= n - 1 - rem && cf_binom(binom, R, n - c, rem + 1) >= Y));
+      lo = k ? base + k - 1 : lo;
+      if (k < 32) break;
+    }
+    idx[pos] = lo;
+    rank -= total - cf_binom(binom, R, n - lo, rem + 1);
+    start = lo + 1;
+  }
+  idx[R - 1] = start + (int)rank;
+}
+
 // x-th prime of S = (B0 without the primes at di) and the primes at ii, x < nD; false: deleted.
 template <int R>
 __device__ __forceinline__ bool cf_in_base(const int (&di)[R], int x) {
@@ -75,8 +97,8 @@ __device__ __forceinline__ CfPairResult cf_check_warp(const u64* __restrict__ po
   out.r = R;
   for (int j = 0; j < CF_MAX_R; ++j) { out.d_idx[j] = 0; out.i_idx[j] = 0; }
   int di[R], ii[R];
-  cf_unrank_lex<R>(pr.d_id, nD, bD, di);
-  cf_unrank_lex<R>(pr.i_id, nI, bI, ii);
+  cf_unrank_warp<R>(pr.d_id, nD, bD, di, lane);
+  cf_unrank_warp<R>(pr.i_id, nI, bI, ii, lane);
   u64 kd, ki;
   if (fast) {
     CfElt32 eD, eI;

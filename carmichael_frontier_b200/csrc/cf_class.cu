@@ -76,11 +76,11 @@ struct CfClassPlan {
   u64 magic;
   u32 ok, d, mp, phi;      // ok: the class join applies; class modulus, filter modulus, classes
   u64 ws_bytes;            // workspace of cf_class_join
-  u32 r, swap, elems, pad0;
+  u32 r, swap, elems, run; // run: list elements per thread of k_cj_count
   u64 i_lo, i_n;
   u64 zero_bytes;
   u32 maxchunks, maxcands;
-  u64 oCtr, oBins, oHeads, oUnits, oInv, oRowBase, oRowTot, oTmp, oBm, oCmeta, oChunkV, oChunks, oList, oCands;
+  u64 oCtr, oBins, oHeads, oUnits, oInv, oRowBase, oRowTot, oRowCnt, oTmp, oBm, oCmeta, oChunkV, oChunks, oList, oCands;
   CjSide side[2];          // 0: build side, 1: probe side
 };
 
@@ -140,39 +140,61 @@ __device__ __forceinline__ bool cj_element(const CjArgs& a, u32 e, int& s, bool&
   return false;
 }
 
+// Next K-subset in lexicographic order.
+__device__ __forceinline__ void cj_next(int n, int K, int (&idx)[4]) {
+  int j = K - 1;
+#pragma unroll
+  for (int t = 3; t > 0; --t)
+    if (t == j && t < K && idx[t] == n - K + t) --j;
+#pragma unroll
+  for (int t = 0; t < 4; ++t) {
+    if (t == j) idx[t] += 1;
+    else if (t > j && t > 0 && t < K) idx[t] = idx[t - 1] + 1;
+  }
+}
+
+// A thread takes `run` consecutive elements and unranks the first only: 4 where the lists fill the GPU
+// all the same (6.4e5 elements: 21 us with runs of 1, 25 with 4; 3.5e6: 138 and 102).
 __global__ void __launch_bounds__(256) k_cj_count(const __grid_constant__ CjArgs a) {
   u32* bins = at<u32>(a, a.p.oBins);
   u32* t_bin = at<u32>(a, a.p.oTmp);
   u32 *t_pos = t_bin + a.p.elems, *t_x = t_pos + a.p.elems, *t_pk = t_x + a.p.elems;
-  for (u32 e = blockIdx.x * blockDim.x + threadIdx.x; e < a.p.elems; e += gridDim.x * blockDim.x) {
-    int s;
-    bool prefix;
-    u32 i;
-    if (!cj_element(a, e, s, prefix, i)) continue;
-    const CjSide& sd = a.p.side[s];
-    const u64* pool = a.pool[s];
-    const int K = (int)(prefix ? sd.A : sd.b);
+  const u32 runs = (a.p.elems + a.p.run - 1) / a.p.run;
+  for (u32 g = blockIdx.x * blockDim.x + threadIdx.x; g < runs; g += gridDim.x * blockDim.x) {
     int idx[4] = {0, 0, 0, 0};
-    cj_unrank(prefix ? sd.p_lo + i : (u64)i, (int)sd.n, pool + cf_pool_off_binom((int)sd.n), (int)sd.R + 1, K, idx);
-    const u64* pr = pool + cf_pool_off_prime((int)sd.n);
-    u64 x = prefix ? sd.mult_m : 1u;
-    u32 c = prefix ? sd.mult_d : 1u % a.p.d;
-    u32 pk = 0;
-    int last = 0;
+    int in = -1;                                   // list of the previous element: 2 * side + prefix
+#pragma unroll 1
+    for (u32 e = g * a.p.run; e < min(a.p.elems, (g + 1) * a.p.run); ++e) {
+      int s;
+      bool prefix;
+      u32 i;
+      if (!cj_element(a, e, s, prefix, i)) continue;
+      const CjSide& sd = a.p.side[s];
+      const u64* pool = a.pool[s];
+      const int K = (int)(prefix ? sd.A : sd.b), n = (int)sd.n;
+      if (in == 2 * s + (int)prefix) cj_next(n, K, idx);
+      else cj_unrank(prefix ? sd.p_lo + i : (u64)i, n, pool + cf_pool_off_binom(n), (int)sd.R + 1, K, idx);
+      in = 2 * s + (int)prefix;
+      const u64* pr = pool + cf_pool_off_prime(n);
+      u64 x = prefix ? sd.mult_m : 1u;
+      u32 c = prefix ? sd.mult_d : 1u % a.p.d;
+      u32 pk = 0;
+      int last = 0;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      if (j >= K) break;
-      const u64 q = pr[idx[j]];                    // below 2^31, x below 2^32
-      x = x * q % a.p.mp;
-      c = c * ((u32)q % a.p.d) % a.p.d;
-      pk |= (u32)idx[j] << (sd.bw * j);
-      last = idx[j];
+      for (int j = 0; j < 4; ++j) {
+        if (j >= K) break;
+        const u64 q = pr[idx[j]];                  // below 2^31, x below 2^32
+        x = x * q % a.p.mp;
+        c = c * ((u32)q % a.p.d) % a.p.d;
+        pk |= (u32)idx[j] << (sd.bw * j);
+        last = idx[j];
+      }
+      const u32 bin = (prefix ? sd.binP : sd.binT) + c * sd.n + (u32)(prefix ? last : idx[0]);
+      t_bin[e] = bin;
+      t_pos[e] = atomicAdd(&bins[bin], 1u);
+      t_x[e] = (u32)x;
+      t_pk[e] = pk;
     }
-    const u32 bin = (prefix ? sd.binP : sd.binT) + c * sd.n + (u32)(prefix ? last : idx[0]);
-    t_bin[e] = bin;
-    t_pos[e] = atomicAdd(&bins[bin], 1u);
-    t_x[e] = (u32)x;
-    t_pk[e] = pk;
   }
 }
 
@@ -211,6 +233,7 @@ __global__ void __launch_bounds__(256) k_cj_rows(const __grid_constant__ CjArgs 
   }
   if (lane == 0) {
     const u32 w = 32 * sd.U;
+    at<u32>(a, a.p.oRowCnt)[row] = run;
     at<u32>(a, a.p.oRowTot)[row] = prefix ? run : (run + w - 1) / w * w;
     if (l == 0) {
       const u32 inv = d == 1 ? 0u : cj_inverse(c, d);
@@ -285,7 +308,24 @@ __global__ void __launch_bounds__(256) k_cj_scatter(const __grid_constant__ CjAr
     } else {
       at<u32>(a, sd.oTX)[to] = x;                  // a unit mod m': never 0, the padding's value
       at<u32>(a, sd.oTI)[to] = pk;
-      atomicMax(at<u32>(a, sd.oBlk) + to / (32 * sd.U), (inv[c] << 16) | (pk & ((1u << sd.bw) - 1u)));
+    }
+  }
+  // per suffix block: inverse of its class and the first index of its last entry (a warp per class row)
+  const u32 lane = threadIdx.x & 31;
+  for (u32 row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < 2 * d; row += (gridDim.x * blockDim.x) >> 5) {
+    const u32 s = row >= d, c = row - s * d;
+    const CjSide& sd = a.p.side[s];
+    const u32 w = 32 * sd.U, nb = at<u32>(a, a.p.oRowTot)[2 * s * d + c] / w,
+              cnt = at<u32>(a, a.p.oRowCnt)[2 * s * d + c];
+    const u32* b = bins + sd.binT + (size_t)c * sd.n;
+    for (u32 i = lane; i < nb; i += 32) {
+      const u32 at_end = min((i + 1) * w, cnt) - 1;
+      u32 lo = 0, hi = sd.n - 1;                   // bin of the block's last entry: largest f with b[f] <= at_end
+      while (lo < hi) {
+        const u32 mid = (lo + hi + 1) >> 1;
+        if (b[mid] <= at_end) lo = mid; else hi = mid - 1;
+      }
+      at<u32>(a, sd.oBlk)[base[2 * s * d + c] / w + i] = (inv[c] << 16) | lo;
     }
   }
 }
@@ -437,41 +477,51 @@ __device__ __forceinline__ void cj_push(const CjArgs& a, CjSink& k, u32 ci, bool
   k.fill += n;
 }
 
+// The first 32 (or the last n) survivors of a warp's ring, one per lane: the records among them go to
+// the chunk list with their V.  A prefix that reaches past the suffix's first index is no record.
+__device__ __forceinline__ void cj_drain(const CjArgs& a, CjSink& k, u32 ci, const uint2* ring, u32 n) {
+  const CjSide& sd = a.p.side[1];
+  const u32 lane = threadIdx.x & 31;
+  u32 V = 0;
+  bool rec = false;
+  uint2 e = make_uint2(0u, 0u);                    // prefix entry, suffix entry
+  if (lane < n) {
+    e = ring[lane];
+    const u32 first = at<u32>(a, sd.oTI)[e.y] & ((1u << sd.bw) - 1u);
+    const u32 last = at<u32>(a, sd.oPI)[e.x] >> (sd.bw * (sd.A - 1));
+    V = cj_v(at<u64>(a, sd.oPW)[e.x], at<u32>(a, sd.oTX)[e.y]);
+    rec = first > last;
+  }
+  cj_push(a, k, ci, rec, V, ((u64)e.x << 32) | e.y);
+}
+
 template <int U>
-__device__ __forceinline__ void cj_probe_range(const CjArgs& a, const u32* s_bm, u32 ci, u32 c, u32 b0, u32 b1) {
+__device__ __forceinline__ void cj_probe_range(const CjArgs& a, const u32* s_bm, uint2* ring, u32 ci, u32 c, u32 b0,
+                                               u32 b1) {
   const CjSide& sd = a.p.side[1];
   const u32 lane = threadIdx.x & 31;
   const u32* TX = at<u32>(a, sd.oTX);
-  const u32* TI = at<u32>(a, sd.oTI);
   const u64* PW = at<u64>(a, sd.oPW);
-  const u32* PI = at<u32>(a, sd.oPI);
-  const u32 fm = (1u << sd.bw) - 1u, sh = sd.bw * (sd.A - 1);
   constexpr u32 G = 32 / U;                        // prefixes per word of outcome bits
+  constexpr u32 kPat = U == 4 ? 0x11111111u : U == 2 ? 0x55555555u : 0xffffffffu;
+  const u32 below = (1u << lane) - 1u;
   CjSink sink{0, 0};
+  u32 held = 0;                                    // survivors in the ring
   for (u32 i0 = 0; b0 + i0 * 32 < b1; i0 += 32) {
     const CjRun mine = cj_lookup(a, sd, 1, c, b0, b1, i0);
     for (u32 todo = __ballot_sync(0xffffffffu, mine.cnt != 0); todo; todo &= todo - 1) {
       const int src = __ffs(todo) - 1;
       const u32 t0 = __shfl_sync(0xffffffffu, mine.b, src) * 32 * U + lane;
       const u32 cnt = __shfl_sync(0xffffffffu, mine.cnt, src), first = __shfl_sync(0xffffffffu, mine.first, src);
-      u32 x[U], f0[(U + 1) / 2], keep = 0;         // keep: outcome bits of entries that are not padding
+      u32 x[U], keep = 0;                          // keep: outcome bits of entries that are not padding
       u64 w = lane < cnt ? PW[first + lane] : 0ull;
-      u32 last = lane < cnt ? PI[first + lane] >> sh : 0u;
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        x[u] = TX[t0 + 32 * u];
-        const u32 fi = TI[t0 + 32 * u] & fm;       // first index of the suffix, 16 bits each
-        f0[u / 2] = (u & 1) ? f0[u / 2] | (fi << 16) : fi;
-      }
+      for (int u = 0; u < U; ++u) x[u] = TX[t0 + 32 * u];
 #pragma unroll
-      for (int u = 0; u < U; ++u)
-        keep |= x[u] ? (u32)((U == 4 ? 0x11111111ull : U == 2 ? 0x55555555ull : 0xffffffffull) << (U - 1 - u)) : 0u;
+      for (int u = 0; u < U; ++u) keep |= x[u] ? kPat << (U - 1 - u) : 0u;
       for (u32 j0 = 0; j0 < cnt; j0 += 32) {
         const u32 m = min(32u, cnt - j0);
-        if (j0) {
-          w = lane < m ? PW[first + j0 + lane] : 0ull;
-          last = lane < m ? PI[first + j0 + lane] >> sh : 0u;
-        }
+        if (j0) w = lane < m ? PW[first + j0 + lane] : 0ull;
         for (u32 g0 = 0; g0 < m; g0 += G) {
           const u32 g1 = min(m, g0 + G);
           u32 acc = 0;                             // bit (prefix, entry), the last one lowest
@@ -486,38 +536,46 @@ __device__ __forceinline__ void cj_probe_range(const CjArgs& a, const u32* s_bm,
             }
           }
           acc &= keep;
-          while (__any_sync(0xffffffffu, acc != 0)) {
-            const bool have = acc != 0;
-            const u32 bit = have ? (u32)__ffs(acc) - 1u : 0u;
-            acc &= acc - 1u;
-            const u32 q = have ? (g1 - g0) * U - 1u - bit : 0u;   // (prefix - g0) * U + entry
-            const u32 j = g0 + q / U, u = q % U;
-            u32 xu = x[0], fu = f0[0];
-#pragma unroll
-            for (int v = 1; v < U; ++v) {
-              xu = u == (u32)v ? x[v] : xu;
-              fu = u == (u32)v ? f0[v / 2] >> (16 * (v & 1)) : fu;
+          const u32 top = (g1 - g0) * U - 1u, pf = first + j0 + g0;
+          for (u32 act; (act = __ballot_sync(0xffffffffu, acc != 0)) != 0;) {
+            if (acc) {
+              const u32 q = top - ((u32)__ffs(acc) - 1u);           // (prefix - g0) * U + entry
+              ring[held + __popc(act & below)] = make_uint2(pf + q / U, t0 + 32 * (q % U));
+              acc &= acc - 1u;
             }
-            const u32 V = cj_v(__shfl_sync(0xffffffffu, w, (int)j), xu);
-            const u32 lj = __shfl_sync(0xffffffffu, last, (int)j);   // every lane takes part
-            // a prefix that reaches past the suffix's first index is no record
-            cj_push(a, sink, ci, have && (fu & 0xffffu) > lj, V, ((u64)(first + j0 + j) << 32) | (t0 + 32 * u));
+            held += __popc(act);
+            if (held >= 32) {                      // a full warp of survivors at a time
+              __syncwarp();
+              cj_drain(a, sink, ci, ring, 32);
+              held -= 32;
+              const uint2 rest = ring[32 + lane];
+              __syncwarp();
+              if (lane < held) ring[lane] = rest;
+              __syncwarp();
+            }
           }
         }
       }
     }
   }
+  if (held) {
+    __syncwarp();
+    cj_drain(a, sink, ci, ring, held);
+  }
+  __syncwarp();
   cj_close(a, sink);
 }
 
-// Bound by integer issue: k = 64, r = 5, 5.9e8 I records in 0.64 ms (9e11 records/s; the fused
-// probe 3.2 ms), issue slots 68% busy, ALU pipe 63%, the multiplier pipe 56%, shared memory 58%; about
-// 12 instructions per 32 records tested, the rest survivors, prefixes past their suffix (10 to 30%)
-// and the block set-up.  32 warps of 64 registers: more registers would halve the warps that hide
-// the shared-memory latency.  CTA g of G takes the g-th of G equal parts of the (class, suffix block) sequence: whole classes
+// Bound by integer issue: k = 64, r = 5, 5.9e8 I records in 0.60 ms (9.8e11 records/s; the fused
+// probe 3.2 ms), issue slots 68% busy, ALU pipe 62%, the multiplier pipe 57%, shared memory 60%; 24
+// instructions per 32 records, of which 12 test, the rest survivors, prefixes past their suffix (10 to
+// 30%) and the block set-up.  Survivors wait in a ring per warp until 32 can be looked up at once
+// (pushed as found, with their V from registers: 0.64 ms).  32 warps of 64 registers: more registers
+// would halve the warps that hide the shared-memory latency.  CTA g of G takes the g-th of G equal parts of the (class, suffix block) sequence: whole classes
 // and a part of one at either end, so a filter is loaded phi + G times in all.
 __global__ void __launch_bounds__(kCjBlock, 1) k_cj_probe(const __grid_constant__ CjArgs a) {
   extern __shared__ __align__(16) u32 s_bm[];
+  uint2* ring = (uint2*)(s_bm + kCjWords) + (threadIdx.x >> 5) * 64;   // this warp's survivors
   const u32 nblk = at<u32>(a, a.p.oCtr)[kCtrNb1];
   const u64 total = (u64)a.p.phi * nblk;
   u64 lo = total * blockIdx.x / gridDim.x;
@@ -531,9 +589,9 @@ __global__ void __launch_bounds__(kCjBlock, 1) k_cj_probe(const __grid_constant_
 #pragma unroll 12
     for (u32 i = threadIdx.x; i < kCjWords / 4; i += kCjBlock) ((uint4*)s_bm)[i] = __ldcg(in + i);
     __syncthreads();
-    if (a.p.side[1].U == 4) cj_probe_range<4>(a, s_bm, ci, c, b0, b1);
-    else if (a.p.side[1].U == 2) cj_probe_range<2>(a, s_bm, ci, c, b0, b1);
-    else cj_probe_range<1>(a, s_bm, ci, c, b0, b1);
+    if (a.p.side[1].U == 4) cj_probe_range<4>(a, s_bm, ring, ci, c, b0, b1);
+    else if (a.p.side[1].U == 2) cj_probe_range<2>(a, s_bm, ring, ci, c, b0, b1);
+    else cj_probe_range<1>(a, s_bm, ring, ci, c, b0, b1);
     lo += b1 - b0;
   }
 }
@@ -907,6 +965,7 @@ extern "C" int cf_class_plan(u64 m, int nD, int nI, int r, u64 i_lo, u64 i_n, in
     sd.mult_m = 1; sd.mult_d = 1 % d;
   }
   P->elems = (u32)el;
+  P->run = el >= (2u << 20) ? 4 : 1;
   const double lam = per / kCjWords, fp = std::min(0.5, (lam + lam * lam) / 256.0);
   const double chunks = 4096.0 + (double)(phi + 148) * kCjWarps + n_probe * std::min(0.6, 1.5 * fp) / 96.0;
   if (chunks > 3.0e7) return CF_OK;               // entry places stay below 2^32
@@ -922,6 +981,7 @@ extern "C" int cf_class_plan(u64 m, int nD, int nI, int r, u64 i_lo, u64 i_n, in
   P->oInv = off; off = up256(off + (u64)d * 4);
   P->oRowBase = off; off = up256(off + (u64)d * 16);
   P->oRowTot = off; off = up256(off + (u64)d * 16);
+  P->oRowCnt = off; off = up256(off + (u64)d * 16);
   P->oTmp = off; off = up256(off + el * 16);
   for (int s = 0; s < 2; ++s) {
     CjSide& sd = P->side[s];
@@ -973,14 +1033,14 @@ extern "C" int cf_class_join(const void* plan, const void* poolD, const void* po
   a.npairs = npairs;
   a.err = err;
   a.max_pairs = max_pairs;
-  const int smem1 = (int)(kCjWords * 4), smem2 = (int)((kCjWords2 + kCjHeads) * 4);
+  const int smem1 = (int)(kCjWords * 4), smemP = smem1 + kCjWarps * 64 * 8, smem2 = (int)((kCjWords2 + kCjHeads) * 4);
   cudaError_t e = cudaFuncSetAttribute(k_cj_build, cudaFuncAttributeMaxDynamicSharedMemorySize, smem1);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cj_probe, cudaFuncAttributeMaxDynamicSharedMemorySize, smem1);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cj_probe, cudaFuncAttributeMaxDynamicSharedMemorySize, smemP);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cj_resolve, cudaFuncAttributeMaxDynamicSharedMemorySize, smem2);
   if (e == cudaSuccess) e = cudaMemsetAsync(ws, 0, P->zero_bytes, st);
   if (e != cudaSuccess) return cf_cuda_status(e, "cf_class_join: set-up");
   const unsigned ge = std::min<u32>((P->elems + 255) / 256, 148 * 16);
-  k_cj_count<<<ge, 256, 0, st>>>(a);
+  k_cj_count<<<std::min<u32>((P->elems / P->run + 256) / 256, 148 * 16), 256, 0, st>>>(a);
   k_cj_rows<<<(4 * P->d * 32 + 255) / 256, 256, 0, st>>>(a);
   k_cj_rowscan<<<1, kCjBlock, 0, st>>>(a);
   k_cj_scatter<<<ge, 256, 0, st>>>(a);
@@ -990,7 +1050,7 @@ extern "C" int cf_class_join(const void* plan, const void* poolD, const void* po
     e = cudaEventRecord((cudaEvent_t)ev_built, st);
     if (e != cudaSuccess) return cf_cuda_status(e, "cf_class_join: event");
   }
-  k_cj_probe<<<148, kCjBlock, smem1, st>>>(a);
+  k_cj_probe<<<148, kCjBlock, smemP, st>>>(a);
   k_cj_resolve<<<g, kCjBlock, smem2, st>>>(a);
   k_cj_emit<<<148 * 4, 128, 0, st>>>(a);
   CF_LAUNCH_CHECK("cf_class_join");
