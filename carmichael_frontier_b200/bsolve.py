@@ -26,7 +26,7 @@ import numpy as np
 from . import _lib
 from .bounded import U128
 from .certify import verify_certificate
-from .tables import pool_table_host, unrank_colex, unrank_colex_batch, wide_modulus
+from .tables import pool_table_host, screen_table_host, unrank_colex, unrank_colex_batch, wide_modulus
 
 RANK_LIMIT = 1 << 32          # positions in the join table are 32-bit
 
@@ -189,14 +189,16 @@ class BoundedSolve:
         if cp is None:
             return None
         multD = pow(inst.P0, -1, M)
-        poolD, poolI = s.tables.pool(B0, r, M, multD), s.tables.pool(INS, r, M, 1)
-        G = s.tables.get(("bcountG", tuple(B0), r, Dmin), lambda: self._bound_table(lib.cf_ddump_bounds, B0, r, Dmin))
-        H = s.tables.get(("bcountH", tuple(INS), r, Icap), lambda: self._bound_table(lib.cf_igen_bounds, INS, r, Icap))
+        # screen bound 1: no pair passes, the check only turns ranks into indices
+        dev = self._upload([pool_table_host(B0, r, M, multD), pool_table_host(INS, r, M, 1),
+                            self._bound_table(lib.cf_ddump_bounds, B0, r, Dmin),
+                            self._bound_table(lib.cf_igen_bounds, INS, r, Icap), screen_table_host(inst.P0, 1, 1e-6)])
+        poolD, poolI, G, H, screen = dev
         misc = s._buf("bctr", 64)[:64]
         misc.zero_()
         sh, base = s._sh(), dp(misc)
-        _lib.check(lib.cf_bounded_count(1, dp(poolD), dp(G), len(B0), r, base + 16, sh), "cf_bounded_count(D)")
-        _lib.check(lib.cf_bounded_count(0, dp(poolI), dp(H), len(INS), r, base + 24, sh), "cf_bounded_count(I)")
+        _lib.check(lib.cf_bounded_count(1, poolD, G, len(B0), r, base + 16, sh), "cf_bounded_count(D)")
+        _lib.check(lib.cf_bounded_count(0, poolI, H, len(INS), r, base + 24, sh), "cf_bounded_count(I)")
         bD, bI = misc[16:32].cpu().numpy().view(np.uint64).tolist()
         if (bD + bI) * self.CLASS_RATIO < total:
             return None
@@ -207,14 +209,13 @@ class BoundedSolve:
         ws_bytes = int(np.frombuffer(cp, dtype=np.uint64, count=1, offset=24)[0])
         ws = s._buf("class", ws_bytes)
         maxp = max(s.tuning.pair_capacity, min(1 << 22, 1 << (8 * nD * nI // M).bit_length()))
-        screen = s.tables.screen(inst.P0, 1, 1e-6)     # no pair passes: the check only turns ranks into indices
         while True:
             pairs = s._buf("pairs", maxp * 16)
             res = s._buf("res", maxp * s.result_bytes)
             misc[:8].zero_()
-            _lib.check(lib.cf_class_join(cp, dp(poolD), dp(poolI), multD % mp, multD % d, dp(ws), ws_bytes, dp(pairs),
+            _lib.check(lib.cf_class_join(cp, poolD, poolI, multD % mp, multD % d, dp(ws), ws_bytes, dp(pairs),
                                          maxp, base, base + 4, None, sh), "cf_class_join")
-            _lib.check(lib.cf_check_pairs(dp(poolD), dp(poolI), dp(screen), r, dp(pairs), base, maxp, dp(res),
+            _lib.check(lib.cf_check_pairs(poolD, poolI, screen, r, dp(pairs), base, maxp, dp(res),
                                           base + 4, sh), "cf_check_pairs")
             self.gen.launches += 10
             npairs, err = misc[:8].cpu().numpy().view(np.uint32).tolist()
@@ -267,20 +268,7 @@ class BoundedSolve:
         parts = [pool_table_host(B0, r, M, 1), pool_table_host(INS, r, M, inst.P0 % M),
                  self._bound_table(lib.cf_ddump_bounds, B0, r, int(Dmin)),
                  self._bound_table(lib.cf_igen_bounds, INS, r, int(Icap))]
-        offs, total = [], 0
-        for a in parts:
-            offs.append(total)
-            total += (a.nbytes + 255) // 256 * 256
-        if self._stage is None or self._stage.numel() < total:
-            self._stage = torch.empty(max(total, 1 << 20), dtype=torch.uint8, pin_memory=True)
-        host = self._stage.numpy()
-        for o, a in zip(offs, parts):
-            host[o:o + a.nbytes] = a.view(np.uint8)
-        dev = self.s._buf("bjtab", max(total, 1 << 20))
-        with torch.cuda.stream(self.s._torch_stream()):
-            dev[:total].copy_(self._stage[:total], non_blocking=True)
-        base = dp(dev)
-        poolD, poolI, G, H = (base + o for o in offs)
+        poolD, poolI, G, H = self._upload(parts)
         sh = self.s._sh()
         n_out, need = C.c_uint64(0), C.c_uint64(0)
         sizes = (C.c_uint64 * 2)()
@@ -313,6 +301,25 @@ class BoundedSolve:
             dd_all, ii_all = unrank_colex_batch(did, r, nb).tolist(), unrank_colex_batch(iid, r, ni).tolist()
         pairs = _confirmed_pairs(dd_all, ii_all, dkey, INS, inst.P0 % M, M)
         return pairs, nD, nI, dict(strategy="bounded", Icap=Icap, Dmin=Dmin, table="D", native=True)
+
+    def _upload(self, parts: list) -> list:
+        """Device addresses of host tables that go up in one copy, packed at 256-byte offsets into a
+        page-locked buffer (reused by the next call: every join waits for its results)."""
+        torch = self.torch
+        offs, total = [], 0
+        for a in parts:
+            offs.append(total)
+            total += (a.nbytes + 255) // 256 * 256
+        if self._stage is None or self._stage.numel() < total:
+            self._stage = torch.empty(max(total, 1 << 20), dtype=torch.uint8, pin_memory=True)
+        host = self._stage.numpy()
+        for o, a in zip(offs, parts):
+            host[o:o + a.nbytes] = a.view(np.uint8)
+        dev = self.s._buf("bjtab", max(total, 1 << 20))
+        with torch.cuda.stream(self.s._torch_stream()):
+            dev[:total].copy_(self._stage[:total], non_blocking=True)
+        base = _lib.ptr(dev)
+        return [base + o for o in offs]
 
     def _bound_table(self, fn, primes, r: int, bound: int) -> np.ndarray:
         """A bound table (cf_ddump_bounds / cf_igen_bounds) of the primes, on the host."""

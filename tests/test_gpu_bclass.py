@@ -81,3 +81,17 @@ def test_bounds_at_a_pair(cuda, monkeypatch):
             got = b._join_class(inst, Ic, Dm)
             ref = lev._join(inst, Ic, Dm, None, None)
             assert got is not None and sorted(got[0]) == sorted(ref[0]) and got[1:3] == ref[1:3]
+
+
+@pytest.mark.gpu
+def test_counts_by_walking_equal_the_level_expansion(cuda):
+    """C(n, r-2) above 2^20 prefixes: the walking form of the count kernel."""
+    B0, INS, r = Q[:76], Q[76:176], 6
+    assert math.comb(76, r - 2) > 1 << 20
+    g = BoundedSolve(Solver(cuda)).gen
+    Dmin = math.prod(B0[-6:]) * 2 // 3
+    Icap = math.prod(INS[:6]) * 3
+    nD = g.generate_D(B0, r, M, Dmin, bitmask=2)[2]
+    it = g.generate_I(INS, r, M, 1, Icap)
+    nI = sum(k.numel() for k, _ in it)
+    assert nD and nI and counts(cuda, B0, INS, r, Icap, Dmin) == [nD, nI]
