@@ -102,7 +102,7 @@ k_gen_linear(const u64* __restrict__ pool, u64 lo, u64 count, int id_mode, int b
 // The same records through the suffix table (fast pools, R >= 3): a record is one 64-bit Montgomery
 // product of its prefix with a table entry read coalesced, and the prefix of R - 2 indices changes
 // once in some thousand records, where the walker above moves to a new (R-1)-prefix about every 30
-// (a serial step of the whole warp).  1.0e7 records of a 126-prime pool at R = 4: 81 us, 134 with
+// (a serial step of the whole warp).  1.0e7 records of a 126-prime pool at R = 4: 73 us, 134 with
 // the walker; the 16 bytes written per record take 25.
 template <int R>
 __global__ void __launch_bounds__(kLinBlock)
@@ -348,8 +348,9 @@ template <int R>
 void launch_gen_tail(const u64* pool, const CfTailEnt* tail, u64 lo, u64 count, int id_mode, int bits, int canon,
                      u64* keys, u64* ids, cudaStream_t st) {
   if constexpr (R >= 3) {
-    // a warp's start (unranking) is a chain of some hundred loads: long ranges once they still fill the GPU
-    const u32 steps = count >= (1u << 22) ? 64u : 16u;
+    // a warp's start (unranking) is a chain of some hundred loads: longer ranges once they still fill the GPU
+    // (1.0e7 records: 73 us with 32 steps, 81 with 64; the next entry loaded a step ahead: 92)
+    const u32 steps = count >= (1u << 22) ? 32u : 16u;
     const u64 per = (u64)kLinBlock * steps;
     k_gen_tail<R><<<(unsigned)((count + per - 1) / per), kLinBlock, 0, st>>>(pool, tail, lo, count, steps, id_mode, bits,
                                                                             canon, keys, ids);

@@ -596,10 +596,18 @@ k_seg_hist(const u64* __restrict__ keys, u64 n, const SegCtl* __restrict__ ctl, 
   for (int i = threadIdx.x; i < bins; i += blockDim.x) s_h[i] = 0;
   const SegScale sc = seg_map(ctl);
   __syncthreads();
-  for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64)gridDim.x * blockDim.x) {
-    const u32 v = sc(keys[i]) >> kSegBits;
-    atomicAdd(&s_h[v & mask], 1u);
-    if (np > 1) atomicAdd(&s_h[(1u << db) + (v >> db)], 1u);
+  constexpr int kU = 8;                                // loads in flight per thread
+  for (u64 i0 = (u64)blockIdx.x * 512 * kU + threadIdx.x; i0 < n; i0 += (u64)gridDim.x * 512 * kU) {
+    u64 k[kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u) k[u] = i0 + u * 512 < n ? keys[i0 + u * 512] : 0ull;
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      if (i0 + u * 512 >= n) break;
+      const u32 v = sc(k[u]) >> kSegBits;
+      atomicAdd(&s_h[v & mask], 1u);
+      if (np > 1) atomicAdd(&s_h[(1u << db) + (v >> db)], 1u);
+    }
   }
   __syncthreads();
   for (int i = threadIdx.x; i < bins; i += blockDim.x)
@@ -616,8 +624,8 @@ k_seg_front(const u64* __restrict__ keys, u32 n, u32 segs, SegCtl* __restrict__ 
   if (threadIdx.x < 256) s_h[threadIdx.x] = 0;
   __syncthreads();
   u64 m = 0;
-#pragma unroll 8
-  for (u32 i = threadIdx.x; i < n; i += 1024) {
+#pragma unroll 4
+  for (u32 i = threadIdx.x; i < n; i += 4096) {        // a quarter of the keys
     const u64 k = keys[i];
     m = k > m ? k : m;
     u32 frac;
@@ -674,31 +682,34 @@ k_seg_front(const u64* __restrict__ keys, u32 n, u32 segs, SegCtl* __restrict__ 
   }
 }
 
-// First record of each segment (records ordered by f >> L), and the largest segment.
-__global__ void __launch_bounds__(256)
+// First record of each segment (records ordered by f >> L), and the largest segment.  A warp per
+// segment, 32 probes a round: five or six dependent loads (a thread's binary search made 23 to 26 of
+// them: 24 us for the 2,243 segments of 7.6e6 records, 9.5 here).
+constexpr int kBoundWarps = 8;                         // segments per CTA; one warp more for the last one's end
+__global__ void __launch_bounds__((kBoundWarps + 1) * 32)
 k_seg_bounds(const u64* __restrict__ keys, u32 n, u32 segs, SegCtl* __restrict__ ctl, u32* __restrict__ starts) {
-  const u32 s = blockIdx.x * blockDim.x + threadIdx.x;
+  __shared__ u32 s_at[kBoundWarps + 1];
+  const u32 wid = threadIdx.x >> 5, lane = threadIdx.x & 31, s = blockIdx.x * kBoundWarps + wid;
   const SegScale sc = seg_map(ctl);
-  u32 lo = 0, hi = s < segs ? n : 0u, len = 0;
-  while (lo < hi) {                                    // lower bound of segment s
-    const u32 mid = (lo + hi) >> 1;
-    if ((sc(keys[mid]) >> kSegBits) < s) lo = mid + 1; else hi = mid;
-  }
-  if (s >= segs) lo = n;
-  if (s <= segs) starts[s] = lo;
-  const u32 next = __shfl_down_sync(0xffffffffu, lo, 1);
-  if ((threadIdx.x & 31) < 31) len = next - lo;
-  else if (s < segs) {                                 // the next warp's first segment
-    u32 l2 = lo, h2 = s + 1 < segs ? n : lo;
-    while (l2 < h2) {
-      const u32 mid = (l2 + h2) >> 1;
-      if ((sc(keys[mid]) >> kSegBits) < s + 1) l2 = mid + 1; else h2 = mid;
+  u32 lo = 0, hi = n;                                  // lower bound of segment s
+  if (s < segs) {
+    while (hi - lo > 32) {
+      const u32 step = (hi - lo) / 33 + 1, p = lo + (lane + 1) * step - 1;
+      const bool less = p < hi && (sc(keys[p]) >> kSegBits) < s;
+      lo += __popc(__ballot_sync(0xffffffffu, less)) * step;
+      hi = min(hi, lo + step - 1);
     }
-    len = (s + 1 < segs ? l2 : n) - lo;
+    const bool less = lo + lane < hi && (sc(keys[lo + lane]) >> kSegBits) < s;
+    lo += __popc(__ballot_sync(0xffffffffu, less));
+  } else {
+    lo = n;
   }
-#pragma unroll
-  for (int o = 16; o; o >>= 1) len = max(len, __shfl_xor_sync(0xffffffffu, len, o));
-  if ((threadIdx.x & 31) == 0 && len) atomicMax(&ctl->max_seg, len);
+  if (lane == 0) s_at[wid] = lo;
+  __syncthreads();
+  if (lane == 0 && wid < kBoundWarps && s <= segs) {
+    starts[s] = lo;
+    if (s < segs) atomicMax(&ctl->max_seg, s_at[wid + 1] - lo);
+  }
 }
 
 // Sort one segment by (key, position).  Bound by its chain of shared-memory phases, the neighbours'
@@ -1170,7 +1181,8 @@ extern "C" int cf_sort_pairs_to(const u64* kin, const u64* iin, u64* kout, u64* 
     if (front) {
       k_seg_front<<<1, 1024, 0, st>>>(kin, (u32)n, segs, ctl, excl, starts);
     } else {
-      k_seg_sample<<<gm, 512, 0, st>>>(kin, n, n >= (1u << 23) ? 64 : n >= (1u << 18) ? 8 : 1, segs, ctl);
+      // 2^19 to 2^20 sampled keys, some fifty per segment at 2^26 records
+      k_seg_sample<<<gm < 148 ? gm : 148, 512, 0, st>>>(kin, n, (u32)(n >> 20) + 1, segs, ctl);
       k_seg_hist<<<gm, 512, 0, st>>>(kin, n, ctl, hist, np, db);
       k_sort_hist_scan<<<1, 32 * np, 0, st>>>(hist, excl, db);
     }
@@ -1187,7 +1199,7 @@ extern "C" int cf_sort_pairs_to(const u64* kin, const u64* iin, u64* kout, u64* 
         sort_pass_launch<9, u32, true>(bulk, (unsigned)tiles, st, ka, ia, kb, ib, n, shift, excl + p * bins, pst,
                                        ctl->tickets + p, errw, ctl);
     }
-    if (!front) k_seg_bounds<<<segs / 256 + 1, 256, 0, st>>>(kout, (u32)n, segs, ctl, starts);
+    if (!front) k_seg_bounds<<<segs / kBoundWarps + 1, (kBoundWarps + 1) * 32, 0, st>>>(kout, (u32)n, segs, ctl, starts);
     k_seg_sort<<<segs, kSegBlock, kSegSmem, st>>>(kout, iout, kout, iout, (u32)n, ctl, starts);
     CF_LAUNCH_CHECK("cf_sort_pairs_to: segments");
     u32 h[2];                                          // largest segment, error word
