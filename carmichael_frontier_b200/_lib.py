@@ -91,6 +91,8 @@ SIGNATURES = [
     ("cf_scan_u64", C.c_int, [vp, u64, vp, vp, sz, vp]),
     ("cf_bgen_count", C.c_int, [C.c_int, C.c_int, C.c_int, C.c_int, u64, vp, vp, vp, vp, C.c_int, C.c_int, C.c_int,
                                 C.c_int, vp, vp, vp]),
+    ("cf_bgen_count_scan", C.c_int, [C.c_int, C.c_int, C.c_int, C.c_int, u64, vp, vp, vp, vp, C.c_int, C.c_int, C.c_int,
+                                     C.c_int, vp, vp, vp, sz, vp]),
     ("cf_bgen_expand", C.c_int, [C.c_int, C.c_int, C.c_int, C.c_int, u64, vp, vp, vp, vp, vp, vp, vp, vp, C.c_int,
                                  C.c_int, u64, u64, vp, vp, vp, vp, vp, vp]),
     ("cf_rec_build", C.c_int, [vp, u64, vp, C.c_int, C.c_int, vp, vp]),

@@ -109,17 +109,6 @@ class BoundedGenerator:
         self.launches = 0
 
     # -- primitives -----------------------------------------------------------
-    def _scan(self, cnt, F: int):
-        torch = self.torch
-        nb = self.lib.cf_scan_tmp_bytes(F)
-        ob = (8 * (F + 1) + 255) // 256 * 256            # offsets, then the scan's scratch (one allocation)
-        buf = torch.empty(ob + max(nb, 16), dtype=torch.uint8, device=self.device)
-        offs = buf[:8 * (F + 1)].view(torch.int64)
-        _lib.check(self.lib.cf_scan_u64(_lib.ptr(cnt), F, _lib.ptr(offs), buf.data_ptr() + ob, nb,
-                                        _lib.stream_handle()), "cf_scan_u64")
-        self.launches += 2
-        return offs
-
     def _frontier(self, side: int, pool, bounds, n: int, r: int, split_idx: int, hmax: int, bitmask: int,
                   xa: int, xb: int, M: int, mult: int, limit: int | None = -1):
         """Nodes at depth r-1 of the block of first indices [xa, xb), their child
@@ -137,13 +126,16 @@ class BoundedGenerator:
         F = 1
         sh = _lib.stream_handle()
         for d in range(r):
-            cx = torch.empty(F + (F + 1) // 2, dtype=torch.int64, device=dev)   # counts, then first indices
-            cnt = cx[:F]
-            xs = cx[F:].view(torch.int32)[:F]
-            _lib.check(lib.cf_bgen_count(side, d, r, n, F, dp(alo), dp(ahi), dp(meta), dp(bounds), split_idx, hmax,
-                                         xa, xb, dp(cnt), dp(xs), sh), "cf_bgen_count")
+            # offsets, first child indices, and the scan's scratch (one allocation)
+            xo = (8 * (F + 1) + 255) // 256 * 256
+            to = xo + (4 * F + 255) // 256 * 256
+            nb = lib.cf_scan_tmp_bytes(F)
+            buf = torch.empty(to + nb, dtype=torch.uint8, device=dev)
+            offs, xs = buf[:8 * (F + 1)].view(torch.int64), buf[xo:xo + 4 * F].view(torch.int32)
+            _lib.check(lib.cf_bgen_count_scan(side, d, r, n, F, dp(alo), dp(ahi), dp(meta), dp(bounds), split_idx, hmax,
+                                              xa, xb, dp(xs), dp(offs), buf.data_ptr() + to, nb, sh),
+                       "cf_bgen_count_scan")
             self.launches += 1
-            offs = self._scan(cnt, F)
             total = int(offs[F].item())
             if d == r - 1:
                 return dict(F=F, key=key, alo=alo, ahi=ahi, ids=ids, meta=meta, offs=offs, xs=xs, total=total)

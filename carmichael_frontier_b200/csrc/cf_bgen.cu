@@ -54,14 +54,12 @@ __device__ __forceinline__ U128 bound_at(const u64* __restrict__ tb, int n, int 
 
 constexpr u32 kRoot = 0xffffu;
 
-// Children of every frontier node at depth d: cnt[i] and the first child index xs[i].
+// Children of frontier node i at depth d: their number, and the first child index in x0.
 template <int SIDE>
-__global__ void __launch_bounds__(256)
-k_bgen_count(int d, int r, int n, u64 F, const u64* __restrict__ alo, const u64* __restrict__ ahi,
-             const u32* __restrict__ meta, const u64* __restrict__ bounds, int split_idx, int hmax, int xa, int xb,
-             u64* __restrict__ cnt, u32* __restrict__ xs) {
-  const u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= F) return;
+__device__ __forceinline__ u64 bgen_children(int d, int r, int n, u64 i, const u64* __restrict__ alo,
+                                             const u64* __restrict__ ahi, const u32* __restrict__ meta,
+                                             const u64* __restrict__ bounds, int split_idx, int hmax, int xa, int xb,
+                                             u32& x0) {
   const int t = r - d - 1;
   const u32 mt = meta[i];
   const int last = (int)(mt & 0xffffu);
@@ -70,7 +68,7 @@ k_bgen_count(int d, int r, int n, u64 F, const u64* __restrict__ alo, const u64*
   A.lo = alo[i];
   A.hi = ahi[i];
   u64 c = 0;
-  u32 x0 = 0;
+  x0 = 0;
   if (SIDE == 0) {                          // I side: ascending, x in [lo, hi] with H[t][x] >= A
     int lo = (last == (int)kRoot) ? 0 : last + 1;
     int hi = n - 1 - t;
@@ -105,7 +103,19 @@ k_bgen_count(int d, int r, int n, u64 F, const u64* __restrict__ alo, const u64*
       x0 = (u32)hi;
     }
   }
-  cnt[i] = c;
+  return c;
+}
+
+// cnt[i] and xs[i] of every frontier node at depth d.
+template <int SIDE>
+__global__ void __launch_bounds__(256)
+k_bgen_count(int d, int r, int n, u64 F, const u64* __restrict__ alo, const u64* __restrict__ ahi,
+             const u32* __restrict__ meta, const u64* __restrict__ bounds, int split_idx, int hmax, int xa, int xb,
+             u64* __restrict__ cnt, u32* __restrict__ xs) {
+  const u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= F) return;
+  u32 x0;
+  cnt[i] = bgen_children<SIDE>(d, r, n, i, alo, ahi, meta, bounds, split_idx, hmax, xa, xb, x0);
   xs[i] = x0;
 }
 
@@ -208,11 +218,8 @@ k_bgen_expand(int d, int r, int n, u64 F, const u64* __restrict__ pool, const u6
 // ---- exclusive scan of u64 counts ---------------------------------------------
 constexpr int kScanBlock = 1024;
 
-__global__ void __launch_bounds__(kScanBlock)
-k_scan_block(const u64* __restrict__ in, u64 n, u64* __restrict__ out, u64* __restrict__ sums) {
-  __shared__ u64 warp_tot[32];
-  const u64 i = (u64)blockIdx.x * kScanBlock + threadIdx.x;
-  const u64 v = i < n ? in[i] : 0;
+// Exclusive prefix of v over the block; the block's total in `total` (every thread).
+__device__ __forceinline__ u64 block_exclusive(u64 v, u64* warp_tot, u64& total) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   u64 s = v;
 #pragma unroll
@@ -232,19 +239,52 @@ k_scan_block(const u64* __restrict__ in, u64 n, u64* __restrict__ out, u64* __re
     warp_tot[lane] = t;                       // inclusive over warps
   }
   __syncthreads();
-  const u64 before = (w ? warp_tot[w - 1] : 0) + s - v;
-  if (i < n) out[i] = before;
-  if (threadIdx.x == kScanBlock - 1) sums[blockIdx.x] = warp_tot[31];
+  total = warp_tot[31];
+  return (w ? warp_tot[w - 1] : 0) + s - v;
 }
 
+// One block of the scan; a scan of one block also writes out[n], its total.
 __global__ void __launch_bounds__(kScanBlock)
-k_scan_add(u64* __restrict__ out, u64 n, const u64* __restrict__ add) {
+k_scan_block(const u64* __restrict__ in, u64 n, u64* __restrict__ out, u64* __restrict__ sums, bool write_total) {
+  __shared__ u64 warp_tot[32];
+  const u64 i = (u64)blockIdx.x * kScanBlock + threadIdx.x;
+  u64 total;
+  const u64 before = block_exclusive(i < n ? in[i] : 0, warp_tot, total);
+  if (i < n) out[i] = before;
+  if (threadIdx.x == kScanBlock - 1) {
+    sums[blockIdx.x] = total;
+    if (write_total && gridDim.x == 1) out[n] = total;
+  }
+}
+
+// k_bgen_count and the first level of the scan of its counts in one pass.
+template <int SIDE>
+__global__ void __launch_bounds__(kScanBlock)
+k_bgen_count_scan(int d, int r, int n, u64 F, const u64* __restrict__ alo, const u64* __restrict__ ahi,
+                  const u32* __restrict__ meta, const u64* __restrict__ bounds, int split_idx, int hmax, int xa, int xb,
+                  u32* __restrict__ xs, u64* __restrict__ out, u64* __restrict__ sums) {
+  __shared__ u64 warp_tot[32];
+  const u64 i = (u64)blockIdx.x * kScanBlock + threadIdx.x;
+  u64 c = 0, total;
+  if (i < F) {
+    u32 x0;
+    c = bgen_children<SIDE>(d, r, n, i, alo, ahi, meta, bounds, split_idx, hmax, xa, xb, x0);
+    xs[i] = x0;
+  }
+  const u64 before = block_exclusive(c, warp_tot, total);
+  if (i < F) out[i] = before;
+  if (threadIdx.x == kScanBlock - 1) {
+    sums[blockIdx.x] = total;
+    if (gridDim.x == 1) out[F] = total;
+  }
+}
+
+// out += the scanned block sums; with in_total, out[n] is the sum of all blocks.
+__global__ void __launch_bounds__(kScanBlock)
+k_scan_add(u64* __restrict__ out, u64 n, const u64* __restrict__ add, const u64* __restrict__ sums, bool write_total) {
   const u64 i = (u64)blockIdx.x * kScanBlock + threadIdx.x;
   if (i < n) out[i] += add[blockIdx.x];
-}
-
-__global__ void k_scan_total(const u64* __restrict__ in, const u64* __restrict__ ex, u64 n, u64* __restrict__ out) {
-  out[n] = n ? ex[n - 1] + in[n - 1] : 0;
+  if (write_total && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) out[n] = add[blockIdx.x] + sums[blockIdx.x];
 }
 
 u64 scan_tmp_words(u64 n) {
@@ -256,15 +296,21 @@ u64 scan_tmp_words(u64 n) {
   return w + 2;
 }
 
-void scan_rec(const u64* in, u64 n, u64* out, u64* tmp, cudaStream_t st) {
+void scan_rec(const u64* in, u64 n, u64* out, u64* tmp, cudaStream_t st, bool write_total);
+
+// The levels of a scan of n values above its first one, whose block sums are in tmp.
+void scan_rest(u64 n, u64* out, u64* tmp, cudaStream_t st, bool write_total) {
   const u64 nb = (n + kScanBlock - 1) / kScanBlock;
-  u64* sums = tmp;
-  k_scan_block<<<(unsigned)nb, kScanBlock, 0, st>>>(in, n, out, sums);
-  if (nb > 1) {
-    u64* sums_ex = tmp + nb + 1;
-    scan_rec(sums, nb, sums_ex, sums_ex + nb + 1, st);
-    k_scan_add<<<(unsigned)nb, kScanBlock, 0, st>>>(out, n, sums_ex);
-  }
+  if (nb <= 1) return;
+  u64* sums_ex = tmp + nb + 1;
+  scan_rec(tmp, nb, sums_ex, sums_ex + nb + 1, st, false);
+  k_scan_add<<<(unsigned)nb, kScanBlock, 0, st>>>(out, n, sums_ex, tmp, write_total);
+}
+
+void scan_rec(const u64* in, u64 n, u64* out, u64* tmp, cudaStream_t st, bool write_total) {
+  const u64 nb = (n + kScanBlock - 1) / kScanBlock;
+  k_scan_block<<<(unsigned)nb, kScanBlock, 0, st>>>(in, n, out, tmp, write_total);
+  scan_rest(n, out, tmp, st, write_total);
 }
 
 }  // namespace
@@ -282,8 +328,7 @@ extern "C" int cf_scan_u64(const u64* in, u64 n, u64* out, void* tmp, size_t tmp
     return CF_OK;
   }
   if (tmp_bytes < cf_scan_tmp_bytes(n)) { cf_set_error("cf_scan_u64: workspace too small%s", ""); return CF_EBADARG; }
-  scan_rec(in, n, out, (u64*)tmp, st);
-  k_scan_total<<<1, 1, 0, st>>>(in, out, n, out);
+  scan_rec(in, n, out, (u64*)tmp, st, true);
   CF_LAUNCH_CHECK("cf_scan_u64");
   return CF_OK;
 }
@@ -310,6 +355,29 @@ extern "C" int cf_bgen_count(int side, int d, int r, int n, u64 F, const u64* al
     k_bgen_count<1><<<g, 256, 0, (cudaStream_t)stream>>>(d, r, n, F, alo, ahi, meta, bounds, split_idx, hmax, xa, xb,
                                                          cnt, xs);
   CF_LAUNCH_CHECK("cf_bgen_count");
+  return CF_OK;
+}
+
+// cf_bgen_count and cf_scan_u64 of its counts: xs[F], offs[F + 1] with the total last.  tmp:
+// cf_scan_tmp_bytes(F).  Two launches fewer per level than the two calls.
+extern "C" int cf_bgen_count_scan(int side, int d, int r, int n, u64 F, const u64* alo, const u64* ahi,
+                                  const u32* meta, const u64* bounds, int split_idx, int hmax, int xa, int xb, u32* xs,
+                                  u64* offs, void* tmp, size_t tmp_bytes, void* stream) {
+  if ((side != 0 && side != 1) || r < 1 || r > CF_MAX_R || d < 0 || d >= r || n < 1 || n > CF_MAX_POOL || F == 0 ||
+      F > (1ull << 40) || !bounds || !xs || !offs || !tmp || !alo || !ahi || !meta || tmp_bytes < cf_scan_tmp_bytes(F)) {
+    cf_set_error("cf_bgen_count_scan: bad arguments%s", "");
+    return CF_EBADARG;
+  }
+  const cudaStream_t st = (cudaStream_t)stream;
+  const unsigned g = (unsigned)((F + kScanBlock - 1) / kScanBlock);
+  if (side == 0)
+    k_bgen_count_scan<0><<<g, kScanBlock, 0, st>>>(d, r, n, F, alo, ahi, meta, bounds, split_idx, hmax, xa, xb, xs, offs,
+                                                   (u64*)tmp);
+  else
+    k_bgen_count_scan<1><<<g, kScanBlock, 0, st>>>(d, r, n, F, alo, ahi, meta, bounds, split_idx, hmax, xa, xb, xs, offs,
+                                                   (u64*)tmp);
+  scan_rest(F, offs, (u64*)tmp, st, true);
+  CF_LAUNCH_CHECK("cf_bgen_count_scan");
   return CF_OK;
 }
 

@@ -23,12 +23,11 @@
 #include "cf_dtab.cuh"
 
 extern "C" size_t cf_scan_tmp_bytes(u64 n);
-extern "C" int cf_scan_u64(const u64* in, u64 n, u64* out, void* tmp, size_t tmp_bytes, void* stream);
 extern "C" u64 cf_key_of(u64 M, u64 v);
 extern "C" size_t cf_dtab_bytes2(int bbits, int fbits);
-extern "C" int cf_bgen_count(int side, int d, int r, int n, u64 F, const u64* alo, const u64* ahi, const u32* meta,
-                             const u64* bounds, int split_idx, int hmax, int xa, int xb, u64* cnt, u32* xs,
-                             void* stream);
+extern "C" int cf_bgen_count_scan(int side, int d, int r, int n, u64 F, const u64* alo, const u64* ahi,
+                                  const u32* meta, const u64* bounds, int split_idx, int hmax, int xa, int xb, u32* xs,
+                                  u64* offs, void* tmp, size_t tmp_bytes, void* stream);
 extern "C" int cf_bgen_expand(int side, int d, int r, int n, u64 F, const void* pool, const u64* key, const u64* alo,
                               const u64* ahi, const u64* id, const u32* meta, const u64* offs, const u32* xs,
                               int split_idx, int bitmask, u64 c0, u64 cc, u64* okey, u64* oalo, u64* oahi, u64* oid,
@@ -102,15 +101,13 @@ int expand_side(int side, int r, int n, const void* pool, const u64* bounds, u64
   if (e == cudaSuccess) e = cudaMemcpyAsync(cur.meta, hostw + 4, 4, cudaMemcpyHostToDevice, st);
   if (e != cudaSuccess) return cf_cuda_status(e, "cf_bounded_join: root");
   for (int d = 0; d < r; ++d) {
-    u64* cnt = (u64*)bump.take(cur.F * 8);
     cur.xs = (u32*)bump.take(cur.F * 4);
     cur.offs = (u64*)bump.take((cur.F + 1) * 8);
     const size_t sb = cf_scan_tmp_bytes(cur.F);
     void* stmp = bump.take(sb);
     if (!bump.ok) return CF_ENOMEM;
-    int rc = cf_bgen_count(side, d, r, n, cur.F, cur.alo, cur.ahi, cur.meta, bounds, split_idx, hmax, 0, n, cnt,
-                           cur.xs, st);
-    if (rc == CF_OK) rc = cf_scan_u64(cnt, cur.F, cur.offs, stmp, sb, st);
+    int rc = cf_bgen_count_scan(side, d, r, n, cur.F, cur.alo, cur.ahi, cur.meta, bounds, split_idx, hmax, 0, n, cur.xs,
+                                cur.offs, stmp, sb, st);
     if (rc != CF_OK) return rc;
     e = cudaMemcpyAsync(hostw + 5, cur.offs + cur.F, 8, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);

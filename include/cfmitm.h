@@ -281,6 +281,10 @@ int cf_scan_u64(const uint64_t* in, uint64_t n, uint64_t* out, void* tmp, size_t
 int cf_bgen_count(int side, int d, int r, int n, uint64_t F, const uint64_t* alo, const uint64_t* ahi,
                   const uint32_t* meta, const uint64_t* bounds, int split_idx, int hmax, int xa, int xb,
                   uint64_t* cnt, uint32_t* xs, void* stream);
+/* cf_bgen_count and cf_scan_u64 of its counts in fewer launches (tmp: cf_scan_tmp_bytes(F)). */
+int cf_bgen_count_scan(int side, int d, int r, int n, uint64_t F, const uint64_t* alo, const uint64_t* ahi,
+                       const uint32_t* meta, const uint64_t* bounds, int split_idx, int hmax, int xa, int xb,
+                       uint32_t* xs, uint64_t* offs, void* tmp, size_t tmp_bytes, void* stream);
 int cf_bgen_expand(int side, int d, int r, int n, uint64_t F, const void* pool, const uint64_t* key,
                    const uint64_t* alo, const uint64_t* ahi, const uint64_t* id, const uint32_t* meta,
                    const uint64_t* offs, const uint32_t* xs, int split_idx, int bitmask, uint64_t c0, uint64_t cc,
