@@ -49,7 +49,7 @@ constexpr u32 kCjWords2 = 32768;         // resolve: filter words of the survivo
 constexpr u32 kCjHeads = 16384;          // resolve: chain heads of the build records that pass it (64 KB)
 constexpr u32 kCjChunk = 128;            // survivors per chunk
 constexpr u32 kCjRoundChunks = 16;       // resolve: chunks a warp takes per round (65,536 survivors a round)
-constexpr u32 kCjListCap = 32768;        // resolve: build records one round may keep
+constexpr u32 kCjListCap = 32768;        // resolve: build records one round may keep, at most (see listcap)
 constexpr u32 kCjCands = kCjWords2 / 4;  // resolve: record pairs equal mod d and m' in one round (64 KB)
 constexpr u32 kCjMaxD = 8192;            // class modulus
 constexpr u64 kCjMaxList = 1ull << 24;   // prefixes or suffixes of one side
@@ -80,6 +80,7 @@ struct CfClassPlan {
   u64 i_lo, i_n;
   u64 zero_bytes;
   u32 maxchunks, maxcands;
+  u32 listcap, pad;
   u64 oCtr, oBins, oHeads, oUnits, oInv, oRowBase, oRowTot, oRowCnt, oTmp, oBm, oCmeta, oChunkV, oChunks, oList, oCands;
   CjSide side[2];          // 0: build side, 1: probe side
 };
@@ -684,7 +685,7 @@ __global__ void __launch_bounds__(kCjBlock, 1) k_cj_resolve(const __grid_constan
   __shared__ u32 s_unit, s_n, s_m, s_at;
   u32* ctr = at<u32>(a, a.p.oCtr);
   const u32 nblk = ctr[kCtrNb0];
-  CjKept* list = at<CjKept>(a, a.p.oList) + (size_t)blockIdx.x * kCjListCap;
+  CjKept* list = at<CjKept>(a, a.p.oList) + (size_t)blockIdx.x * a.p.listcap;
   for (;;) {
     __syncthreads();
     if (threadIdx.x == 0) s_unit = atomicAdd(ctr + kCtrResolve, 1u);
@@ -713,7 +714,7 @@ __global__ void __launch_bounds__(kCjBlock, 1) k_cj_resolve(const __grid_constan
         cj_place2(V >> 3, w, m);
         if ((s_bm[w] & m) == m) {
           const u32 k = atomicAdd(&s_n, 1u);
-          if (k < kCjListCap) {
+          if (k < a.p.listcap) {
             CjKept e;
             e.V = V;
             e.p = p;
@@ -727,7 +728,7 @@ __global__ void __launch_bounds__(kCjBlock, 1) k_cj_resolve(const __grid_constan
       });
       __syncthreads();
       // the kept records' own filter (64 KB of the first one's place): nearly every survivor stops there
-      const u32 kept = min(s_n, kCjListCap);
+      const u32 kept = min(s_n, a.p.listcap);
       for (u32 i = threadIdx.x; i < kCjWords2 / 8; i += kCjBlock) ((uint4*)s_bm)[i] = make_uint4(0u, 0u, 0u, 0u);
       __syncthreads();
       for (u32 i = threadIdx.x; i < kept; i += kCjBlock) {
@@ -989,11 +990,14 @@ extern "C" int cf_class_plan(u64 m, int nD, int nI, int r, u64 i_lo, u64 i_n, in
     sd.oPW = off; off = up256(off + sd.nP * 8ull);
     sd.oPI = off; off = up256(off + sd.nP * 4ull);
   }
-  P->oBm = off; off = up256(off + (u64)phi * kCjWords * 4);
+  // the filters are read by the probe, the kept records' lists by the resolve after it: one place.  A round
+  // keeps about one build record in fifty, and the candidates of one round bound the true matches
+  P->listcap = (u32)std::min<double>(kCjListCap, per / 8 + kCjCands + 4096);
+  P->oBm = P->oList = off;
+  off = up256(off + std::max((u64)phi * kCjWords * 4, 148ull * P->listcap * sizeof(CjKept)));
   P->oCmeta = off; off = up256(off + (u64)P->maxchunks * 8);
   P->oChunkV = off; off = up256(off + (u64)P->maxchunks * kCjChunk * 4);
   P->oChunks = off; off = up256(off + (u64)P->maxchunks * kCjChunk * 8);
-  P->oList = off; off = up256(off + 148ull * kCjListCap * sizeof(CjKept));
   // record pairs that agree mod d and m' by chance, V within one: twice 3 n n' / (phi m') and more
   const double cands = 65536.0 + 6.0 * n_build * n_probe / ((double)phi * mp);
   if (cands > 1e8) return CF_OK;

@@ -136,8 +136,15 @@ class BatchSolver:
         t = self._bufs.get(key)
         if t is None or t.numel() < nbytes:
             self._drop_graphs()
-            with self.torch.cuda.stream(self._torch_stream()):
+            st = self._torch_stream()
+            # the memory is the caller's stream's, where the next solver finds it again: a set's own stream is
+            # a new one in each solver
+            pool = st if self._capture is not None else self._base_stream()
+            with self.torch.cuda.stream(pool):
                 t = self.torch.empty(max(nbytes, 16), dtype=self.torch.uint8, device=self.device)
+            if st != pool:
+                st.wait_stream(pool)             # what used the memory before
+                t.record_stream(st)
             self._bufs[key] = t
         return t
 

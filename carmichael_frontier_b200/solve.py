@@ -141,6 +141,11 @@ def _i_lo(plan: dict) -> int:
     return int(plan.get("i_lo") or 0)
 
 
+def _ws_bytes(cp: bytes) -> int:
+    """Workspace bytes of a class plan."""
+    return int(np.frombuffer(cp, dtype=np.uint64, count=1, offset=24)[0])
+
+
 def _pow2ceil(x: int) -> int:
     return 1 if x <= 1 else 1 << (x - 1).bit_length()
 
@@ -258,6 +263,8 @@ class Solver:
         self.tables = DeviceTables(self.device, stream=stream, async_upload=True)
         self._bufs: dict[str, object] = {}
         self._rows = self.READBACK_ROWS  # checked rows that come back with a solve's counters
+        self._pool = None                # solve_many: the caller's stream, from whose memory _buf allocates, so
+                                         # that the next solver finds it again (its own streams are new ones)
         self._bufset = 0                 # which of two buffer sets the next enqueue uses (solve_many)
         self.d2h_bytes = 0               # bytes read back from the device by collect()
         self._pinned: dict = {}
@@ -272,7 +279,15 @@ class Solver:
         if t is None or t.numel() < nbytes:
             if t is not None:                  # a growing buffer grows by half at least: few reallocations in a list
                 nbytes = max(nbytes, t.numel() * 3 // 2)
-            t = self.torch.empty(max(nbytes, 16), dtype=self.torch.uint8, device=self.device)
+            if self._pool is None:
+                t = self.torch.empty(max(nbytes, 16), dtype=self.torch.uint8, device=self.device)
+            else:
+                st = self._torch_stream()
+                with self.torch.cuda.stream(self._pool):
+                    t = self.torch.empty(max(nbytes, 16), dtype=self.torch.uint8, device=self.device)
+                if st != self._pool:
+                    st.wait_stream(self._pool)     # what used the memory before, on the caller's stream
+                    t.record_stream(st)
             self._bufs[key] = t
         return t
 
@@ -377,7 +392,7 @@ class Solver:
             _ok, d, mp, _phi = np.frombuffer(cp, dtype=np.uint32, count=4, offset=8).tolist()
             q.class_plan = C.cast(C.c_char_p(cp), C.c_void_p)
             q.multD_mp, q.multD_d = multD % mp, multD % d
-            q.ws_bytes = int(np.frombuffer(cp, dtype=np.uint64, count=1, offset=24)[0])
+            q.ws_bytes = _ws_bytes(cp)
             ws = self._buf("class", q.ws_bytes)
         else:
             q.ws_bytes = lib.cf_dtab_bytes2(q.bbits, q.fbits)
@@ -743,7 +758,11 @@ class Solver:
 
         pending = None
         self._rows = int(readback_rows)
+        self._pool = base
         try:
+            for k in range(min(2, len(insts)) if class_plans else 0):
+                with use(k):                       # the workspace of a set at once, not grown plan by plan
+                    self._buf("class", max(_ws_bytes(cp) for cp in class_plans[k::2]))
             for i in range(len(insts) + 1):
                 cur = None
                 if i < len(insts):
@@ -773,6 +792,7 @@ class Solver:
                 pending = cur
         finally:
             self._bufset = 0
+            self._pool = None
             self._rows = self.READBACK_ROWS
             self.stream, self.tables.stream = saved
             for st in sts:
