@@ -334,12 +334,14 @@ __global__ void __launch_bounds__(256) k_cj_scatter(const __grid_constant__ CjAr
 // Scaled residue of prefix w times suffix x.
 __device__ __forceinline__ u32 cj_v(u64 w, u32 x) { return (u32)(w >> 32) * x + __umulhi((u32)w, x); }
 
-// Filter place of V: word and two bits (the second may equal the first).
-__device__ __forceinline__ void cj_place(u32 V, u32& word, u32& mask) {
+// Filter place of V: word and two bits (the second may equal the first), from the bits 22 and up of
+// V * kCjWords; returns the bits below.
+__device__ __forceinline__ u32 cj_place(u32 V, u32& word, u32& mask) {
   const u64 q = (u64)V * kCjWords;
   const u32 lo = (u32)q;
   word = (u32)(q >> 32);
   mask = (1u << (lo >> 27)) | (1u << ((lo >> 22) & 31u));
+  return lo & 0x3fffffu;
 }
 
 // One warp's share of the suffix blocks [b0, b1) of a class, 32 blocks at a time, one per lane: the
@@ -369,7 +371,8 @@ __device__ __forceinline__ CjRun cj_lookup(const CjArgs& a, const CjSide& sd, in
 
 // Run f(V, prefix entry, suffix entry) for every build-side record of class c (this warp's blocks).
 // Class rows of the smaller side are short (tens of entries), so the block set-up and the lanes past
-// their last prefix weigh as much as the records: 7.6e6 records in 49 us (build) at 144 classes.
+// their last prefix weigh as much as the records: 7.6e6 records in 30 us (build) at 144
+// classes; 49 with the places of V - 1 and V + 1 computed for every record.
 template <int U, class F>
 __device__ __forceinline__ void cj_sweep(const CjArgs& a, const CjSide& sd, int s, u32 c, u32 nblk, F f) {
   const u32 lane = threadIdx.x & 31;
@@ -427,13 +430,13 @@ __global__ void __launch_bounds__(kCjBlock, 1) k_cj_build(const __grid_constant_
     const u32 c = at<u32>(a, a.p.oUnits)[ci];
     cj_sweep_u(a, a.p.side[0], 0, c, nblk, [&](u32 V, u32, u32) {
       u32 w0, m0;
-      cj_place(V, w0, m0);
+      const u32 rest = cj_place(V, w0, m0);
       atomicOr(&s_bm[w0], m0);
-#pragma unroll
-      for (int k = -1; k <= 1; k += 2) {           // the neighbours of V nearly always share its place
-        u32 w1, m1;
-        cj_place(V + (u32)k, w1, m1);
-        if (w1 != w0 || m1 != m0) atomicOr(&s_bm[w1], m1);
+      // V - 1 and V + 1 have the same place unless kCjWords less or more leaves the bits below it: 1 in 85 each
+      const bool down = rest < kCjWords, up = rest >= 0x400000u - kCjWords;
+      if (down || up) {
+        cj_place(down ? V - 1u : V + 1u, w0, m0);
+        atomicOr(&s_bm[w0], m0);
       }
     });
     __syncthreads();
@@ -891,13 +894,12 @@ extern "C" int cf_class_plan(u64 m, int nD, int nI, int r, u64 i_lo, u64 i_n, in
   const double want = std::max(140.0, n_build / 100000);
   struct Cand { double score; u32 mask, d, phi; };
   std::vector<Cand> cs;
-  for (u32 mask = 0; mask < (1u << f.size()); ++mask) {
-    u64 d = 1, phi = 1;
-    for (size_t i = 0; i < f.size() && d <= kCjMaxD; ++i)
-      if (mask >> i & 1) { d *= f[i].first; phi *= f[i].first - 1; }
-    if (d > kCjMaxD) continue;
-    cs.push_back({fabs(log2((double)phi / want)) + 0.4 * log2(ceil(phi / 148.0) * 148.0 / (double)phi), mask, (u32)d, (u32)phi});
-  }
+  cs.push_back({0.0, 0u, 1u, 1u});                 // the subsets of f with a product up to kCjMaxD: about 130 of 2^14
+  for (size_t i = 0; i < f.size(); ++i)            // (a walk over all masks took half of a plan's 40 us)
+    for (size_t k = 0, n = cs.size(); k < n; ++k)
+      if (cs[k].d * f[i].first <= kCjMaxD)
+        cs.push_back({0.0, cs[k].mask | 1u << i, (u32)(cs[k].d * f[i].first), (u32)(cs[k].phi * (f[i].first - 1))});
+  for (Cand& x : cs) x.score = fabs(log2(x.phi / want)) + 0.4 * log2(ceil(x.phi / 148.0) * 148.0 / x.phi);
   std::sort(cs.begin(), cs.end(), [](const Cand& x, const Cand& y) { return x.score < y.score || (x.score == y.score && x.mask < y.mask); });
   u64 mp = 0;
   size_t pick = 0;
