@@ -221,6 +221,11 @@ __device__ __forceinline__ SegScale seg_map(const SegCtl* c) {
 // otherwise by plain coalesced loads.  Each item's digit (DB + 1 bits, R = no
 // item) rides in the top bits of its local offset.
 // MSD: the digit is taken from the scaled key (SegScale) instead of the key.
+//
+// Bound by the shared-memory pipe (69% busy) and barriers (a quarter of the stalls): about 50
+// wavefronts per 32 records for ranking, staging and write-out, DRAM at 32% under the profiler.  Peers
+// found by 8 ballots instead of the shared mask: 7% slower; two items ranked at a time: no difference;
+// tiles of 2048 records on 256 threads, four CTAs per SM: 5% slower (runs of 64 bytes, twice the status words).
 template <int DB, bool BULK, typename SW, bool MSD>
 __global__ void __launch_bounds__(kSortBlock, 2)
 k_sort_pass(const u64* __restrict__ kin, const u64* __restrict__ iin, u64* __restrict__ kout,
@@ -363,10 +368,57 @@ k_sort_pass(const u64* __restrict__ kin, const u64* __restrict__ iin, u64* __res
   }
   __syncthreads();
   if (threadIdx.x < R) {
-    const int d = threadIdx.x;
     u32 add = 0;
     for (int w = 0; w < wid; ++w) add += s_scan[w];
-    s_doff[d] += add;
+    s_doff[threadIdx.x] += add;
+  }
+  __syncthreads();
+  // keys and ids are staged before the look-back, while the predecessors publish their counts (2^26
+  // records of 61 bits, LSD: 8-bit passes 6.28 -> 6.08 ms, 9-bit 6.54 -> 6.33 against the look-back first
+  // and the ids staged after the keys were written)
+  {
+    u32 add[kSortItems];
+#pragma unroll
+    for (int it = 0; it < kSortItems; ++it) {
+      const u32 d = loc[it] >> 16;
+      add[it] = d < kNone ? s_doff[d] + (u32)wc[d] : 0u;
+    }
+#pragma unroll
+    for (int it = 0; it < kSortItems; ++it) {
+      const u32 d = loc[it] >> 16;
+      if (d < kNone) {
+        const u32 l = (loc[it] & 0xffffu) + add[it];
+        loc[it] = l | (d << 16);
+        s_kin[l] = key[it];
+        s_dj[l] = (Dig)d;
+      }
+    }
+  }
+  bool lost = keys_lost;
+  if (BULK) {
+    bool ok = mbar_wait(&s_bar[1], 0, kMbarLimit);
+    if (!ok) {
+      atomicOr(err, CF_ERR_SPIN_LIMIT);
+      ok = mbar_wait(&s_bar[1], 0, kMbarLimit);
+    }
+    lost |= !ok;
+  }
+  {
+    u64 idv[kSortItems];
+#pragma unroll
+    for (int it = 0; it < kSortItems; ++it) {
+      const int e = wid * 32 * kSortItems + it * 32 + lane;
+      idv[it] = (loc[it] >> 16) < kNone ? s_iin[e] : 0ull;
+    }
+    lost = __syncthreads_or(lost) != 0;
+    if (!lost) {
+#pragma unroll
+      for (int it = 0; it < kSortItems; ++it)
+        if ((loc[it] >> 16) < kNone) s_iin[loc[it] & 0xffffu] = idv[it];
+    }
+  }
+  if (threadIdx.x < R) {
+    const int d = threadIdx.x;
     u64 excl = 0;
     if (tile > 0) {
       // decoupled look-back, kLookWin predecessors per round trip, bounded.  Tile 0
@@ -401,62 +453,17 @@ k_sort_pass(const u64* __restrict__ kin, const u64* __restrict__ iin, u64* __res
     s_gbase[d] = gexcl[d] + excl - s_doff[d];   // wraps mod 2^64; j >= s_doff[d] brings it back
   }
   __syncthreads();
-  {
-    u32 add[kSortItems];
-#pragma unroll
-    for (int it = 0; it < kSortItems; ++it) {
-      const u32 d = loc[it] >> 16;
-      add[it] = d < kNone ? s_doff[d] + (u32)wc[d] : 0u;
-    }
-#pragma unroll
-    for (int it = 0; it < kSortItems; ++it) {
-      const u32 d = loc[it] >> 16;
-      if (d < kNone) {
-        const u32 l = (loc[it] & 0xffffu) + add[it];
-        loc[it] = l | (d << 16);
-        s_kin[l] = key[it];
-        s_dj[l] = (Dig)d;
-      }
-    }
+  if (lost) {
+    // nothing is written; before the CTA gives up its shared memory, wait (bounded) once
+    // more for copies still in flight, so a late copy is unlikely to land in a later CTA's tile
+    if (keys_lost) mbar_wait(&s_bar[0], 0, kMbarLimit);
+    mbar_wait(&s_bar[1], 0, kMbarLimit);
+    return;
   }
-  __syncthreads();
   u64 dst[kSortItems];
   tile_places(s_dj, s_gbase, tr, dst);
   write_tile(s_kin, dst, kout, tr);
-  bool ids_lost = false;
-  if (BULK) {
-    bool ok = mbar_wait(&s_bar[1], 0, kMbarLimit);
-    if (!ok) {
-      atomicOr(err, CF_ERR_SPIN_LIMIT);
-      ok = mbar_wait(&s_bar[1], 0, kMbarLimit);
-    }
-    ids_lost = __syncthreads_or(!ok) != 0;
-  } else {
-    __syncthreads();
-  }
-  if (keys_lost || ids_lost) {
-    // nothing more is written; before the CTA gives up its shared memory, wait (bounded) once
-    // more for copies still in flight, so a late copy is unlikely to land in a later CTA's tile
-    if (keys_lost) mbar_wait(&s_bar[0], 0, kMbarLimit);
-    if (ids_lost || keys_lost) mbar_wait(&s_bar[1], 0, kMbarLimit);
-    return;
-  }
-  {
-    u64 idv[kSortItems];
-#pragma unroll
-    for (int it = 0; it < kSortItems; ++it) {
-      const int e = wid * 32 * kSortItems + it * 32 + lane;
-      idv[it] = (loc[it] >> 16) < kNone ? s_iin[e] : 0ull;
-    }
-#pragma unroll
-    for (int it = 0; it < kSortItems; ++it)
-      if ((loc[it] >> 16) < kNone) s_kin[loc[it] & 0xffffu] = idv[it];
-  }
-  __syncthreads();
-  // the 8-bit pass keeps the places in registers across the id wait (1.5% faster); the 9-bit pass
-  // reads them again (1% faster there)
-  if constexpr (DB != 8) tile_places(s_dj, s_gbase, tr, dst);
-  write_tile(s_kin, dst, iout, tr);
+  write_tile(s_iin, dst, iout, tr);
 }
 
 // ---------------------------------------------------------------------------
