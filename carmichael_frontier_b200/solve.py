@@ -9,12 +9,18 @@ r-subset of INS = Q \\ B0.  Because every prime q of the pool Q = Q(M) has
 
 (the reference matches P0 * prod(I) == prod(D), gpu/mitm_gpu_mstar_driver.py:214-237;
 both sides here carry the constant on the D side, so the large I side needs no
-multiplier).  Device pipeline, all on one stream:
+multiplier).  Device pipeline of the default ("fused") strategy, queued on one
+stream by one native call (cf_solve):
 
-  1. k_gen_part(D)  : every r-subset of B0, key form, scattered into residue partitions
-  2. k_gen_part(I)  : every r-subset of INS (in rank chunks if the side exceeds the budget)
-  3. k_join_part    : per partition, shared-memory table of D, stream I, emit equal pairs
-  4. k_check_pairs  : recompute residues, fp64 size screen, exact size, Korselt
+  1. class join (csrc/cf_class.cu) where the probing side has 2^22 records or more:
+     lists of prefixes and suffixes by residue class, one shared-memory filter per
+     class, every probe record tested there, survivors matched exactly;
+     else a table of the smaller side in L2 and a fused generate-and-probe of the
+     other (csrc/cf_dtab.cuh, csrc/cf_fused.cu)
+  2. k_check_pairs  : recompute residues, fp64 size screen, exact size, Korselt
+
+The "partition" strategy materialises both sides (k_gen_part, k_join_part) instead;
+the "bounded" one prunes them by the size bound (bsolve.py).
 
 then one synchronisation, a copy of the (rare) checked pairs, and host
 certification of every hit by ``certify.verify_certificate``.
@@ -736,8 +742,8 @@ class Solver:
         kernels.  With streams = 2 the two buffer sets also have a CUDA stream each, so one
         solve's table build can run beside the previous solve's probe.  The results equal
         solve_instance's on each instance (i_lo, i_limit: the same I-rank window for every
-        instance; class_plans: their class plans where the caller has them).  marks_list (optional list) receives one marks list per instance (see
-        enqueue)."""
+        instance; class_plans: their class plans where the caller has them).  marks_list (optional
+        list) receives one marks list per instance (see enqueue)."""
         torch = self.torch
         out: list = [None] * len(insts)
         base = self._torch_stream()
