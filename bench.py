@@ -395,7 +395,9 @@ def run_ours(args):
     t_path = kt["gen_D"] + kt["gen_I"] + kt["join"] + kt["probe"]
     achieved = BYTES_PER_RECORD * recs / t_path / 1e9 if t_path > 0 else None
     traffic = None     # DRAM bytes per step of the join-path kernels, scaled from the committed ncu capture
-    tfile = os.path.join(ROOT, "profiles", "k_fused_k64_r5_seed0.md")
+    by_class = args.strategy == "fused" and bool((solver._direct_plan(timed[0], None) or {}).get("class_plan"))
+    tname = "profiles/k_cj_k64_r5.md" if by_class else "profiles/k_fused_k64_r5_seed0.md"
+    tfile = os.path.join(ROOT, tname)
     if args.strategy == "fused" and os.path.exists(tfile):
         per = {}
         for line in open(tfile):
@@ -458,10 +460,14 @@ def run_ours(args):
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": (achieved / peak) if achieved else None, "traffic": traffic,
                          "traffic_source": ("ncu dram__bytes_read.sum + dram__bytes_write.sum per D and per I record "
-                                            "of one capture (profiles/k_fused_k64_r5_seed0.md), scaled by this "
+                                            f"of one capture ({tname}), scaled by this "
                                             "run's record counts" if traffic is not None else None),
-                         "kernel": ("k_fused build + probe" if solver.tuning.strategy == "fused"
-                                    else "k_gen_part + k_join_part") + " (join path, 32 B/record)",
+                         "kernel": ("k_cj lists, build, probe, resolve" if by_class else "k_fused build + probe"
+                                    if solver.tuning.strategy == "fused" else "k_gen_part + k_join_part")
+                                   + " (join path, 32 B/record)",
+                         "note": ("the materialised join's 32 B per record over the join time; the class join writes "
+                                  "no record (traffic: its DRAM bytes) and is bound by integer issue"
+                                  if by_class else None),
                          "peak_source": peak_src},
             "strategy": solver.tuning.strategy,
             "kernels": kern,
@@ -472,7 +478,7 @@ def run_ours(args):
                           "frac": n_probe / kt["probe"] / l2_ceiling,
                           "note": "one 32-byte L2 sector read per probing record; ceiling = random 32-B loads/s "
                                   "from a 32 MiB table, measured in this run (measure/cf_micro.cu)"}
-                         if kt["probe"] > 0 and l2_ceiling else None),
+                         if kt["probe"] > 0 and l2_ceiling and not by_class else None),
             "cpu_baseline": cpu,
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": h2d // max(1, len(timed)),
                     "d2h_bytes_per_step": d2h // max(1, len(timed)), "api": "carmichael_frontier_b200.solve_many",
