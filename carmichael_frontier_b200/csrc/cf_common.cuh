@@ -128,8 +128,7 @@ struct CfPoolHdr {
   u64 a, n, R;
   u64 mult_key;    // key(mult mod M): first factor of every product
   u64 total;       // C(n, R) (saturated)
-  u64 inv2a;       // (2^a)^-1 mod m                  (canonical conversion)
-  u64 inv2aR;      // (2^a)^-1 * 2^64 mod m           (canonical conversion)
+  u64 unused[2];   // 0
   u64 r2;          // 2^128 mod m
   u64 one_key;     // key(1)
   u64 fast32;      // 1 if every prime < 2^31 (fast path available)

@@ -135,9 +135,6 @@ static int pool_fill(const u64* primes, int n, int r, const HostMod& h, u64 mult
   hd->mult_key = host_key2(h, mult_odd, mult2);
   hd->one_key = host_key2(h, 1, 1);
   hd->r2 = h.r2;
-  const u64 half = (h.m + 1) / 2;          // 2^-1 mod m (m odd)
-  hd->inv2a = mod_pow(half, (u64)h.a, h.m);
-  hd->inv2aR = (u64)((u128)hd->inv2a * h.Rm % h.m);
   u64 maxp = 0;
   for (int i = 0; i < n; ++i) maxp = primes[i] > maxp ? primes[i] : maxp;
   hd->fast32 = (maxp < (1ull << 31)) ? 1 : 0;
