@@ -24,6 +24,7 @@ ERR_PAIR_OVERFLOW = 2
 ERR_TABLE_FULL = 4
 ERR_SPIN_LIMIT = 8
 ERR_KEY_MISMATCH = 16
+ERR_BAD_ARG = 32
 
 HIT_KEY_EQUAL = 1
 HIT_SCREEN = 2
@@ -59,7 +60,7 @@ SIGNATURES = [
     ("cf_screen_bytes", sz, []),
     ("cf_screen_prepare", C.c_int, [vp, C.c_int, C.c_double, C.c_double, C.c_double, vp, sz]),
     ("cf_gen_subsets", C.c_int, [vp, C.c_int, C.c_int, u64, u64, C.c_int, C.c_int, C.c_int, vp, vp, vp]),
-    ("cf_gen_subsets_tail", C.c_int, [vp, vp, C.c_int, C.c_int, u64, u64, C.c_int, C.c_int, C.c_int, vp, vp, vp]),
+    ("cf_gen_subsets_tail", C.c_int, [vp, vp, C.c_int, C.c_int, u64, u64, C.c_int, C.c_int, C.c_int, vp, vp, vp, vp]),
     ("cf_tail_bytes", sz, [C.c_int, C.c_int]),
     ("cf_build_tail", C.c_int, [vp, C.c_int, C.c_int, vp, vp]),
     ("cf_gen_part_shapes", C.c_int, []),

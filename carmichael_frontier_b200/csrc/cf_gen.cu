@@ -107,12 +107,15 @@ k_gen_linear(const u64* __restrict__ pool, u64 lo, u64 count, int id_mode, int b
 template <int R>
 __global__ void __launch_bounds__(kLinBlock)
 k_gen_tail(const u64* __restrict__ pool, const CfTailEnt* __restrict__ tail, u64 lo, u64 count, u32 steps, int id_mode,
-           int bits, int canon, u64* __restrict__ keys, u64* __restrict__ ids) {
+           int bits, int canon, u64* __restrict__ keys, u64* __restrict__ ids, u32* __restrict__ err) {
   constexpr int B = 2, A = R - B;
   __shared__ u32 s_p[CF_MAX_POOL];
   const CfPoolHdr* hd = (const CfPoolHdr*)pool;
   const int n = (int)hd->n;
-  if (!hd->fast32 || hd->tail_b != (u64)B) return;     // the caller sends other pools to k_gen_linear
+  if (!hd->fast32 || hd->tail_b != (u64)B) {           // no table of two-prime suffixes: nothing is written
+    if (err && threadIdx.x == 0) atomicOr(err, CF_ERR_BAD_ARG);
+    return;
+  }
   const u64* pr = pool + cf_pool_off_prime(n);
   for (int i = threadIdx.x; i < n; i += kLinBlock) s_p[i] = (u32)pr[i];
   __syncthreads();
@@ -346,14 +349,14 @@ void launch_gen_linear(const u64* pool, u64 lo, u64 count, int id_mode, int bits
 
 template <int R>
 void launch_gen_tail(const u64* pool, const CfTailEnt* tail, u64 lo, u64 count, int id_mode, int bits, int canon,
-                     u64* keys, u64* ids, cudaStream_t st) {
+                     u64* keys, u64* ids, u32* err, cudaStream_t st) {
   if constexpr (R >= 3) {
     // a warp's start (unranking) is a chain of some hundred loads: longer ranges once they still fill the GPU
     // (1.0e7 records: 73 us with 32 steps, 81 with 64; the next entry loaded a step ahead: 92)
     const u32 steps = count >= (1u << 22) ? 32u : 16u;
     const u64 per = (u64)kLinBlock * steps;
     k_gen_tail<R><<<(unsigned)((count + per - 1) / per), kLinBlock, 0, st>>>(pool, tail, lo, count, steps, id_mode, bits,
-                                                                            canon, keys, ids);
+                                                                            canon, keys, ids, err);
   }
 }
 
@@ -444,10 +447,21 @@ extern "C" int cf_gen_subsets(const void* pool_dev, int n, int r, u64 lo, u64 co
   return CF_OK;
 }
 
-// cf_gen_subsets for a pool whose tail table (cf_build_tail) the caller has: primes below 2^31, 2-adic
-// part of M at most 2^32, r >= 3.
+// C(n, k), saturated at 2^64 - 1 (k <= 10).
+static u64 host_binom(int n, int k) {
+  if (k < 0 || k > n) return 0;
+  unsigned __int128 v = 1;
+  for (int i = 1; i <= k; ++i) v = v * (unsigned)(n - k + i) / (unsigned)i;
+  return v >> 64 ? ~0ull : (u64)v;
+}
+
+// cf_gen_subsets for a pool whose tail table (cf_build_tail) the caller has, r >= 3.  The ranks must lie in
+// [0, C(n, r)): beyond, the walker would read past the table.  *err (device, or null) receives
+// CF_ERR_BAD_ARG, and nothing is written, for a pool that has no table of two-prime suffixes (primes of
+// 2^31 or more, 2-adic part of M above 2^32); a second walker in the kernel for such pools would slow the
+// others (its call alone: 72 -> 84 us for 1.0e7 records at r = 4).
 extern "C" int cf_gen_subsets_tail(const void* pool_dev, const void* tail, int n, int r, u64 lo, u64 count, int id_mode,
-                                   int bits, int canon, u64* keys, u64* ids, void* stream) {
+                                   int bits, int canon, u64* keys, u64* ids, u32* err, void* stream) {
   if (!pool_dev || !tail || n < 1 || n > CF_MAX_POOL || r < 3 || r > CF_MAX_DISPATCH_R || r > n) {
     cf_set_error("cf_gen_subsets_tail: bad pool arguments (n 1..1024, r 3..10)%s", "");
     return CF_EBADARG;
@@ -459,8 +473,12 @@ extern "C" int cf_gen_subsets_tail(const void* pool_dev, const void* tail, int n
   if (count == 0) return CF_OK;
   if (!keys || !ids) { cf_set_error("cf_gen_subsets_tail: null output%s", ""); return CF_EBADARG; }
   if (count > (1ull << 40)) { cf_set_error("cf_gen_subsets_tail: count too large for one launch%s", ""); return CF_EBADARG; }
+  if (const u64 total = host_binom(n, r); lo > total || count > total - lo) {
+    cf_set_error("cf_gen_subsets_tail: ranks beyond C(n, r)%s", "");
+    return CF_EBADARG;
+  }
   CF_DISPATCH_R(r, launch_gen_tail, (const u64*)pool_dev, (const CfTailEnt*)tail, lo, count, id_mode, bits, canon, keys,
-                ids, (cudaStream_t)stream);
+                ids, err, (cudaStream_t)stream);
   CF_LAUNCH_CHECK("cf_gen_subsets_tail");
   return CF_OK;
 }
@@ -470,13 +488,6 @@ extern "C" int cf_gen_part_shapes(void) { return kNumShapes; }
 extern "C" size_t cf_gen_part_smem_bytes(int n, int r, int pbits, int shape) {
   if (shape < 0 || shape >= kNumShapes || pbits < 0 || pbits > 12) return 0;
   return gen_part_layout(kShapes[shape][0], kShapes[shape][1], n, r, pbits).total;
-}
-
-static u64 host_binom(int n, int k) {
-  if (k < 0 || k > n) return 0;
-  unsigned __int128 v = 1;
-  for (int i = 1; i <= k; ++i) v = v * (unsigned)(n - k + i) / (unsigned)i;
-  return (u64)v;
 }
 
 extern "C" size_t cf_tail_bytes(int n, int r) {

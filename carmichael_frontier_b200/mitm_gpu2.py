@@ -82,7 +82,7 @@ def generate(primes, r: int, M: int, mult: int = 1, bits: int = 10, lo: int = 0,
     if r >= 3 and count >= GEN_TAIL_MIN and max(primes) < 1 << 31 and M % (1 << 33):
         tail = _dtables(dev).tail(primes, r, M, mult, pool)
         _lib.check(lib.cf_gen_subsets_tail(_lib.ptr(pool), _lib.ptr(tail), n, r, lo, count, 0, bits, 1, _lib.ptr(keys),
-                                           _lib.ptr(ids), _lib.stream_handle()), "generate")
+                                           _lib.ptr(ids), None, _lib.stream_handle()), "generate")
     else:
         _lib.check(lib.cf_gen_subsets(_lib.ptr(pool), n, r, lo, count, 0, bits, 1, _lib.ptr(keys), _lib.ptr(ids),
                                       _lib.stream_handle()), "generate")

@@ -110,10 +110,11 @@ int cf_screen_prepare(const uint32_t* limbsB, int nlimbs, double lgP0, double lg
 int cf_gen_subsets(const void* pool_dev, int n, int r, uint64_t lo, uint64_t count, int id_mode, int bits,
                    int canon, uint64_t* keys, uint64_t* ids, void* stream);
 
-/* cf_gen_subsets through the pool's suffix table (cf_build_tail): r >= 3, primes below 2^31, 2-adic
- * part of M at most 2^32. */
+/* cf_gen_subsets through the pool's suffix table (cf_build_tail): r >= 3, ranks within [0, C(n, r)),
+ * else CF_EBADARG.  err (device word, or null) receives CF_ERR_BAD_ARG, and no record is written, when the
+ * pool has no table of two-prime suffixes (primes of 2^31 or more, 2-adic part of M above 2^32). */
 int cf_gen_subsets_tail(const void* pool_dev, const void* tail, int n, int r, uint64_t lo, uint64_t count, int id_mode,
-                        int bits, int canon, uint64_t* keys, uint64_t* ids, void* stream);
+                        int bits, int canon, uint64_t* keys, uint64_t* ids, uint32_t* err, void* stream);
 
 /* Tail table of a pool (device, cf_tail_bytes(n, r) bytes): the products of all
  * b-subsets of the pool, b = min(r, 2), in lexicographic order, 16 bytes each.
