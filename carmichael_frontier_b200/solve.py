@@ -274,6 +274,7 @@ class Solver:
         self._bufset = 0                 # which of two buffer sets the next enqueue uses (solve_many)
         self.d2h_bytes = 0               # bytes read back from the device by collect()
         self._pinned: dict = {}
+        self._queued: dict = {}          # buffer set -> handle of the solve queued on it and not collected
         self._bounded = None
         self.result_bytes = self.lib.cf_pair_result_bytes()
         assert self.result_bytes == RESULT_DTYPE.itemsize
@@ -297,15 +298,31 @@ class Solver:
             self._bufs[key] = t
         return t
 
-    def _pinned_buf(self, name: str, nbytes: int):
+    def _pinned_buf(self, name: str, nbytes: int, dev=None):
         """Page-locked host buffer of the current buffer set (rewritten only after the solve that
-        last used it has been collected)."""
+        last used it has been collected, see _leave_staging).
+        dev: the device buffer that a native call copies to or from it.  Torch, which hands freed
+        page-locked memory out again, does not see such a copy, so one byte goes up through torch once per
+        buffer and stream: the memory, once freed, then waits for that stream."""
         key = (name, self._bufset)
-        t = self._pinned.get(key)
+        t, streams = self._pinned.get(key) or (None, None)
         if t is None or t.numel() < nbytes:
-            t = self.torch.empty(max(nbytes, 64), dtype=self.torch.uint8, pin_memory=True)
-            self._pinned[key] = t
+            t, streams = self.torch.empty(max(nbytes, 64), dtype=self.torch.uint8, pin_memory=True), set()
+            self._pinned[key] = t, streams
+        if dev is not None:
+            sh = self._sh()
+            if sh not in streams:
+                with self.torch.cuda.stream(self._torch_stream()):
+                    dev[:1].copy_(t[:1], non_blocking=True)
+                streams.add(sh)
         return t
+
+    def _leave_staging(self):
+        """Before a solve's tables are staged: page-locked buffers that a solve queued on this set and not
+        collected may still read or write are left to it (freed, they wait for its stream)."""
+        if self._queued.pop(self._bufset, None) is not None:
+            for name in ("stage", "readback", "pdesc"):
+                self._pinned.pop((name, self._bufset), None)
 
     def _sh(self):
         return _lib.stream_handle(self.stream)
@@ -341,9 +358,14 @@ class Solver:
         """Queue the whole device pipeline for `inst` on the stream (no host sync).
         `marks` (optional list) receives (tag, CUDA event) pairs around every kernel."""
         if plan.get("strategy", "fused") == "fused":
+            self._leave_staging()
+            self._queued[self._bufset] = True      # also when a launch below fails
             pshape = self._part_shape(inst, plan)
-            return self._enqueue_solve(inst, plan, marks) if pshape is None \
+            h = self._enqueue_solve(inst, plan, marks) if pshape is None \
                 else self._enqueue_fused(inst, plan, pshape, marks)
+            h["set"] = self._bufset
+            self._queued[self._bufset] = h
+            return h
         return self._enqueue_partition(inst, plan, marks)
 
     def _side_tables(self, inst: Instance, side: str):
@@ -393,7 +415,8 @@ class Solver:
         # L2-resident while built); larger tables the wide entries
         q.side_format = 1 if q.bbits <= 20 else 0
         tb = lib.cf_solve_table_bytes(len(pD), len(pI), r)
-        stage, tabs = self._pinned_buf("stage", tb), self._buf("tables", tb)
+        tabs = self._buf("tables", tb)
+        stage = self._pinned_buf("stage", tb, tabs)
         if cp:
             _ok, d, mp, _phi = np.frombuffer(cp, dtype=np.uint32, count=4, offset=8).tolist()
             q.class_plan = C.cast(C.c_char_p(cp), C.c_void_p)
@@ -409,7 +432,7 @@ class Solver:
         rb = self.result_bytes
         rows = max(0, min(self._rows, maxp))
         pairs, res, ctr = self._buf("pairs", maxp * 16), self._buf("res", maxp * rb), self._buf("ctr", 64)
-        hm = self._pinned_buf("readback", 8 + rows * rb)
+        hm = self._pinned_buf("readback", 8 + rows * rb, ctr)
         q.stage, q.tables, q.ws, q.pairs, q.results, q.misc = \
             stage.data_ptr(), dp(tabs), dp(ws), dp(pairs), dp(res), dp(ctr)
         q.max_pairs, q.rows, q.readback = maxp, rows, hm.data_ptr()
@@ -596,6 +619,8 @@ class Solver:
             ev.synchronize()
             misc = h["hread"][:8].numpy().view(np.uint32).copy()
             self.d2h_bytes += 8 + h["hrows"] * self.result_bytes
+        if self._queued.get(h.get("set")) is h:
+            del self._queued[h["set"]]
         npairs, err = int(misc[0]), int(misc[1])
         plan = h["plan"]
         if err & _lib.ERR_TABLE_FULL:
