@@ -497,6 +497,8 @@ class Solver:
         nD, nI = ncomb(len(inst.B0), inst.r), _i_window(inst, plan)
         if not tu.class_join or plan.get("no_class") or max(nD, nI) < tu.class_min_probe or not tu.l2_table_bytes:
             return None                       # (no L2 for tables: the caller wants the table join's filter level)
+        if (inst.B0[-1] | inst.INS[-1]) >> 31:
+            return None                       # the class join's kernels multiply 32-bit factors
         out = np.zeros(lib.cf_class_plan_bytes(), dtype=np.uint8)
         _lib.check(lib.cf_class_plan(split_modulus(inst.M)[0], len(inst.B0), len(inst.INS), inst.r, _i_lo(plan), nI,
                                      int(bool(plan.get("swap"))), out.ctypes.data, out.nbytes), "cf_class_plan")
