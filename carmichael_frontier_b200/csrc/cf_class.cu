@@ -863,7 +863,7 @@ extern "C" size_t cf_class_plan_bytes(void) { return sizeof(CfClassPlan); }
 // join does not apply: no class modulus with about the wanted number of classes and an m' of at
 // least 2^27 beside it, lists above 2^24 entries, or a radius outside 2..8.  Host code, no device call.
 extern "C" int cf_class_plan(u64 m, int nD, int nI, int r, u64 i_lo, u64 i_n, int swap, void* plan,
-                             size_t plan_bytes) {
+                             size_t plan_bytes) try {
   if (!plan || plan_bytes < sizeof(CfClassPlan) || nD < 1 || nI < 1 || nD > CF_MAX_POOL || nI > CF_MAX_POOL) {
     cf_set_error("cf_class_plan: bad arguments%s", "");
     return CF_EBADARG;
@@ -1008,6 +1008,9 @@ extern "C" int cf_class_plan(u64 m, int nD, int nI, int r, u64 i_lo, u64 i_n, in
   P->ws_bytes = off;
   P->ok = 1;
   return CF_OK;
+} catch (...) {                                    // the lists of divisors did not fit host memory
+  cf_set_error("cf_class_plan: out of host memory%s", "");
+  return CF_ENOMEM;
 }
 
 // Run a planned class join on the stream: equal-residue pairs {D rank, I rank} are appended through

@@ -1,13 +1,15 @@
 """Which instances take the class join: decided on the host, so tested without a GPU."""
 import math
+import os
 
 import pytest
 
-from carmichael_frontier_b200 import Instance, Solver, Tuning
+from carmichael_frontier_b200 import Instance, Solver, Tuning, _lib
 from carmichael_frontier_b200.workloads import eligible_pool
 
 M = 2 ** 6 * 3 ** 3 * 5 ** 2 * 7 * 11 * 13 * 17 * 19 * 23 * 29
 Q = eligible_pool(M, 10 ** 5)
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 def instance(k, n, r):
@@ -28,3 +30,34 @@ def test_primes_of_2_31_or_more_do_not_take_the_class_join(side):
     getattr(x, side)[-1] = (1 << 31) + 11
     x.P0 = math.prod(x.B0)
     assert class_plan(x) is None
+
+
+EXHAUSTED = """
+import ctypes as C, resource, sys
+from carmichael_frontier_b200 import _lib
+lib = _lib.load()
+libc = C.CDLL(None)
+libc.malloc.restype = C.c_void_p
+libc.malloc.argtypes = [C.c_size_t]
+n = lib.cf_class_plan_bytes()
+out = C.create_string_buffer(n)
+at, m, i_n = C.addressof(out), %d, %d
+assert lib.cf_class_plan(m, 64, 120, 4, 0, i_n, 0, at, n) == _lib.CF_OK
+assert lib.cf_class_plan(m, 0, 120, 4, 0, i_n, 0, at, n) == _lib.CF_EBADARG   # this thread's error text exists
+pages = int(open("/proc/self/statm").read().split()[0])
+resource.setrlimit(resource.RLIMIT_AS, (pages * resource.getpagesize(),) * 2)
+for size in (1 << 20, 1 << 12, 256, 64, 16):
+    while libc.malloc(size):
+        pass
+rc = lib.cf_class_plan(m, 64, 120, 4, 0, i_n, 0, at, n)
+sys.stdout.write("status %%d" %% rc)
+"""
+
+
+def test_a_plan_without_host_memory_returns_a_status():
+    # an exception that leaves a C function ends the process
+    import subprocess
+    import sys
+    p = subprocess.run([sys.executable, "-c", EXHAUSTED % (M // (M & -M), math.comb(120, 4))], capture_output=True,
+                       text=True, cwd=ROOT, timeout=120)
+    assert p.returncode == 0 and p.stdout in (f"status {_lib.CF_OK}", f"status {_lib.CF_ENOMEM}"), (p.returncode, p.stderr[-500:])
