@@ -167,7 +167,7 @@ class BoundedSolve:
 
         k = 76, r = 6, 1.4e8 D records, 4.3e9 I leaves: 124 ms as a level loop with leaf probes, 16.5 ms on
         the device here (1.4 of it the counts); k = 78, r = 4, 1.4e6 and 2.6e7: 0.89 against 0.64 ms in all."""
-        from .solve import RESULT_DTYPE, Instance
+        from .solve import RESULT_DTYPE, Instance, _ws_bytes, class_pairs
         lib, dp, s = self.lib, _lib.ptr, self.s
         r, M = inst.r, inst.M
         if Icap <= 1 or Dmin >= U128:
@@ -206,9 +206,12 @@ class BoundedSolve:
         if bD == 0 or bI == 0:
             return [], bD, bI, out
         _ok, d, mp, _phi = np.frombuffer(cp, dtype=np.uint32, count=4, offset=8).tolist()
-        ws_bytes = int(np.frombuffer(cp, dtype=np.uint64, count=1, offset=24)[0])
-        ws = s._buf("class", ws_bytes)
-        maxp = max(s.tuning.pair_capacity, min(1 << 22, 1 << (8 * nD * nI // M).bit_length()))
+        ws_bytes = _ws_bytes(cp)
+        try:
+            ws = s._buf("class", ws_bytes)
+        except self.torch.OutOfMemoryError:               # a shared device: the level loop needs less
+            return None
+        maxp = class_pairs(nD, nI, M, s.tuning)
         while True:
             pairs = s._buf("pairs", maxp * 16)
             res = s._buf("res", maxp * s.result_bytes)
@@ -220,7 +223,9 @@ class BoundedSolve:
             self.gen.launches += 10
             npairs, err = misc[:8].cpu().numpy().view(np.uint32).tolist()
             if err & _lib.ERR_PART_OVERFLOW:
-                return None                           # a survivor list ran out
+                del ws                                # a survivor list ran out; its memory goes to the level loop
+                s._bufs.pop(("class", s._bufset), None)
+                return None
             if err & _lib.ERR_PAIR_OVERFLOW:
                 maxp = max(2 * maxp, npairs + 16)
                 continue

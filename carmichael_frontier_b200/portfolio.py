@@ -37,7 +37,7 @@ import numpy as np
 from . import _lib
 from .certify import verify_certificate
 from .solve import (MOD_DTYPE, RESULT_DTYPE, Hit, Instance, SolveResult, Solver, Tuning, dtab_shape, finish_rows,
-                    part_shape)
+                    _ws_bytes, part_shape)
 from .tables import ncomb, pool_table_host, screen_table_host
 
 _ALIGN = 256
@@ -194,7 +194,8 @@ class BatchSolver:
         tu = self.tuning.dtab
         if not self.tuning.class_join or not tu.class_join or max(nD, nI) < tu.class_min_probe or tu.strategy != "fused":
             return None
-        return self._solver()._class_plan(x, dict(i_limit=i_limit, i_lo=0, swap=nI < nD))
+        cp = self._solver()._class_plan(x, dict(i_limit=i_limit, i_lo=0, swap=nI < nD, sets=2))
+        return cp if cp and 2 * _ws_bytes(cp) <= self.tuning.mem_budget else None
 
     def prepare(self, instances: list, i_limit: int | None = None) -> PreparedPortfolio:
         """Host tables of every modulus, one upload, device tail tables, batch split."""

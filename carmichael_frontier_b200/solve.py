@@ -113,6 +113,7 @@ class Tuning:
     part_lb: int = 10               # log2 buckets per range of the partitioned build (9 or 10)
     part_sigma: float = 8.0         # bucket-range capacity = mean + sigma*sqrt(mean) + 32
     class_join: bool = True         # fused: join by residue classes (csrc/cf_class.cu) where it applies
+    class_ws_bytes: int = 24 << 30  # ... and its workspace is at most this, half of it for each of a list's two
     class_min_probe: int = 1 << 22  # ... and the probing side has this many records or more (below, the
                                     # plan's 40 us of host time weigh more than the device time it saves)
 
@@ -154,6 +155,11 @@ def _ws_bytes(cp: bytes) -> int:
 
 def _pow2ceil(x: int) -> int:
     return 1 if x <= 1 else 1 << (x - 1).bit_length()
+
+
+def class_pairs(nD: int, nI: int, M: int, tu: "Tuning") -> int:
+    """Pair capacity of a class join: room for the pairs a modulus with few units has (8 nD nI / M)."""
+    return max(tu.pair_capacity, min(1 << 22, _pow2ceil(8 * nD * nI // M)))
 
 
 def _cap(mean: float, sigma: float) -> int:
@@ -284,8 +290,9 @@ class Solver:
         key = (name, self._bufset)
         t = self._bufs.get(key)
         if t is None or t.numel() < nbytes:
-            if t is not None:                  # a growing buffer grows by half at least: few reallocations in a list
-                nbytes = max(nbytes, t.numel() * 3 // 2)
+            if t is not None:                  # a growing buffer grows by half (64 MB at most) at least, the old one
+                nbytes = max(nbytes, min(t.numel() * 3 // 2, t.numel() + (64 << 20)))       # freed before it
+                del self._bufs[key], t
             if self._pool is None:
                 t = self.torch.empty(max(nbytes, 16), dtype=self.torch.uint8, device=self.device)
             else:
@@ -422,7 +429,10 @@ class Solver:
             q.class_plan = C.cast(C.c_char_p(cp), C.c_void_p)
             q.multD_mp, q.multD_d = multD % mp, multD % d
             q.ws_bytes = _ws_bytes(cp)
-            ws = self._buf("class", q.ws_bytes)
+            try:
+                ws = self._buf("class", q.ws_bytes)
+            except self.torch.OutOfMemoryError:    # a shared device: the table join needs less
+                return self.enqueue(inst, self._replan(inst, dict(plan, no_class=True)), marks)
         else:
             q.ws_bytes = lib.cf_dtab_bytes2(q.bbits, q.fbits)
             ws = self._buf("dtab", q.ws_bytes)
@@ -502,7 +512,12 @@ class Solver:
         out = np.zeros(lib.cf_class_plan_bytes(), dtype=np.uint8)
         _lib.check(lib.cf_class_plan(split_modulus(inst.M)[0], len(inst.B0), len(inst.INS), inst.r, _i_lo(plan), nI,
                                      int(bool(plan.get("swap"))), out.ctypes.data, out.nbytes), "cf_class_plan")
-        return out.tobytes() if out[8:12].view(np.uint32)[0] else None
+        if not out[8:12].view(np.uint32)[0]:
+            return None
+        # k = 64: r = 5 54 to 210 MB, r = 6 0.8 to 13 GB, r = 7 1.3 to 40 GB (the table join 0.2, 1.3 and 10)
+        cp = out.tobytes()
+        sets = 1 if self._pool is None else 2
+        return cp if _ws_bytes(cp) * plan.get("sets", sets) <= tu.class_ws_bytes else None
 
     def _part_build(self, inst: Instance, plan: dict, pshape: tuple, tables: tuple, tab, nD: int, nIt: int,
                     swap: bool, misc):
@@ -679,8 +694,8 @@ class Solver:
             plan["strategy"] = "partition"
         if plan["strategy"] == "fused":
             plan["class_plan"] = cp or self._class_plan(inst, plan)
-            if plan["class_plan"]:            # room for the pairs a modulus with few units has (8 nD nI / M)
-                plan["pairs"] = max(plan["pairs"], min(1 << 22, _pow2ceil(8 * nD * nI // inst.M)))
+            if plan["class_plan"]:
+                plan["pairs"] = class_pairs(nD, nI, inst.M, self.tuning)
         return plan
 
     def _replan(self, inst: Instance, newp: dict) -> dict:
@@ -692,6 +707,8 @@ class Solver:
         plan["i_lo"] = _i_lo(newp)
         plan["no_part"] = newp.get("no_part", False)
         plan["no_class"] = newp.get("no_class", False)
+        if plan["no_class"]:
+            self._bufs.pop(("class", self._bufset), None)   # not held beside the other join's buffers
         if plan["strategy"] == "fused":
             plan["class_plan"] = self._class_plan(inst, plan)
         return plan
@@ -795,7 +812,10 @@ class Solver:
         try:
             for k in range(min(2, len(insts)) if class_plans else 0):
                 with use(k):                       # the workspace of a set at once, not grown plan by plan
-                    self._buf("class", max(_ws_bytes(cp) for cp in class_plans[k::2]))
+                    try:
+                        self._buf("class", max(_ws_bytes(cp) for cp in class_plans[k::2]))
+                    except torch.OutOfMemoryError:
+                        pass                       # the plans that do not fit take the table join one by one
             for i in range(len(insts) + 1):
                 cur = None
                 if i < len(insts):

@@ -5,6 +5,8 @@ import os
 import pytest
 
 from carmichael_frontier_b200 import Instance, Solver, Tuning, _lib
+from carmichael_frontier_b200.portfolio import BatchSolver, BatchTuning
+from carmichael_frontier_b200.solve import _ws_bytes
 from carmichael_frontier_b200.workloads import eligible_pool
 
 M = 2 ** 6 * 3 ** 3 * 5 ** 2 * 7 * 11 * 13 * 17 * 19 * 23 * 29
@@ -30,6 +32,22 @@ def test_primes_of_2_31_or_more_do_not_take_the_class_join(side):
     getattr(x, side)[-1] = (1 << 31) + 11
     x.P0 = math.prod(x.B0)
     assert class_plan(x) is None
+
+
+def test_workspaces_above_the_limit_are_declined():
+    x = instance(64, 160, 5)
+    need = _ws_bytes(class_plan(x))
+    assert class_plan(x, class_ws_bytes=need) is not None and class_plan(x, class_ws_bytes=need - 1) is None
+    big = instance(64, 155, 6)                     # 1.5e10 I records: 10 GB, the table join 1.4
+    assert _ws_bytes(class_plan(big)) > 8 << 30 and class_plan(big, class_ws_bytes=8 << 30) is None
+    s = Solver("cuda", tuning=Tuning(class_ws_bytes=2 * need - 1))
+    plan = s.plan(math.comb(64, 5), math.comb(160, 5))
+    assert s._class_plan(x, plan) is not None
+    s._pool = object()                             # in a list: two workspaces are held
+    assert s._class_plan(x, plan) is None
+    for budget, taken in ((2 * need, True), (2 * need - 1, False)):
+        b = BatchSolver("cuda", tuning=BatchTuning(mem_budget=budget))
+        assert (b._class_plan(x, math.comb(64, 5), math.comb(160, 5), None) is not None) == taken
 
 
 EXHAUSTED = """
