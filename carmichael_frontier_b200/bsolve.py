@@ -167,7 +167,7 @@ class BoundedSolve:
 
         k = 76, r = 6, 1.4e8 D records, 4.3e9 I leaves: 124 ms as a level loop with leaf probes, 16.5 ms on
         the device here (1.4 of it the counts); k = 78, r = 4, 1.4e6 and 2.6e7: 0.89 against 0.64 ms in all."""
-        from .solve import RESULT_DTYPE, Instance, _ws_bytes, class_pairs
+        from .solve import RESULT_DTYPE, Instance, class_pairs, plan_head
         lib, dp, s = self.lib, _lib.ptr, self.s
         r, M = inst.r, inst.M
         if Icap <= 1 or Dmin >= U128:
@@ -205,8 +205,7 @@ class BoundedSolve:
         out = dict(strategy="bounded", Icap=Icap, Dmin=Dmin, table="class", class_plan=cp)
         if bD == 0 or bI == 0:
             return [], bD, bI, out
-        _ok, d, mp, _phi = np.frombuffer(cp, dtype=np.uint32, count=4, offset=8).tolist()
-        ws_bytes = _ws_bytes(cp)
+        _ok, d, mp, _phi, ws_bytes = plan_head(cp)
         try:
             ws = s._buf("class", ws_bytes)
         except self.torch.OutOfMemoryError:               # a shared device: the level loop needs less
@@ -224,7 +223,7 @@ class BoundedSolve:
             npairs, err = misc[:8].cpu().numpy().view(np.uint32).tolist()
             if err & _lib.ERR_PART_OVERFLOW:
                 del ws                                # a survivor list ran out; its memory goes to the level loop
-                s._bufs.pop(("class", s._bufset), None)
+                s._drop_class()
                 return None
             if err & _lib.ERR_PAIR_OVERFLOW:
                 maxp = max(2 * maxp, npairs + 16)

@@ -29,6 +29,7 @@ from __future__ import annotations
 
 import ctypes as C
 import math
+import struct
 from dataclasses import dataclass, field
 
 import numpy as np
@@ -148,9 +149,17 @@ def _i_lo(plan: dict) -> int:
     return int(plan.get("i_lo") or 0)
 
 
+_PLAN_HEAD = struct.Struct("<8x4IQ")
+
+
+def plan_head(cp) -> tuple[int, int, int, int, int]:
+    """(ok, class modulus, filter modulus, classes, workspace bytes) of a class plan."""
+    return _PLAN_HEAD.unpack_from(cp)
+
+
 def _ws_bytes(cp: bytes) -> int:
     """Workspace bytes of a class plan."""
-    return int(np.frombuffer(cp, dtype=np.uint64, count=1, offset=24)[0])
+    return _PLAN_HEAD.unpack_from(cp)[4]
 
 
 def _pow2ceil(x: int) -> int:
@@ -281,6 +290,8 @@ class Solver:
         self.d2h_bytes = 0               # bytes read back from the device by collect()
         self._pinned: dict = {}
         self._queued: dict = {}          # buffer set -> handle of the solve queued on it and not collected
+        self._reserved: dict = {}        # buffer set -> bytes by name that lists have reserved
+        self._class_cover = 0.0          # survivor estimate that the lists' class workspaces were reserved for
         self._bounded = None
         self.result_bytes = self.lib.cf_pair_result_bytes()
         assert self.result_bytes == RESULT_DTYPE.itemsize
@@ -425,10 +436,9 @@ class Solver:
         tabs = self._buf("tables", tb)
         stage = self._pinned_buf("stage", tb, tabs)
         if cp:
-            _ok, d, mp, _phi = np.frombuffer(cp, dtype=np.uint32, count=4, offset=8).tolist()
+            _ok, d, mp, _phi, q.ws_bytes = plan_head(cp)
             q.class_plan = C.cast(C.c_char_p(cp), C.c_void_p)
             q.multD_mp, q.multD_d = multD % mp, multD % d
-            q.ws_bytes = _ws_bytes(cp)
             try:
                 ws = self._buf("class", q.ws_bytes)
             except self.torch.OutOfMemoryError:    # a shared device: the table join needs less
@@ -509,15 +519,13 @@ class Solver:
             return None                       # (no L2 for tables: the caller wants the table join's filter level)
         if (inst.B0[-1] | inst.INS[-1]) >> 31:
             return None                       # the class join's kernels multiply 32-bit factors
-        out = np.zeros(lib.cf_class_plan_bytes(), dtype=np.uint8)
+        cp = C.create_string_buffer(lib.cf_class_plan_bytes())
         _lib.check(lib.cf_class_plan(split_modulus(inst.M)[0], len(inst.B0), len(inst.INS), inst.r, _i_lo(plan), nI,
-                                     int(bool(plan.get("swap"))), out.ctypes.data, out.nbytes), "cf_class_plan")
-        if not out[8:12].view(np.uint32)[0]:
-            return None
+                                     int(bool(plan.get("swap"))), C.addressof(cp), len(cp)), "cf_class_plan")
+        ok, _d, _mp, _phi, ws = plan_head(cp)
         # k = 64: r = 5 54 to 210 MB, r = 6 0.8 to 13 GB, r = 7 1.3 to 40 GB (the table join 0.2, 1.3 and 10)
-        cp = out.tobytes()
-        sets = 1 if self._pool is None else 2
-        return cp if _ws_bytes(cp) * plan.get("sets", sets) <= tu.class_ws_bytes else None
+        sets = plan.get("sets") or (1 if self._pool is None else 2)
+        return cp.raw if ok and ws * sets <= tu.class_ws_bytes else None
 
     def _part_build(self, inst: Instance, plan: dict, pshape: tuple, tables: tuple, tab, nD: int, nIt: int,
                     swap: bool, misc):
@@ -708,10 +716,16 @@ class Solver:
         plan["no_part"] = newp.get("no_part", False)
         plan["no_class"] = newp.get("no_class", False)
         if plan["no_class"]:
-            self._bufs.pop(("class", self._bufset), None)   # not held beside the other join's buffers
+            self._drop_class()
         if plan["strategy"] == "fused":
             plan["class_plan"] = self._class_plan(inst, plan)
         return plan
+
+    def _drop_class(self):
+        """Give the set's class workspace up: it is not held beside the other join's buffers."""
+        self._bufs.pop(("class", self._bufset), None)
+        self._reserved.get(self._bufset, {}).pop("class", None)
+        self._class_cover = 0.0
 
     def solve_instance(self, inst: Instance, verify: bool = True, timed: bool = False,
                        marks: list | None = None, i_limit: int | None = None, i_lo: int = 0) -> SolveResult:
@@ -777,6 +791,68 @@ class Solver:
         ev.record(st)
         h.update(ev=ev, hread=hm, hrows=rows)
 
+    def _reserve(self, insts: list, i_limit: int | None, i_lo: int, class_plans: list | None, use) -> dict:
+        """The buffers of a list's fused solves, in both sets, at the sizes of its largest instances: grown
+        solve by solve, a list of uneven pools met the device allocator (a millisecond of each of the first
+        solves) between its kernels.  A class workspace is known by its plan only: unless one was reserved for
+        longer survivor lists before, the instance whose lists should be the longest is planned here, and
+        an eighth is added for the others' moduli.  Returns the plans made, by position."""
+        tu, lib, plans = self.tuning, self.lib, {}
+        if tu.strategy != "fused":
+            return plans
+        mb = mi = mr = small = 0
+        by_class = []
+        pairs = tu.pair_capacity
+        for (nb, ni, r), i in {(len(x.B0), len(x.INS), x.r): i for i, x in enumerate(insts)}.items():
+            nD, nI = ncomb(nb, r), ncomb(ni, r)
+            nI = max(0, (nI if i_limit is None else min(nI, i_limit)) - i_lo)
+            n, m = (nD, nI) if nD < nI else (nI, nD)
+            if r == 0 or n == 0 or n >= 1 << 32:
+                continue
+            mb, mi, mr = max(mb, nb), max(mi, ni), max(mr, r)
+            if not tu.class_join or m < tu.class_min_probe:
+                small = max(small, n)
+                continue
+            if nD * nI >> insts[i].M.bit_length() >= tu.pair_capacity >> 4:
+                pairs = max(pairs, class_pairs(nD, nI, insts[i].M, tu))
+            load = min(n / 140, 1e5) / 49152            # filter load, and passes of the filter, see cf_class_plan
+            by_class.append((m * (load + load * load), i))
+        if not mr:
+            return plans
+        mb, mi = max(mb, mr), max(mi, mr)
+        need = dict(ctr=64, pairs=pairs * 16, res=pairs * self.result_bytes, tables=lib.cf_solve_table_bytes(mb, mi, mr))
+        if small:
+            need["dtab"] = lib.cf_dtab_bytes2(*dtab_shape(small, tu))
+            need["tails"] = lib.cf_solve_tail_bytes(mb, mi, mr)
+        if class_plans:
+            need["class"] = max(map(_ws_bytes, class_plans))
+        elif by_class:
+            for est, i in sorted(by_class, reverse=True)[:3]:
+                if est <= self._class_cover:
+                    break
+                plans[i] = self._direct_plan(insts[i], i_limit, i_lo)
+                cp = plans[i].get("class_plan")
+                if cp:
+                    need["class"] = _ws_bytes(cp) * 9 // 8
+                    self._class_cover = est
+                    break
+        rows = 8 + max(0, min(self._rows, tu.pair_capacity)) * self.result_bytes
+        for k in range(min(2, len(insts))):
+            have = self._reserved.setdefault(k, {})
+            if rows <= have.get("rows", 0) and all([v <= have.get(name, 0) for name, v in need.items()]):
+                continue
+            with use(k):
+                try:
+                    for name, v in need.items():        # the workspace last: the rest is small
+                        have[name] = self._buf(name, v).numel()
+                except self.torch.OutOfMemoryError:
+                    pass                                # the solves that do not fit find out one by one
+                else:
+                    self._pinned_buf("stage", need["tables"])
+                    self._pinned_buf("readback", rows)
+                    have["rows"] = rows
+        return plans
+
     def solve_many(self, insts: list, verify: bool = True, marks_list: list | None = None,
                    i_limit: int | None = None, readback_rows: int = 256, streams: int = 2,
                    i_lo: int = 0, class_plans: list | None = None) -> list[SolveResult]:
@@ -810,12 +886,7 @@ class Solver:
         self._rows = int(readback_rows)
         self._pool = base
         try:
-            for k in range(min(2, len(insts)) if class_plans else 0):
-                with use(k):                       # the workspace of a set at once, not grown plan by plan
-                    try:
-                        self._buf("class", max(_ws_bytes(cp) for cp in class_plans[k::2]))
-                    except torch.OutOfMemoryError:
-                        pass                       # the plans that do not fit take the table join one by one
+            plans = self._reserve(insts, i_limit, i_lo, class_plans, use)
             for i in range(len(insts) + 1):
                 cur = None
                 if i < len(insts):
@@ -825,7 +896,8 @@ class Solver:
                         marks = []
                         marks_list.append(marks)
                     with use(i):                   # the set (and stream) the solve in flight does not use
-                        plan = self._direct_plan(inst, i_limit, i_lo, class_plans[i] if class_plans else None)
+                        plan = plans.get(i) or self._direct_plan(inst, i_limit, i_lo,
+                                                                 class_plans[i] if class_plans else None)
                         if plan is None:
                             out[i] = self.solve_instance(inst, verify=verify, marks=marks, i_limit=i_limit,
                                                          i_lo=i_lo)
