@@ -73,6 +73,15 @@ def prunes(inst) -> bool:
     return Icap <= math.prod(inst.INS[-r:]) or Dmin > math.prod(inst.B0[:r])
 
 
+def bounded_pools(inst, Icap: int, Dmin: int) -> tuple[int, list[int]]:
+    """Base primes below the first that a subset with product >= Dmin can hold (their number), and the
+    insertion primes that a subset with product < Icap can hold; r primes of each side at least stay."""
+    r = inst.r
+    small, large = math.prod(inst.INS[:r - 1]), math.prod(inst.B0[-(r - 1):])
+    INS = [q for x, q in enumerate(inst.INS) if x < r or q * small < Icap]
+    return next((x for x in range(len(inst.B0) - r) if inst.B0[x] * large >= Dmin), len(inst.B0) - r), INS
+
+
 class BoundedSolve:
     """Solves one instance with the bounded producers and a record-table join.
 
@@ -172,9 +181,7 @@ class BoundedSolve:
         r, M = inst.r, inst.M
         if Icap <= 1 or Dmin >= U128:
             return None
-        small, large = math.prod(inst.INS[:r - 1]), math.prod(inst.B0[-(r - 1):])
-        INS = [q for x, q in enumerate(inst.INS) if x < r or q * small < Icap]
-        skip = next((x for x in range(len(inst.B0) - r) if inst.B0[x] * large >= Dmin), len(inst.B0) - r)
+        skip, INS = bounded_pools(inst, Icap, Dmin)
         B0 = inst.B0[skip:]
         total = math.comb(len(B0), r) + math.comb(len(INS), r)
         if total < self.CLASS_MIN or math.comb(max(len(B0), len(INS)), r - 3) >> 32:

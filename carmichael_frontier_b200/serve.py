@@ -84,19 +84,18 @@ def _dtab_bytes(n: int, tu: Tuning) -> int:
     return (164 << bb) + ((32 << fb) if fb else 0)
 
 
-def _class_bytes(inst: Instance, tu: Tuning) -> int:
-    """Device bytes of the instance's class join (its whole sides), 0 where it does not apply."""
-    import numpy as np
+def _class_bytes(M: int, B0, INS, r: int, tu: Tuning) -> tuple[int, int]:
+    """Device bytes of a class join of whole sides: its workspace (0 where it is not taken), which is given
+    up before another join starts, and its pair and result buffers, which are not."""
     from . import _lib
-    from .tables import split_modulus
-    nD, nI = math.comb(len(inst.B0), inst.r), math.comb(len(inst.INS), inst.r)
-    if not tu.class_join or not nD or not nI or max(nD, nI) < tu.class_min_probe:
-        return 0
-    lib = _lib.load()
-    out = np.zeros(lib.cf_class_plan_bytes(), dtype=np.uint8)
-    _lib.check(lib.cf_class_plan(split_modulus(inst.M)[0], len(inst.B0), len(inst.INS), inst.r, 0, min(nI, 2 ** 64 - 1),
-                                 int(nI < nD), out.ctypes.data, out.nbytes), "cf_class_plan")
-    return int(out[24:32].view(np.uint64)[0]) if out[8:12].view(np.uint32)[0] else 0
+    from .solve import RESULT_DTYPE, class_pairs, make_class_plan
+    nD, nI = math.comb(len(B0), r), math.comb(len(INS), r)
+    if not tu.class_join or not nD or not nI or max(nD, nI) < tu.class_min_probe or (B0[-1] | INS[-1]) >> 31:
+        return 0, 0
+    cp, ws = make_class_plan(_lib.load(), M, len(B0), len(INS), r, 0, min(nI, 2 ** 64 - 1), nI < nD)
+    if cp is None or ws > tu.class_ws_bytes:
+        return 0, 0
+    return ws, class_pairs(nD, nI, M, tu) * (16 + RESULT_DTYPE.itemsize)
 
 
 def footprint(inst: Instance, tu: Tuning) -> dict:
@@ -119,11 +118,16 @@ def footprint(inst: Instance, tu: Tuning) -> dict:
         # most min(nI, nD) of them) or on the D records (I leaves probed, never written)
         m = min(nI, nD)
         side = max(16 * m + _dtab_bytes(m, tu), _dtab_bytes(nD, tu))
-        need = max(16 * nD + frontier * 2 + side, _class_bytes(inst, tu))
-        return dict(bytes=fixed + need, strategy="bounded", nD=nD, nI=nI, work=nD + nI)
+        ws = rows = 0
+        if tu.class_join and 3 <= r <= 8 and Icap > 1:
+            skip, INS = bsolve.bounded_pools(inst, Icap, Dmin)
+            ws, rows = _class_bytes(inst.M, inst.B0[skip:], INS, r, tu)
+        return dict(bytes=fixed + rows + max(16 * nD + frontier * 2 + side, ws), strategy="bounded", nD=nD, nI=nI,
+                    work=nD + nI)
     small = min(math.comb(nB, r), math.comb(nI_full, r))
     tails = 16 * (math.comb(nB, 2) + math.comb(nI_full, 2))
-    return dict(bytes=fixed + max(_dtab_bytes(small, tu) + tails, _class_bytes(inst, tu)), strategy="fused",
+    ws, rows = _class_bytes(inst.M, inst.B0, inst.INS, r, tu)
+    return dict(bytes=fixed + rows + max(_dtab_bytes(small, tu) + tails, ws), strategy="fused",
                 work=math.comb(nB, r) + math.comb(nI_full, r))
 
 

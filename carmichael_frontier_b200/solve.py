@@ -162,6 +162,15 @@ def _ws_bytes(cp: bytes) -> int:
     return _PLAN_HEAD.unpack_from(cp)[4]
 
 
+def make_class_plan(lib, M: int, nB: int, nINS: int, r: int, i_lo: int, n_I: int, swap: bool) -> tuple[bytes | None, int]:
+    """cf_class_plan: (plan, workspace bytes), or (None, 0) where the class join does not apply."""
+    cp = C.create_string_buffer(lib.cf_class_plan_bytes())
+    _lib.check(lib.cf_class_plan(split_modulus(M)[0], nB, nINS, r, i_lo, n_I, int(swap), C.addressof(cp), len(cp)),
+               "cf_class_plan")
+    ok, _d, _mp, _phi, ws = plan_head(cp)
+    return (cp.raw, ws) if ok else (None, 0)
+
+
 def _pow2ceil(x: int) -> int:
     return 1 if x <= 1 else 1 << (x - 1).bit_length()
 
@@ -519,13 +528,11 @@ class Solver:
             return None                       # (no L2 for tables: the caller wants the table join's filter level)
         if (inst.B0[-1] | inst.INS[-1]) >> 31:
             return None                       # the class join's kernels multiply 32-bit factors
-        cp = C.create_string_buffer(lib.cf_class_plan_bytes())
-        _lib.check(lib.cf_class_plan(split_modulus(inst.M)[0], len(inst.B0), len(inst.INS), inst.r, _i_lo(plan), nI,
-                                     int(bool(plan.get("swap"))), C.addressof(cp), len(cp)), "cf_class_plan")
-        ok, _d, _mp, _phi, ws = plan_head(cp)
+        cp, ws = make_class_plan(lib, inst.M, len(inst.B0), len(inst.INS), inst.r, _i_lo(plan), nI,
+                                 bool(plan.get("swap")))
         # k = 64: r = 5 54 to 210 MB, r = 6 0.8 to 13 GB, r = 7 1.3 to 40 GB (the table join 0.2, 1.3 and 10)
         sets = plan.get("sets") or (1 if self._pool is None else 2)
-        return cp.raw if ok and ws * sets <= tu.class_ws_bytes else None
+        return cp if ws * sets <= tu.class_ws_bytes else None
 
     def _part_build(self, inst: Instance, plan: dict, pshape: tuple, tables: tuple, tab, nD: int, nIt: int,
                     swap: bool, misc):
