@@ -325,10 +325,10 @@ class Solver:
             self._bufs[key] = t
         return t
 
-    def _pinned_buf(self, name: str, nbytes: int, dev=None):
+    def _pinned_buf(self, name: str, nbytes: int, dev=None, sh: int = 0):
         """Page-locked host buffer of the current buffer set (rewritten only after the solve that
         last used it has been collected, see _leave_staging).
-        dev: the device buffer that a native call copies to or from it.  Torch, which hands freed
+        dev: the device buffer that a native call on stream sh copies to or from it.  Torch, which hands freed
         page-locked memory out again, does not see such a copy, so one byte goes up through torch once per
         buffer and stream: the memory, once freed, then waits for that stream."""
         key = (name, self._bufset)
@@ -336,12 +336,10 @@ class Solver:
         if t is None or t.numel() < nbytes:
             t, streams = self.torch.empty(max(nbytes, 64), dtype=self.torch.uint8, pin_memory=True), set()
             self._pinned[key] = t, streams
-        if dev is not None:
-            sh = self._sh()
-            if sh not in streams:
-                with self.torch.cuda.stream(self._torch_stream()):
-                    dev[:1].copy_(t[:1], non_blocking=True)
-                streams.add(sh)
+        if dev is not None and sh not in streams:
+            with self.torch.cuda.stream(self._torch_stream()):
+                dev[:1].copy_(t[:1], non_blocking=True)
+            streams.add(sh)
         return t
 
     def _leave_staging(self):
@@ -442,8 +440,9 @@ class Solver:
         # L2-resident while built); larger tables the wide entries
         q.side_format = 1 if q.bbits <= 20 else 0
         tb = lib.cf_solve_table_bytes(len(pD), len(pI), r)
+        sh = self._sh()
         tabs = self._buf("tables", tb)
-        stage = self._pinned_buf("stage", tb, tabs)
+        stage = self._pinned_buf("stage", tb, tabs, sh)
         if cp:
             _ok, d, mp, _phi, q.ws_bytes = plan_head(cp)
             q.class_plan = C.cast(C.c_char_p(cp), C.c_void_p)
@@ -461,7 +460,7 @@ class Solver:
         rb = self.result_bytes
         rows = max(0, min(self._rows, maxp))
         pairs, res, ctr = self._buf("pairs", maxp * 16), self._buf("res", maxp * rb), self._buf("ctr", 64)
-        hm = self._pinned_buf("readback", 8 + rows * rb, ctr)
+        hm = self._pinned_buf("readback", 8 + rows * rb, ctr, sh)
         q.stage, q.tables, q.ws, q.pairs, q.results, q.misc = \
             stage.data_ptr(), dp(tabs), dp(ws), dp(pairs), dp(res), dp(ctr)
         q.max_pairs, q.rows, q.readback = maxp, rows, hm.data_ptr()
@@ -469,7 +468,7 @@ class Solver:
             for j, tag in enumerate(("start", "gen_D", "probe", "check")):
                 self._mark(marks, tag)             # makes the event; cf_solve records it again in its place
                 q.events[j] = marks[-1][1].cuda_event
-        _lib.check(lib.cf_solve(C.byref(q), self._sh()), "cf_solve")
+        _lib.check(lib.cf_solve(C.byref(q), sh), "cf_solve")
         ev = self.torch.cuda.Event()
         ev.record(self._torch_stream())
         return dict(misc=ctr[:64].view(self.torch.int32), dcnt=None, icnt=None, res=res, nD=nD, nI=nIt, plan=plan,
