@@ -191,7 +191,7 @@ class BoundedSolve:
         plan = s.plan(nD, nI)
         if min(nD, nI) >= RANK_LIMIT or max(nD, nI) < s.tuning.class_min_probe:
             return None
-        plan.update(strategy="fused", i_limit=None, i_lo=0)
+        plan.update(strategy="fused", i_limit=None, i_lo=0, class_least=0)    # against the level loop, at any radius
         cp = s._class_plan(sub, plan)
         if cp is None:
             return None

@@ -37,10 +37,13 @@ import numpy as np
 from . import _lib
 from .certify import verify_certificate
 from .solve import (MOD_DTYPE, RESULT_DTYPE, Hit, Instance, SolveResult, Solver, Tuning, dtab_shape, finish_rows,
-                    _ws_bytes, part_shape)
+                    _ws_bytes, class_least, part_shape)
 from .tables import ncomb, pool_table_host, screen_table_host
 
 _ALIGN = 256
+# Moduli of radius 3 and 4 below class_least that are worth a batch of their own.  I ranks [0, 2^22), r = 4, class
+# join against batch, ms: 4 moduli .90 / 1.12, 16 moduli 3.7 / 2.3; r = 3: .90 / 1.07 and 2.8 / 2.2.
+EITHER_BATCH = 8
 
 
 def _up(x: int, a: int = _ALIGN) -> int:
@@ -194,7 +197,8 @@ class BatchSolver:
         tu = self.tuning.dtab
         if not self.tuning.class_join or not tu.class_join or max(nD, nI) < tu.class_min_probe or tu.strategy != "fused":
             return None
-        cp = self._solver()._class_plan(x, dict(i_limit=i_limit, i_lo=0, swap=nI < nD, sets=2))
+        cp = self._solver()._class_plan(x, dict(i_limit=i_limit, i_lo=0, swap=nI < nD, sets=2,
+                                               class_least=tu.class_min_probe))
         return cp if cp and 2 * _ws_bytes(cp) <= self.tuning.mem_budget else None
 
     def prepare(self, instances: list, i_limit: int | None = None) -> PreparedPortfolio:
@@ -212,10 +216,16 @@ class BatchSolver:
         fallback: list = []
         batched: list = []
         single: dict = {}
+        # small probing sides at radius 3 and 4: a batch takes them faster where there is one
+        m = [max(nD[k], nI[k]) if x.r and nD[k] and nI[k] else 0 for k, x in enumerate(insts)]
+        least = tu.dtab.class_min_probe
+        either = {k for k, x in enumerate(insts) if least <= m[k] < class_least(x.r, min(nD[k], nI[k]), tu.dtab)}
+        if len(either) < EITHER_BATCH and not any(0 < v < least for v in m):
+            either = set()
         for k, x in enumerate(insts):
-            if x.r == 0 or nD[k] == 0 or nI[k] == 0:
+            if m[k] == 0:
                 trivial[k] = None
-            elif (cp := self._class_plan(x, nD[k], nI[k], i_limit)) is not None:
+            elif k not in either and (cp := self._class_plan(x, nD[k], nI[k], i_limit)) is not None:
                 single[k] = cp
             elif x.r > self.max_r or min(nD[k], nI[k]) >= 1 << 32:
                 fallback.append(k)

@@ -84,13 +84,13 @@ def _dtab_bytes(n: int, tu: Tuning) -> int:
     return (164 << bb) + ((32 << fb) if fb else 0)
 
 
-def _class_bytes(M: int, B0, INS, r: int, tu: Tuning) -> tuple[int, int]:
+def _class_bytes(M: int, B0, INS, r: int, tu: Tuning, least: int) -> tuple[int, int]:
     """Device bytes of a class join of whole sides: its workspace (0 where it is not taken), which is given
     up before another join starts, and its pair and result buffers, which are not."""
     from . import _lib
     from .solve import RESULT_DTYPE, class_pairs, make_class_plan
     nD, nI = math.comb(len(B0), r), math.comb(len(INS), r)
-    if not tu.class_join or not nD or not nI or max(nD, nI) < tu.class_min_probe or (B0[-1] | INS[-1]) >> 31:
+    if not tu.class_join or not nD or not nI or max(nD, nI) < least or (B0[-1] | INS[-1]) >> 31:
         return 0, 0
     cp, ws = make_class_plan(_lib.load(), M, len(B0), len(INS), r, 0, min(nI, 2 ** 64 - 1), nI < nD)
     if cp is None or ws > tu.class_ws_bytes:
@@ -102,6 +102,7 @@ def footprint(inst: Instance, tu: Tuning) -> dict:
     """Upper bound on the device bytes one solve of `inst` holds at once, and the
     strategy it will use ('bounded' or 'fused')."""
     from . import bsolve
+    from .solve import class_least
     max_nodes = tu.max_nodes
     r = inst.r
     nB, nI_full = len(inst.B0), len(inst.INS)
@@ -121,12 +122,12 @@ def footprint(inst: Instance, tu: Tuning) -> dict:
         ws = rows = 0
         if tu.class_join and 3 <= r <= 8 and Icap > 1:
             skip, INS = bsolve.bounded_pools(inst, Icap, Dmin)
-            ws, rows = _class_bytes(inst.M, inst.B0[skip:], INS, r, tu)
+            ws, rows = _class_bytes(inst.M, inst.B0[skip:], INS, r, tu, tu.class_min_probe)
         return dict(bytes=fixed + rows + max(16 * nD + frontier * 2 + side, ws), strategy="bounded", nD=nD, nI=nI,
                     work=nD + nI)
     small = min(math.comb(nB, r), math.comb(nI_full, r))
     tails = 16 * (math.comb(nB, 2) + math.comb(nI_full, 2))
-    ws, rows = _class_bytes(inst.M, inst.B0, inst.INS, r, tu)
+    ws, rows = _class_bytes(inst.M, inst.B0, inst.INS, r, tu, class_least(r, small, tu))
     return dict(bytes=fixed + rows + max(_dtab_bytes(small, tu) + tails, ws), strategy="fused",
                 work=math.comb(nB, r) + math.comb(nI_full, r))
 

@@ -115,8 +115,18 @@ class Tuning:
     part_sigma: float = 8.0         # bucket-range capacity = mean + sigma*sqrt(mean) + 32
     class_join: bool = True         # fused: join by residue classes (csrc/cf_class.cu) where it applies
     class_ws_bytes: int = 24 << 30  # ... and its workspace is at most this, half of it for each of a list's two
-    class_min_probe: int = 1 << 22  # ... and the probing side has this many records or more (below, the
-                                    # plan's 40 us of host time weigh more than the device time it saves)
+    class_min_probe: int = 1 << 22  # ... and the probing side has this many records or more (see class_least)
+
+
+def class_least(r: int, n_build: int, tu: Tuning) -> int:
+    """Least probing side of a class join at radius r, n_build records on the other side.  Its lists and plan cost 0.13 ms whatever the sides; a
+    table probe costs more per record at larger radii.  Whole solves, class join against table join, ms:
+    r = 3, 6.5e6 records .227 / .203, 1.2e7 .228 / .236, 2.9e7 .266 / .337; r = 4, 4.2e6 .212 / .198, 8.2e6
+    .220 / .213, 1.5e7 .243 / .278; r = 5, 4.2e6 .190 / .189 (nD = 1.4e5) and .247 / .289 (7.6e6), 2.4e7
+    .290 / .451; r = 6, 4.5e6 .197 / .219; r = 7, 5.4e6 .189 / .288; r = 8, 5.9e6 .226 / .364.  A table of few
+    records is probed at the same few sectors: r = 3, 4.5e6 against 1,140 records .194 / .245, against 10,000
+    .222 / .210; r = 4, 4.6e6 against 495 .183 / .266, against 27,405 .198 / .171."""
+    return tu.class_min_probe * (3 if r < 5 and n_build >= 4096 else 1)
 
 
 def dtab_shape(nD: int, tu: Tuning) -> tuple[int, int]:
@@ -517,13 +527,12 @@ class Solver:
 
     def _class_plan(self, inst: Instance, plan: dict) -> bytes | None:
         """The class join's plan for a fused solve (see cf_class_plan), or None where the table join
-        is taken: a small probing side, a modulus without fitting divisors, a run after an overflow.
-        Whole solve, class join against table join, k = 64: r = 5, 5.9e8 I records 0.86 against
-        3.42 ms; r = 5, 1.9e7 0.21 against 0.36; r = 6, 4.7e8 2.2 against 15.7; r = 7, 1.2e10 63
-        against 323; r = 4, 1.4e7 0.15 against 0.23."""
+        is taken: a small probing side (class_least, or plan["class_least"]), a modulus without fitting
+        divisors, a workspace above the limit, a run after an overflow."""
         tu, lib = self.tuning, self.lib
         nD, nI = ncomb(len(inst.B0), inst.r), _i_window(inst, plan)
-        if not tu.class_join or plan.get("no_class") or max(nD, nI) < tu.class_min_probe or not tu.l2_table_bytes:
+        least = plan.get("class_least", class_least(inst.r, min(nD, nI), tu))
+        if not tu.class_join or plan.get("no_class") or max(nD, nI) < least or not tu.l2_table_bytes:
             return None                       # (no L2 for tables: the caller wants the table join's filter level)
         if (inst.B0[-1] | inst.INS[-1]) >> 31:
             return None                       # the class join's kernels multiply 32-bit factors
@@ -816,7 +825,7 @@ class Solver:
             if r == 0 or n == 0 or n >= 1 << 32:
                 continue
             mb, mi, mr = max(mb, nb), max(mi, ni), max(mr, r)
-            if not tu.class_join or m < tu.class_min_probe:
+            if not tu.class_join or m < class_least(r, n, tu):
                 small = max(small, n)
                 continue
             if nD * nI >> insts[i].M.bit_length() >= tu.pair_capacity >> 4:

@@ -2,6 +2,7 @@
 import math
 import os
 
+import numpy as np
 import pytest
 
 from carmichael_frontier_b200 import Instance, Solver, Tuning, _lib
@@ -27,7 +28,7 @@ def class_plan(x, **tuning):
 @pytest.mark.parametrize("side", ["B0", "INS"])
 def test_primes_of_2_31_or_more_do_not_take_the_class_join(side):
     # its kernels multiply 32-bit factors; Instance.build refuses such primes, the class itself does not
-    x = instance(64, 120, 4)
+    x = instance(64, 150, 4)
     assert class_plan(x) is not None
     getattr(x, side)[-1] = (1 << 31) + 11
     x.P0 = math.prod(x.B0)
@@ -79,3 +80,31 @@ def test_a_plan_without_host_memory_returns_a_status():
     p = subprocess.run([sys.executable, "-c", EXHAUSTED % (M // (M & -M), math.comb(120, 4))], capture_output=True,
                        text=True, cwd=ROOT, timeout=120)
     assert p.returncode == 0 and p.stdout in (f"status {_lib.CF_OK}", f"status {_lib.CF_ENOMEM}"), (p.returncode, p.stderr[-500:])
+
+
+def test_small_probing_sides_keep_the_table_join_at_small_radii():
+    for k, n, r, taken in ((64, 102, 4, False), (64, 120, 4, False), (64, 140, 4, True), (64, 200, 3, False),
+                           (100, 440, 3, True), (104, 12, 4, True), (104, 30, 4, False), (64, 58, 5, True), (30, 58, 5, True)):
+        assert max(math.comb(k, r), math.comb(n, r)) >= 1 << 20
+        assert (class_plan(instance(k, n, r)) is not None) == taken, (k, n, r)
+
+
+def test_portfolio_batches_small_probing_sides_where_there_is_a_batch(monkeypatch):
+    # nothing is launched here: the split is made before the tables go up
+    class Split(Exception):
+        pass
+
+    def stop(*a):
+        raise Split(a[0])
+
+    import carmichael_frontier_b200.portfolio as P
+    for counts, batched in (((5, 0, 2), 0), ((8, 0, 2), 8), ((1, 1, 1), 2), ((1, 0, 0), 0)):
+        xs = [instance(64, 110, 4)] * counts[0] + [instance(20, 30, 3)] * counts[1] + [instance(64, 60, 5)] * counts[2]
+        seen = []
+        monkeypatch.setattr(P, "pool_table_host", lambda *a: seen.append(a) or np.zeros(8, dtype=np.uint8))
+        monkeypatch.setattr(P, "screen_table_host", lambda *a: np.zeros(8, dtype=np.uint8))
+        b = BatchSolver("cuda")
+        monkeypatch.setattr(b, "torch", type("T", (), {"from_numpy": staticmethod(stop)}))
+        with pytest.raises(Split):
+            b.prepare(xs)
+        assert len(seen) == 2 * batched
