@@ -20,6 +20,7 @@ subsets that no hit can contain.  Where the bound prunes hard (B = prod(B0) *
 from __future__ import annotations
 
 import math
+from bisect import bisect_left, bisect_right
 
 import numpy as np
 
@@ -78,8 +79,33 @@ def bounded_pools(inst, Icap: int, Dmin: int) -> tuple[int, list[int]]:
     insertion primes that a subset with product < Icap can hold; r primes of each side at least stay."""
     r = inst.r
     small, large = math.prod(inst.INS[:r - 1]), math.prod(inst.B0[-(r - 1):])
-    INS = [q for x, q in enumerate(inst.INS) if x < r or q * small < Icap]
-    return next((x for x in range(len(inst.B0) - r) if inst.B0[x] * large >= Dmin), len(inst.B0) - r), INS
+    n = bisect_right(inst.INS, (Icap - 1) // small)                     # q * small < Icap
+    skip = bisect_left(inst.B0, -(-Dmin // large))                      # p * large >= Dmin
+    return min(skip, len(inst.B0) - r), inst.INS[:max(n, r)]
+
+
+def bounded_share(B0, INS, r: int, Icap: int, Dmin: int) -> float:
+    """Estimated share of the r-subsets of both sides that the bounds keep.  First from the place of the bound's
+    r-th root in each pool, the logarithms taken as even (3 us; 1,700 bounds over 12 moduli: below 0.05 the share
+    was below 1/8, from 0.4 on above it); between, from the mean and variance of the logarithms (40 us,
+    within 0.04), a sum of r of them taken as normal."""
+    nD, nI = math.comb(len(B0), r), math.comb(len(INS), r)
+
+    def by_place(primes, bound: int) -> float:
+        q = bisect_left(primes, math.exp(math.log(max(bound, 1)) / r)) / len(primes)
+        return 0.5 + 0.5 * math.erf((q - 0.5) * math.sqrt(6 * r))
+
+    def by_moments(primes, bound: int) -> float:
+        lg, n = np.log(np.asarray(primes, dtype=np.float64)), len(primes)
+        var = float(lg.var()) * r * (n - r) / max(n - 1, 1)
+        z = math.log(max(bound, 1)) - r * float(lg.mean())
+        return 0.5 + 0.5 * math.erf(z / math.sqrt(2 * var)) if var > 0 else float(z > 0)
+
+    for below in (by_place, by_moments):
+        share = ((1 - below(B0, Dmin)) * nD + below(INS, Icap) * nI) / (nD + nI)
+        if not 0.05 <= share < 0.4:
+            break
+    return share
 
 
 class BoundedSolve:
@@ -158,8 +184,7 @@ class BoundedSolve:
         Icap, Dmin = caps(inst)
         got = None
         if self.s.tuning.class_join and 3 <= inst.r <= 8:
-            with self.torch.cuda.stream(self.s._torch_stream()):
-                got = self._join_class(inst, Icap, Dmin)
+            got = self._join_class(inst, Icap, Dmin)
         pairs, nD, nI, plan = got or self._join(inst, Icap, Dmin, None, None)
         return self._finish(inst, pairs, nD, nI, plan, verify)
 
@@ -176,15 +201,20 @@ class BoundedSolve:
 
         k = 76, r = 6, 1.4e8 D records, 4.3e9 I leaves: 124 ms as a level loop with leaf probes, 16.5 ms on
         the device here (1.4 of it the counts); k = 78, r = 4, 1.4e6 and 2.6e7: 0.89 against 0.64 ms in all."""
-        from .solve import RESULT_DTYPE, Instance, class_pairs, plan_head
-        lib, dp, s = self.lib, _lib.ptr, self.s
-        r, M = inst.r, inst.M
+        from .solve import Instance
+        s, r, M = self.s, inst.r, inst.M
         if Icap <= 1 or Dmin >= U128:
+            return None
+        if math.comb(len(inst.B0), r) + math.comb(len(inst.INS), r) < self.CLASS_MIN:
             return None
         skip, INS = bounded_pools(inst, Icap, Dmin)
         B0 = inst.B0[skip:]
         total = math.comb(len(B0), r) + math.comb(len(INS), r)
         if total < self.CLASS_MIN or math.comb(max(len(B0), len(INS)), r - 3) >> 32:
+            return None
+        # Without this guess, hard bounds paid for the plan, the tables and a wait for the exact counts, and then
+        # for the level loop: k = 64, r = 5, 100 insertion primes, B = 10 P0: 0.80 ms, the level loop 0.52.
+        if bounded_share(B0, INS, r, Icap, Dmin) * self.CLASS_RATIO < 1:
             return None
         sub = Instance(M, list(B0), INS, r, inst.B, inst.P0)
         nD, nI = math.comb(len(B0), r), math.comb(len(INS), r)
@@ -195,6 +225,15 @@ class BoundedSolve:
         cp = s._class_plan(sub, plan)
         if cp is None:
             return None
+        with self.torch.cuda.stream(s._torch_stream()):
+            return self._run_class(inst, Icap, Dmin, skip, B0, INS, cp)
+
+    def _run_class(self, inst, Icap, Dmin, skip: int, B0, INS, cp: bytes):
+        """The class join of the pools B0 and INS (see _join_class) on the solver's stream."""
+        from .solve import RESULT_DTYPE, class_pairs, plan_head
+        lib, dp, s = self.lib, _lib.ptr, self.s
+        r, M = inst.r, inst.M
+        nD, nI = math.comb(len(B0), r), math.comb(len(INS), r)
         multD = pow(inst.P0, -1, M)
         # screen bound 1: no pair passes, the check only turns ranks into indices
         dev = self._upload([pool_table_host(B0, r, M, multD), pool_table_host(INS, r, M, 1),
@@ -207,7 +246,7 @@ class BoundedSolve:
         _lib.check(lib.cf_bounded_count(1, poolD, G, len(B0), r, base + 16, sh), "cf_bounded_count(D)")
         _lib.check(lib.cf_bounded_count(0, poolI, H, len(INS), r, base + 24, sh), "cf_bounded_count(I)")
         bD, bI = misc[16:32].cpu().numpy().view(np.uint64).tolist()
-        if (bD + bI) * self.CLASS_RATIO < total:
+        if (bD + bI) * self.CLASS_RATIO < nD + nI:
             return None
         out = dict(strategy="bounded", Icap=Icap, Dmin=Dmin, table="class", class_plan=cp)
         if bD == 0 or bI == 0:
