@@ -177,40 +177,52 @@ struct PassLayout {
 
 // Control words of the segment sort (below) and its scaled key.
 constexpr int kSegLog = 64 * 32;   // pieces of the logarithmic map: 32 per power of two
-struct SegCtl {            // zeroed before the sort, except where noted
-  u64 scale, max_key;
-  u32 top;                 // 2^L NS - 1
-  u32 linear;              // 1: f = mulhi(key, scale); 0: f from the piecewise map
-  u32 blocks_done, max_seg, err, pad, tickets[2];
+struct SegCtl {
+  u32 cdf[kSegLog + 2];    // f at the start of each piece; the rest is zeroed before the sort:
+  u32 full[kSegLog];       // all keys per piece
   u32 hist[kSegLog];       // sampled keys per piece
-  u32 cdf[kSegLog + 1];    // (not zeroed) f at the start of each piece
+  u64 scale, max_key;      // from here on also for the sides of k_seg_front
+  u64 cap;                 // largest key of kMapNarrow
+  u32 top;                 // 2^L NS - 1
+  u32 mode;                // f(key), see SegScale
+  u32 met;                 // sampled keys that met their equal from another run
+  u32 max_seg, err, bail;  // bail: the LSD sort takes these keys, nothing is moved
+  u32 blocks_done, pieces_done, tickets[2];
 };
-// Piece of a key and its place in the piece, 20 bits.
+// Piece of a key (0 counts as 1) and its place in the piece, 26 bits.
 __device__ __forceinline__ u32 seg_piece(u64 key, u32& frac) {
-  const int z = __clzll((long long)(key | 1ull));
-  const u32 h = (u32)(((key | 1ull) << z) >> 32);
-  frac = (h >> 6) & 0xfffffu;
+  const u64 k = key ? key : 1ull;
+  const int z = __clzll((long long)k);
+  const u32 h = (u32)((k << z) >> 32);
+  frac = h & 0x3ffffffu;
   return ((u32)(63 - z) << 5) | ((h >> 26) & 31u);
 }
+// f of a key, monotone, at most top.  (One linear form for narrow keys too, a minimum and a shift more, costs the
+// passes 2%: a mode of its own.)
+enum { kMapPieces = 0, kMapEven = 1, kMapNarrow = 2 };
 struct SegScale {
-  u64 s;
-  u32 top, linear;
+  u64 s, cap;
+  u32 top, mode;
   const u32* cdf;
+  __device__ __forceinline__ u32 even(u64 key) const {
+    const u64 f = __umul64hi(key, s);
+    return f < top ? (u32)f : top;
+  }
+  __device__ __forceinline__ u32 narrow(u64 key) const { return (u32)((key < cap ? key : cap) * s >> 32); }
   __device__ __forceinline__ u32 operator()(u64 key) const {
-    if (linear) {                                      // uniform over the launch
-      const u64 f = __umul64hi(key, s);
-      return f < top ? (u32)f : top;
-    }
+    if (mode == kMapEven) return even(key);            // uniform over the launch
+    if (mode == kMapNarrow) return narrow(key);
     u32 frac;
     const u32 i = seg_piece(key, frac), c0 = __ldg(cdf + i), c1 = __ldg(cdf + i + 1);
-    return min(c0 + (u32)(((u64)(c1 - c0) * frac) >> 20), top);
+    return (u32)min((u64)c0 + (((u64)(c1 - c0) * frac) >> 26), (u64)top);
   }
 };
 __device__ __forceinline__ SegScale seg_map(const SegCtl* c) {
   SegScale r;
   r.s = c->scale;
+  r.cap = c->cap;
   r.top = c->top;
-  r.linear = c->linear;
+  r.mode = c->mode;
   r.cdf = c->cdf;
   return r;
 }
@@ -255,7 +267,9 @@ k_sort_pass(const u64* __restrict__ kin, const u64* __restrict__ iin, u64* __res
   __shared__ u32 s_scan[kWarps];
 
   if (threadIdx.x == 0) {
-    s_tile = atomicAdd(ticket, 1u);
+    const u32 stop = MSD ? scale->bail : 0u;
+    const u32 mine = atomicAdd(ticket, 1u);
+    s_tile = stop ? ~0u : mine;
     if (BULK) {
       mbar_init(&s_bar[0], 1);
       mbar_init(&s_bar[1], 1);
@@ -264,7 +278,10 @@ k_sort_pass(const u64* __restrict__ kin, const u64* __restrict__ iin, u64* __res
   }
   __syncthreads();
   SegScale sc{};
-  if constexpr (MSD) sc = seg_map(scale);
+  if constexpr (MSD) {
+    if (s_tile == ~0u) return;                // uniform, before any copy is started
+    sc = seg_map(scale);
+  }
   const u32 tile = s_tile;
   const u64 base = (u64)tile * kSortTile;
   const u64 left = n - base;
@@ -480,10 +497,13 @@ k_sort_pass(const u64* __restrict__ kin, const u64* __restrict__ iin, u64* __res
 //
 // Residues are even over [0, M) once products wrap; the D side's are not (products of few small
 // primes stay below M).  The keys are sampled by pieces of their logarithm (32 per power of two),
-// and where the sample is not even f runs through each piece by the piece's share of it.
+// and where the sample is not even, all keys are counted by piece and f runs through each piece by the
+// piece's share of them.  Even keys below 2^L NS are spread by a factor instead of mulhi.
 //
 // A segment above kSegCap records (few distinct keys, clusters) leaves the records as
-// the passes left them, a stable reordering, and the caller runs the LSD sort on that.
+// the passes left them, a stable reordering, and the caller runs the LSD sort on that.  Where the
+// sample meets the same key often, the LSD sort, which skips digits that all keys share, is the faster
+// one: nothing is moved then (seg_dup_limit).
 // ---------------------------------------------------------------------------
 constexpr int kSegBlock = 512;
 constexpr int kSegItems = 8;
@@ -518,11 +538,21 @@ __device__ __forceinline__ u64 block_max(u64 m, u64* s_m) {
   return m;
 }
 
-// The map of the sampled keys counted in h (shared memory, kSegLog pieces), by one CTA of T threads:
-// linear when every piece holds what even keys below the maximum would (within six deviations and a
-// twentieth), else piecewise, f rising by a piece's share of the sample over the piece.
-template <int T>
-__device__ __forceinline__ void seg_make_map(const u32* h, u64 max_key, u32 segs, SegCtl* ctl, u32* s_w) {
+// Keys that a sample of 1 in `step` (at least 2^19 keys, runs of 32) may have missed above its largest:
+// sorted input hides up to 32 * step of them, 2^-14 of the records.
+__device__ __forceinline__ u64 seg_reach(u64 max_key, u32 step) {
+  const u64 more = step > 1 ? max_key >> 13 : 0;
+  return max_key + more < max_key ? ~0ull : max_key + more;
+}
+
+// The map of the keys counted in h (shared memory, kSegLog pieces), by one CTA of T threads: linear
+// when every piece holds what even keys below the maximum would (within six deviations and a
+// twentieth), else (or with `pieces`) piecewise, f rising by a piece's share of the keys over the piece --
+// over the part of it below `reach` in the last one, which even keys may fill up to there.
+// FRONT: the map also in h (kSegLog + 1 entries) and *sc, for the CTA itself.
+template <int T, bool FRONT>
+__device__ __forceinline__ void seg_make_map(u32* h, u64 max_key, u64 reach, u32 segs, bool pieces, SegCtl* ctl, u32* s_w,
+                                             SegScale* sc) {
   constexpr int P = kSegLog / T;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   u32 c[P], sum = 0;
@@ -543,33 +573,71 @@ __device__ __forceinline__ void seg_make_map(const u32* h, u64 max_key, u32 segs
   }
   const u64 range = (u64)segs << kSegBits;
   const float per = (float)total / ((float)max_key + 1.0f);
-  bool even = true;
+  bool even = !pieces;
+  u32 unused, over = 0;                                // over: end of the last piece's own range
+  const u32 last = seg_piece(reach, unused);
 #pragma unroll
   for (int q = 0; q < P; ++q) {
     const u32 i = threadIdx.x * P + q;
-    ctl->cdf[i] = (u32)((u64)run * range / (total ? total : 1u));
+    const u64 c0 = (u64)run * range / (total ? total : 1u);
     run += c[q];
+    if (i <= last) {
+      ctl->cdf[i] = (u32)c0;
+      if (FRONT) h[i] = (u32)c0;
+    }
     // keys [2^e (1 + j/32), 2^e (1 + (j+1)/32)) cut at the maximum
     const float lo = ldexpf(1.0f + (float)(i & 31u) / 32.0f, (int)(i >> 5)), w = ldexpf(1.0f / 32.0f, (int)(i >> 5));
+    if (i == last) {
+      const float have = fminf(w, (float)reach + 1.0f - lo);
+      const float end = (float)c0 + ((float)range - (float)c0) * (have > 0.0f ? fminf(w / have, 1024.0f) : 1.0f);
+      over = end < 4.2e9f ? max((u32)end, (u32)range) : 4200000000u;
+    }
     const float e = per * fminf(w, fmaxf(0.0f, (float)max_key + 1.0f - lo));
-    even = even && fabsf((float)c[q] - e) <= 0.05f * e + 6.0f * sqrtf(e) + 16.0f;
+    even = even && (i < 160u || fabsf((float)c[q] - e) <= 0.05f * e + 6.0f * sqrtf(e) + 16.0f);   // keys below 32: pieces below one key
   }
-  if (threadIdx.x == T - 1) ctl->cdf[kSegLog] = (u32)range;
   const int lin = __syncthreads_and(even);
+  if (over) s_w[0] = over;
+  __syncthreads();
+  over = s_w[0];                                       // the pieces above hold no key, or a few that were not sampled
+  for (u32 i = last + 1 + threadIdx.x; i <= (u32)kSegLog; i += T) {
+    ctl->cdf[i] = over;
+    if (FRONT) h[i] = over;
+  }
   if (threadIdx.x == 0) {
-    ctl->scale = seg_scale(max_key, segs);
-    ctl->top = (u32)(range - 1);
-    ctl->linear = (u32)lin;
+    SegScale r{};
+    r.mode = !lin ? kMapPieces : reach < range ? kMapNarrow : kMapEven;
+    r.s = r.mode == kMapNarrow ? (range << 32) / (reach + 1) : seg_scale(reach, segs);   // (reach + 1) s <= 2^32 range
+    r.cap = reach;
+    r.top = (u32)(range - 1);
+    ctl->scale = r.s;
+    ctl->cap = r.cap;
+    ctl->top = r.top;
+    ctl->mode = r.mode;
+    if (FRONT) *sc = r;
   }
 }
 
-// Sampled keys (one run of 32 of every 32 * step): their maximum and pieces; the last CTA makes the map.
+// Sampled keys (one run of 32 of every 32 * step): their maximum, their pieces, and how many met their
+// equal from another run in a table of the CTA's last keys; the last CTA makes the map.  (Equal
+// keys within a run are not counted: in ordered input every key that occurs twice is beside its equal.)
+constexpr u32 kSegSeen = 8192;                         // table entries: 24 bits of hash, 8 of the run
+// Records per key from which the LSD sort is taken: equal keys share a bin, where records are compared with one
+// another, and make segments uneven (deviation sqrt(3400 (g + 1)) for g records a key).  Segment sort / LSD
+// sort, us: 7.6e6 records, g = 4, 50-bit keys 447 / 791, narrow keys 424 / 455; g = 8 974 / 789 and 486 / 454; 2^26
+// narrow, g = 4 2946 / 3033, g = 8 3427 / 3008; 2^20 wide, g = 12 184 / 212, g = 16 233 / 214.  Below 2^19 records
+// finding out costs what the LSD sort gains (25 us: 3.0e5, g = 32 130 / 108).
+__device__ __forceinline__ float seg_dup_limit(u64 n) {
+  return n < (1ull << 19) ? 3.0e38f : n < (1ull << 22) ? 12.0f : 7.0f;
+}
 __global__ void __launch_bounds__(512) k_seg_sample(const u64* __restrict__ keys, u64 n, u32 step, u32 segs, SegCtl* ctl) {
   __shared__ u64 s_m[16];
-  __shared__ u32 s_h[kSegLog], s_w[16], s_last;
+  __shared__ u32 s_h[kSegLog], s_seen[kSegSeen], s_w[16], s_last, s_met;
   for (int i = threadIdx.x; i < kSegLog; i += 512) s_h[i] = 0;
+  for (u32 i = threadIdx.x; i < kSegSeen; i += 512) s_seen[i] = 0;
+  if (threadIdx.x == 0) s_met = 0;
   __syncthreads();
   u64 m = 0;
+  u32 met = 0;
   const u64 lanes = (u64)gridDim.x * 512;
   for (u64 t = (u64)blockIdx.x * 512 + threadIdx.x;; t += lanes) {
     const u64 i = (t >> 5) * 32 * step + (t & 31);
@@ -578,11 +646,19 @@ __global__ void __launch_bounds__(512) k_seg_sample(const u64* __restrict__ keys
     m = k > m ? k : m;
     u32 frac;
     atomicAdd(&s_h[seg_piece(k, frac)], 1u);
+    const u64 h = (k ^ (k >> 32)) * 0x9E3779B97F4A7C15ull;
+    const u32 tag = ((u32)(h >> 19) & 0xffffff00u) | (u32)((t >> 5) & 255u);
+    const u32 old = atomicExch(&s_seen[h >> 51], tag);
+    met += ((old ^ tag) >> 8) == 0u && ((old ^ tag) & 255u) != 0u;
   }
+  if (met) atomicAdd(&s_met, met);
   m = block_max<512>(m, s_m);
   for (int i = threadIdx.x; i < kSegLog; i += 512)
     if (s_h[i]) atomicAdd(&ctl->hist[i], s_h[i]);
-  if (threadIdx.x == 0) atomicMax((unsigned long long*)&ctl->max_key, (unsigned long long)m);
+  if (threadIdx.x == 0) {
+    atomicMax((unsigned long long*)&ctl->max_key, (unsigned long long)m);
+    if (s_met) atomicAdd(&ctl->met, s_met);
+  }
   __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) s_last = atomicAdd(&ctl->blocks_done, 1u) == gridDim.x - 1;
@@ -591,12 +667,59 @@ __global__ void __launch_bounds__(512) k_seg_sample(const u64* __restrict__ keys
   __threadfence();
   for (int i = threadIdx.x; i < kSegLog; i += 512) s_h[i] = __ldcg(&ctl->hist[i]);
   __syncthreads();
-  seg_make_map<512>(s_h, __ldcg(&ctl->max_key), segs, ctl, s_w);
+  const u64 max_key = __ldcg(&ctl->max_key);
+  seg_make_map<512, false>(s_h, max_key, seg_reach(max_key, step), segs, false, ctl, s_w, nullptr);
+  if (threadIdx.x == 0) {
+    // a CTA's x table-fulls of keys leave 1 - (1 - e^-x) / x of a table for the average key to meet; of those a
+    // key that occurs g times equals g / n
+    const float sampled = (float)(n + 32ull * step - 1) / (float)step, x = sampled / gridDim.x / (float)kSegSeen;
+    const float seen = (float)kSegSeen * (1.0f - (1.0f - __expf(-x)) / x);
+    const float g = (float)__ldcg(&ctl->met) * (float)n / (sampled * seen);
+    if (__ldcg(&ctl->met) >= 8u && g > seg_dup_limit(n)) {
+      ctl->bail = 1;
+      ctl->max_seg = ~0u;
+    }
+  }
+}
+
+// All keys by piece where the sample was not even and thin (above 1.0e7 records: fewer than 340 sampled keys a
+// segment; 2^26 records: 50, and pieces of few segments then miss the capacity: products of small primes
+// 7.3 ms with the LSD sort behind it, 2.8 so).
+__global__ void __launch_bounds__(512) k_seg_pieces(const u64* __restrict__ keys, u64 n, u32 step, u32 segs, SegCtl* ctl) {
+  if (ctl->mode != kMapPieces || ctl->bail) return;    // uniform over the launch
+  __shared__ u32 s_h[kSegLog], s_w[16], s_last;
+  for (int i = threadIdx.x; i < kSegLog; i += 512) s_h[i] = 0;
+  __syncthreads();
+  constexpr int kU = 8;
+  for (u64 i0 = (u64)blockIdx.x * 512 * kU + threadIdx.x; i0 < n; i0 += (u64)gridDim.x * 512 * kU) {
+    u64 k[kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u) k[u] = i0 + u * 512 < n ? keys[i0 + u * 512] : 0ull;
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      if (i0 + u * 512 >= n) break;
+      u32 frac;
+      atomicAdd(&s_h[seg_piece(k[u], frac)], 1u);
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < kSegLog; i += 512)
+    if (s_h[i]) atomicAdd(&ctl->full[i], s_h[i]);
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(&ctl->pieces_done, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  for (int i = threadIdx.x; i < kSegLog; i += 512) s_h[i] = __ldcg(&ctl->full[i]);
+  __syncthreads();
+  seg_make_map<512, false>(s_h, ctl->max_key, seg_reach(ctl->max_key, step), segs, true, ctl, s_w, nullptr);
 }
 
 // Histograms of the one or two digits of f >> L: db low bits, then the rest.
 __global__ void __launch_bounds__(512)
 k_seg_hist(const u64* __restrict__ keys, u64 n, const SegCtl* __restrict__ ctl, u64* __restrict__ hist, int np, int db) {
+  if (ctl->bail) return;                               // uniform over the launch
   __shared__ u32 s_h[2 << 9];
   const int bins = np << db;
   const u32 mask = (1u << db) - 1u;
@@ -622,51 +745,44 @@ k_seg_hist(const u64* __restrict__ keys, u64 n, const SegCtl* __restrict__ ctl, 
 }
 
 // Up to kSegFrontMax records, one digit (segs <= 256): map, counts, offsets and starts in one CTA.
-__global__ void __launch_bounds__(1024)
+__global__ void __launch_bounds__(1024, 1)
 k_seg_front(const u64* __restrict__ keys, u32 n, u32 segs, SegCtl* __restrict__ ctl, u64* __restrict__ excl,
             u32* __restrict__ starts) {
   __shared__ u64 s_m[32];
-  __shared__ u32 s_l[kSegLog], s_h[256], s_w[32];
+  __shared__ u32 s_l[kSegLog + 1], s_h[256], s_w[32];
+  __shared__ SegScale s_sc;
   for (int i = threadIdx.x; i < kSegLog; i += 1024) s_l[i] = 0;
   if (threadIdx.x < 256) s_h[threadIdx.x] = 0;
   __syncthreads();
   u64 m = 0;
 #pragma unroll 4
-  for (u32 i = threadIdx.x; i < n; i += 4096) {        // a quarter of the keys
+  for (u32 i = 4 * (threadIdx.x & ~31u) + (threadIdx.x & 31u); i < n; i += 4096) {   // 32 of every 128 keys
     const u64 k = keys[i];
     m = k > m ? k : m;
     u32 frac;
     atomicAdd(&s_l[seg_piece(k, frac)], 1u);
   }
   m = block_max<1024>(m, s_m);
-  seg_make_map<1024>(s_l, m, segs, ctl, s_w);
-  __threadfence_block();
+  seg_make_map<1024, true>(s_l, m, m, segs, false, ctl, s_w, &s_sc);
   __syncthreads();
-  SegScale sc{};
-  sc.s = *(volatile u64*)&ctl->scale;
-  sc.top = *(volatile u32*)&ctl->top;
-  sc.linear = *(volatile u32*)&ctl->linear;
-  for (int i = threadIdx.x; i <= kSegLog; i += 1024) {   // the pieces' starts, in shared memory
-    const u32 v = *(volatile u32*)&ctl->cdf[i];
-    if (i < kSegLog) s_l[i] = v;
-  }
-  __syncthreads();
-  const u32 end = (segs << kSegBits);
+  const SegScale sc = s_sc;
+  bool differ = sc.mode == kMapEven;                   // even over 2^L NS values and more
+  if (differ) {
 #pragma unroll 8
-  for (u32 i = threadIdx.x; i < n; i += 1024) {
-    const u64 k = keys[i];
-    u32 f;
-    if (sc.linear) {
-      const u64 g = __umul64hi(k, sc.s);
-      f = g < sc.top ? (u32)g : sc.top;
-    } else {
+    for (u32 i = threadIdx.x; i < n; i += 1024) atomicAdd(&s_h[sc.even(keys[i]) >> kSegBits], 1u);
+  } else {
+    const u64 k0 = keys[0];
+#pragma unroll 4
+    for (u32 i = threadIdx.x; i < n; i += 1024) {
+      const u64 k = keys[i];
+      differ = differ || k != k0;
       u32 frac;
-      const u32 q = seg_piece(k, frac), c0 = s_l[q], c1 = q + 1 < (u32)kSegLog ? s_l[q + 1] : end;
-      f = min(c0 + (u32)(((u64)(c1 - c0) * frac) >> 20), sc.top);
+      const u32 q = seg_piece(k, frac), c0 = s_l[q], c1 = s_l[q + 1];   // as SegScale, from shared memory
+      const u32 f = sc.mode == kMapNarrow ? sc.narrow(k) : (u32)min((u64)c0 + (((u64)(c1 - c0) * frac) >> 26), (u64)sc.top);
+      atomicAdd(&s_h[f >> kSegBits], 1u);
     }
-    atomicAdd(&s_h[f >> kSegBits], 1u);
   }
-  __syncthreads();
+  const bool one_key = __syncthreads_or(differ) == 0;  // in order as it is: the pass copies it, no segment is sorted
   const int lane = threadIdx.x & 31;
   u32 v = 0, incl = 0;
   if (threadIdx.x < 256) {
@@ -677,15 +793,14 @@ k_seg_front(const u64* __restrict__ keys, u32 n, u32 segs, SegCtl* __restrict__ 
       if (lane >= o) incl += x;
     }
     if (lane == 31) s_w[threadIdx.x >> 5] = incl;
-    atomicMax(&ctl->max_seg, v);
+    if (!one_key) atomicMax(&ctl->max_seg, v);
   }
   __syncthreads();
   if (threadIdx.x < 256) {
     u32 add = 0;
     for (u32 w = 0; w < threadIdx.x >> 5; ++w) add += s_w[w];
     excl[threadIdx.x] = add + incl - v;
-    if (threadIdx.x <= segs) starts[threadIdx.x] = add + incl - v;
-    if (threadIdx.x == 255 && segs == 256) starts[256] = add + incl;
+    if (threadIdx.x <= segs) starts[threadIdx.x] = one_key ? 0u : add + incl - v;
   }
 }
 
@@ -696,6 +811,7 @@ constexpr int kBoundWarps = 8;                         // segments per CTA; one 
 __global__ void __launch_bounds__((kBoundWarps + 1) * 32)
 k_seg_bounds(const u64* __restrict__ keys, u32 n, u32 segs, SegCtl* __restrict__ ctl, u32* __restrict__ starts) {
   __shared__ u32 s_at[kBoundWarps + 1];
+  if (ctl->bail) return;                               // uniform over the launch
   const u32 wid = threadIdx.x >> 5, lane = threadIdx.x & 31, s = blockIdx.x * kBoundWarps + wid;
   const SegScale sc = seg_map(ctl);
   u32 lo = 0, hi = n;                                  // lower bound of segment s
@@ -767,7 +883,7 @@ k_seg_sort(const u64* kin, const u64* iin, u64* kout, u64* iout, u32 n, const Se
     __syncthreads();
     sc.s = s_m[0];
     sc.top = kSegBins - 1u;
-    sc.linear = 1;
+    sc.mode = kMapEven;
   }
   u32 bs[kSegItems];                                   // bin << 16 | slot in the bin
 #pragma unroll
@@ -1162,7 +1278,6 @@ extern "C" int cf_sort_pairs_to(const u64* kin, const u64* iin, u64* kout, u64* 
     return cf_cuda_status(cudaStreamSynchronize(st), "cf_sort_pairs_to");
   }
   const u64 *src_k = kin, *src_i = iin;
-  u32 max_seg = ~0u, herr = 0;
   if (n <= kSegMaxN) {
     const u32 segs = (u32)((n + kSegMean - 1) / kSegMean);
     const int np = segs <= 512 ? 1 : 2, db = segs <= 256 || (np == 2 && segs <= 65536) ? 8 : 9, bins = 1 << db;
@@ -1173,23 +1288,27 @@ extern "C" int cf_sort_pairs_to(const u64* kin, const u64* iin, u64* kout, u64* 
     const size_t side = (size_t)(n + (n & 1)) * 8;     // 16-byte aligned ids for the bulk copies
     u64* k2 = (u64*)w; w += side;
     u64* i2 = (u64*)w; w += side;
-    SegCtl* ctl = (SegCtl*)w; w += (sizeof(SegCtl) + 255) & ~(size_t)255;
+    // whole lines of 128 bytes for the status rows (7.6e6 records 359 us with rows across lines, 351)
+    SegCtl* ctl = (SegCtl*)(((uintptr_t)w + 255) & ~(uintptr_t)255);
+    w = (unsigned char*)ctl + ((sizeof(SegCtl) + 255) & ~(size_t)255);
+    unsigned char* zero = front ? (unsigned char*)&ctl->scale : (unsigned char*)ctl->full;
     u32* errw = &ctl->err;
     u64* hist = (u64*)w; w += (size_t)np * bins * 8;
     u32* status = (u32*)w; w += (size_t)np * tiles * bins * 4;
-    const size_t zeroed = (size_t)(w - (unsigned char*)ctl);
+    const size_t zeroed = (size_t)(w - zero);
     u64* excl = (u64*)(((uintptr_t)w + 7) & ~(uintptr_t)7); w = (unsigned char*)(excl + (size_t)np * bins);
     u32* starts = (u32*)w; w += (size_t)4 * segs + 4;
     if ((size_t)(w - (unsigned char*)tmp) > tmp_bytes) { cf_set_error("cf_sort_pairs_to: workspace too small%s", ""); return CF_ENOMEM; }
     e = db == 8 ? sort_pass_attrs<8, u32, true>() : sort_pass_attrs<9, u32, true>();
-    if (e == cudaSuccess) e = cudaMemsetAsync(ctl, 0, zeroed, st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(zero, 0, zeroed, st);
     if (e != cudaSuccess) return cf_cuda_status(e, "cf_sort_pairs_to: set-up");
     const unsigned g = (unsigned)((n + 4095) / 4096), gm = g < 148 * 4 ? g : 148 * 4;
     if (front) {
       k_seg_front<<<1, 1024, 0, st>>>(kin, (u32)n, segs, ctl, excl, starts);
     } else {
-      // 2^19 to 2^20 sampled keys, some fifty per segment at 2^26 records
-      k_seg_sample<<<gm < 148 ? gm : 148, 512, 0, st>>>(kin, n, (u32)(n >> 20) + 1, segs, ctl);
+      const u32 step = (u32)(n >> 20) + 1;             // 2^19 to 2^20 sampled keys
+      k_seg_sample<<<gm < 148 ? gm : 148, 512, 0, st>>>(kin, n, step, segs, ctl);
+      if (step > 10) k_seg_pieces<<<148 * 2, 512, 0, st>>>(kin, n, step, segs, ctl);
       k_seg_hist<<<gm, 512, 0, st>>>(kin, n, ctl, hist, np, db);
       k_sort_hist_scan<<<1, 32 * np, 0, st>>>(hist, excl, db);
     }
@@ -1209,17 +1328,18 @@ extern "C" int cf_sort_pairs_to(const u64* kin, const u64* iin, u64* kout, u64* 
     if (!front) k_seg_bounds<<<segs / kBoundWarps + 1, (kBoundWarps + 1) * 32, 0, st>>>(kout, (u32)n, segs, ctl, starts);
     k_seg_sort<<<segs, kSegBlock, kSegSmem, st>>>(kout, iout, kout, iout, (u32)n, ctl, starts);
     CF_LAUNCH_CHECK("cf_sort_pairs_to: segments");
-    u32 h[2];                                          // largest segment, error word
-    static_assert(offsetof(SegCtl, err) == offsetof(SegCtl, max_seg) + 4, "read together");
-    e = cudaMemcpyAsync(h, &ctl->max_seg, 8, cudaMemcpyDeviceToHost, st);
+    u32 h[3];                                          // largest segment, error word, no segments at all
+    static_assert(offsetof(SegCtl, err) == offsetof(SegCtl, max_seg) + 4 && offsetof(SegCtl, bail) == offsetof(SegCtl, err) + 4,
+                  "read together");
+    e = cudaMemcpyAsync(h, &ctl->max_seg, 12, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return cf_cuda_status(e, "cf_sort_pairs_to: control words");
-    max_seg = h[0];
-    herr = h[1];
-    if (herr & CF_ERR_SPIN_LIMIT) { cf_set_error("cf_sort_pairs_to: look-back wait exceeded its limit%s", ""); return CF_ETIMEOUT; }
-    if (max_seg <= (u32)kSegCap) return CF_OK;
-    src_k = kout;                                      // ordered by the top bits, equal keys in input order
-    src_i = iout;
+    if (h[1] & CF_ERR_SPIN_LIMIT) { cf_set_error("cf_sort_pairs_to: look-back wait exceeded its limit%s", ""); return CF_ETIMEOUT; }
+    if (!h[2] && h[0] <= (u32)kSegCap) return CF_OK;
+    if (!h[2]) {
+      src_k = kout;                                    // ordered by the top bits, equal keys in input order
+      src_i = iout;
+    }
   }
   if (src_k == kin) {
     e = cudaMemcpyAsync(kout, src_k, n * 8, cudaMemcpyDeviceToDevice, st);
