@@ -54,7 +54,11 @@ def _workspace(dev, name: str, nbytes: int):
     return t
 
 
-GEN_TAIL_MIN = 1 << 17        # records from which generate uses the pool's suffix table (a launch of 6 us to make)
+# Records from which generate uses the pool's suffix table, by radius: 2^17, 2^18 at r = 5, 2^22 at r = 4, never at
+# r = 3.  The table takes a launch of 6 us and some host time on a new pool; device time with it and with the walker,
+# us: r = 3, 1.0e7 records 70 / 70; r = 4, 2^20 22 / 27, 2^22 43 / 49, 1.0e7 78 / 100; r = 5, 2^17 19 / 29, 2^20 23 / 35;
+# r = 6, 2^17 33 / 59; r = 7, 2^17 37 / 61.
+GEN_TAIL_MIN = 1 << 17
 
 
 def generate(primes, r: int, M: int, mult: int = 1, bits: int = 10, lo: int = 0, hi=None, device=None):
@@ -77,9 +81,11 @@ def generate(primes, r: int, M: int, mult: int = 1, bits: int = 10, lo: int = 0,
         return keys, ids
     if M < 2:
         raise ValueError("M must be at least 2")
+    primes = tuple(map(int, primes))
     pool = _dtables(dev).pool(primes, r, M, mult)
     lib = _lib.load()
-    if r >= 3 and count >= GEN_TAIL_MIN and max(primes) < 1 << 31 and M % (1 << 33):
+    least = GEN_TAIL_MIN << {3: 40, 4: 5, 5: 1}.get(r, 0)
+    if r >= 3 and count >= least and max(primes) < 1 << 31 and M % (1 << 33):
         tail = _dtables(dev).tail(primes, r, M, mult, pool)
         _lib.check(lib.cf_gen_subsets_tail(_lib.ptr(pool), _lib.ptr(tail), n, r, lo, count, 0, bits, 1, _lib.ptr(keys),
                                            _lib.ptr(ids), None, _lib.stream_handle()), "generate")

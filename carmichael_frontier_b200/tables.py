@@ -92,6 +92,11 @@ class _PinnedRing:
         return True
 
 
+def _ints(primes) -> tuple:
+    """The primes as a tuple (a caller's tuple holds ints already)."""
+    return primes if type(primes) is tuple else tuple(map(int, primes))
+
+
 class DeviceTables:
     """Content-keyed cache of device copies of small host tables.
 
@@ -169,13 +174,13 @@ class DeviceTables:
         self._made.clear()
 
     def pool(self, primes, r: int, M: int, mult: int):
-        key = ("pool", tuple(int(p) for p in primes), r, M, int(mult) % M)
+        key = ("pool", _ints(primes), r, M, int(mult) % M)
         return self.get(key, lambda: pool_table_host(primes, r, M, mult))
 
     def tail(self, primes, r: int, M: int, mult: int, pool_dev):
         """Device tail table (b-subset products) of a pool, built on the device once."""
         import torch
-        key = ("tail", tuple(int(p) for p in primes), r, M, int(mult) % M)
+        key = ("tail", _ints(primes), r, M, int(mult) % M)
         t = self._cache.get(key)
         if t is not None:
             return self._use(key, t)
