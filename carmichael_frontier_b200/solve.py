@@ -114,14 +114,15 @@ class Tuning:
     part_lb: int = 10               # log2 buckets per range of the partitioned build (9 or 10)
     part_sigma: float = 8.0         # bucket-range capacity = mean + sigma*sqrt(mean) + 32
     class_join: bool = True         # fused: join by residue classes (csrc/cf_class.cu) where it applies
-    class_ws_bytes: int = 24 << 30  # ... and its workspace is at most this, half of it for each of a list's two
+    class_ws_bytes: int = 36 << 30  # ... and its workspace is at most this, a fifth of the device (half of it for each
+                                    # of a list's two)
     class_min_probe: int = 1 << 22  # ... and the probing side has this many records or more (see class_least)
 
 
 def class_least(r: int, n_build: int, tu: Tuning) -> int:
-    """Least probing side of a class join at radius r, n_build records on the other side.  Its lists and plan cost 0.13 ms whatever the sides; a
-    table probe costs more per record at larger radii.  Whole solves, class join against table join, ms:
-    r = 3, 6.5e6 records .227 / .203, 1.2e7 .228 / .236, 2.9e7 .266 / .337; r = 4, 4.2e6 .212 / .198, 8.2e6
+    """Least probing side of a class join at radius r, n_build records on the other side.  Its lists and plan cost
+    0.13 ms whatever the sides; a table probe costs more per record at larger radii.  Whole solves, class join
+    against table join, ms: r = 3, 6.5e6 records .227 / .203, 1.2e7 .228 / .236, 2.9e7 .266 / .337; r = 4, 4.2e6 .212 / .198, 8.2e6
     .220 / .213, 1.5e7 .243 / .278; r = 5, 4.2e6 .190 / .189 (nD = 1.4e5) and .247 / .289 (7.6e6), 2.4e7
     .290 / .451; r = 6, 4.5e6 .197 / .219; r = 7, 5.4e6 .189 / .288; r = 8, 5.9e6 .226 / .364.  A table of few
     records is probed at the same few sectors: r = 3, 4.5e6 against 1,140 records .194 / .245, against 10,000
