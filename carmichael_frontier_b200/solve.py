@@ -309,6 +309,7 @@ class Solver:
         self._bufset = 0                 # which of two buffer sets the next enqueue uses (solve_many)
         self.d2h_bytes = 0               # bytes read back from the device by collect()
         self._pinned: dict = {}
+        self._on: dict = {}              # buffer set -> raw stream of its last solve
         self._queued: dict = {}          # buffer set -> handle of the solve queued on it and not collected
         self._reserved: dict = {}        # buffer set -> bytes by name that lists have reserved
         self._class_cover = 0.0          # survivor estimate that the lists' class workspaces were reserved for
@@ -324,15 +325,13 @@ class Solver:
             if t is not None:                  # a growing buffer grows by half (64 MB at most) at least, the old one
                 nbytes = max(nbytes, min(t.numel() * 3 // 2, t.numel() + (64 << 20)))       # freed before it
                 del self._bufs[key], t
-            if self._pool is None:
+            st = self._torch_stream()
+            pool = self._pool or st
+            with self.torch.cuda.stream(pool):
                 t = self.torch.empty(max(nbytes, 16), dtype=self.torch.uint8, device=self.device)
-            else:
-                st = self._torch_stream()
-                with self.torch.cuda.stream(self._pool):
-                    t = self.torch.empty(max(nbytes, 16), dtype=self.torch.uint8, device=self.device)
-                if st != self._pool:
-                    st.wait_stream(self._pool)     # what used the memory before, on the caller's stream
-                    t.record_stream(st)
+            if st != pool:
+                st.wait_stream(pool)               # what used the memory before, on the caller's stream
+                t.record_stream(st)
             self._bufs[key] = t
         return t
 
@@ -396,6 +395,12 @@ class Solver:
         if plan.get("strategy", "fused") == "fused":
             self._leave_staging()
             self._queued[self._bufset] = True      # also when a launch below fails
+            sh = self._sh()
+            if self._on.get(self._bufset) != sh:   # buffers made for another stream: kept until this one has passed too
+                self._on[self._bufset] = sh
+                for (_name, k), t in self._bufs.items():
+                    if k == self._bufset:
+                        t.record_stream(self._torch_stream())
             pshape = self._part_shape(inst, plan)
             h = self._enqueue_solve(inst, plan, marks) if pshape is None \
                 else self._enqueue_fused(inst, plan, pshape, marks)
