@@ -287,21 +287,21 @@ def run_ours(args):
     from carmichael_frontier_b200 import Tuning
     solver = Solver(dev, tuning=Tuning(strategy=args.strategy))
     insts = [Instance.build(w.M, w.Q, w.B0, w.r, w.B) for w in seq]
-    # inputs resident in HBM for the device-timed region: pool tables uploaded before timing
+    # a fused solve prepares and uploads its tables inside the timed region; the forms that keep them by content
+    # (the partition strategy, the table build by ranges) find them resident
+    plans = [solver._direct_plan(x, None) for x in insts]
     solver.tables.max_entries = 10 ** 6
-    for inst in insts:
-        md = pow(inst.P0, -1, inst.M)
-        pd = solver.tables.pool(inst.B0, inst.r, inst.M, md)
-        pi = solver.tables.pool(inst.INS, inst.r, inst.M, 1)
-        solver.tables.tail(inst.B0, inst.r, inst.M, md, pd)
-        solver.tables.tail(inst.INS, inst.r, inst.M, 1, pi)
-        solver.tables.screen(inst.P0, inst.B, 1e-6)
+    for inst, plan in zip(insts, plans):
+        if plan and (plan["strategy"] != "fused" or solver._part_shape(inst, plan)):
+            solver._tables_for(inst)
     torch.cuda.synchronize(dev)
     clocks = ClockSampler(gpu_uuid(torch, dev))
     clocks.start()
-    # warm-up through the same pipelined call (both buffer sets allocated before timing)
+    # warm-up through the same pipelined call, and the two largest moduli: both buffer sets at their sizes
+    largest = sorted(range(len(insts)), key=lambda k: len(insts[k].INS))[-2:]
     solver.solve_many(insts[:args.warmup], verify=True)
-    # ---- device-timed region: K solves, inputs resident
+    solver.solve_many([insts[k] for k in largest], verify=True)
+    # ---- device-timed region: K solves
     stream = torch.cuda.current_stream(dev)
     import collections
     kt = collections.defaultdict(float)
@@ -352,7 +352,7 @@ def run_ours(args):
 
     _default_solvers.clear()
     if timed:                                # one untimed call: the public solver's device buffers
-        public_solve_many(timed[:2], device=dev, strategy=args.strategy)
+        public_solve_many([seq[k] for k in largest], device=dev, strategy=args.strategy)
     s = public_solver()
     barrier()
     torch.cuda.synchronize(dev)
@@ -395,7 +395,7 @@ def run_ours(args):
     t_path = kt["gen_D"] + kt["gen_I"] + kt["join"] + kt["probe"]
     achieved = BYTES_PER_RECORD * recs / t_path / 1e9 if t_path > 0 else None
     traffic = None     # DRAM bytes per step of the join-path kernels, scaled from the committed ncu capture
-    by_class = args.strategy == "fused" and bool((solver._direct_plan(timed[0], None) or {}).get("class_plan"))
+    by_class = args.strategy == "fused" and bool((plans[-1] or {}).get("class_plan"))
     tname = "profiles/k_cj_k64_r5.md" if by_class else "profiles/k_fused_k64_r5_seed0.md"
     tfile = os.path.join(ROOT, tname)
     if args.strategy == "fused" and os.path.exists(tfile):
@@ -410,6 +410,18 @@ def run_ours(args):
             traffic = (per["traffic_bytes_per_I_record"] * n_i_all
                        + per.get("traffic_bytes_per_D_record", 0.0) * n_d_all) / len(timed)
 
+    if by_class:       # no record is written: the probe is bound by integer issue, 12 instructions per tested record
+        n_test = sum(max(math.comb(len(w.B0), w.r), math.comb(len(w.INS), w.r)) for w in timed)
+        peak = 148 * 128 * (clk["sm_mhz"] or 1965.0) * 1e6 / 1e12
+        achieved = 12 * n_test / kt["probe"] / 1e12 if kt["probe"] > 0 else None
+        bound = {"bound": "integer issue", "achieved": achieved, "peak": peak, "unit": "T instructions/s (lanes)",
+                 "frac": achieved / peak if achieved else None, "kernel": "k_cj_probe with k_cj_resolve and k_cj_emit",
+                 "peak_source": "148 SMs x 128 lanes at the sampled clock"}
+    else:
+        bound = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
+                 "frac": (achieved / peak) if achieved else None,
+                 "kernel": ("k_fused build + probe" if solver.tuning.strategy == "fused" else "k_gen_part + k_join_part")
+                           + " (join path, 32 B/record)", "peak_source": peak_src}
     cpu = None
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
         try:
@@ -457,18 +469,10 @@ def run_ours(args):
             "config": {"workload": WORKLOAD, "r": 5, "k": 64, "B": "10^148", "moduli_per_step_per_gpu": 1,
                        "seeds": [w.name for w in timed][:8], "l2": "inputs larger than L2 (I side 0.17-11 GB per step)",
                        "parallelism": f"modulus-sharded x{world}", "records_per_gpu": recs},
-            "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                         "frac": (achieved / peak) if achieved else None, "traffic": traffic,
+            "roofline": {**bound, "traffic": traffic,
                          "traffic_source": ("ncu dram__bytes_read.sum + dram__bytes_write.sum per D and per I record "
                                             f"of one capture ({tname}), scaled by this "
-                                            "run's record counts" if traffic is not None else None),
-                         "kernel": ("k_cj lists, build, probe, resolve" if by_class else "k_fused build + probe"
-                                    if solver.tuning.strategy == "fused" else "k_gen_part + k_join_part")
-                                   + " (join path, 32 B/record)",
-                         "note": ("the materialised join's 32 B per record over the join time; the class join writes "
-                                  "no record (traffic: its DRAM bytes) and is bound by integer issue"
-                                  if by_class else None),
-                         "peak_source": peak_src},
+                                            "run's record counts" if traffic is not None else None)},
             "strategy": solver.tuning.strategy,
             "kernels": kern,
             "kernels_source": ("CUDA events around each kernel in a second pass over the timed solves on one "
@@ -537,14 +541,6 @@ def measure_portfolio(dev, args, compact: bool = False) -> dict:
     torch.cuda.synchronize(dev)
     t_p = time.perf_counter() - t0
     npl = len(insts) if compact else min(args.plain_moduli, len(insts))
-    # the plain form's sort: radix digit width per size class of its sides, by the autotuner
-    from carmichael_frontier_b200 import autotune, mitm_gpu2
-    sides = [n for k in range(npl) for n in (prep.nD[k], min(prep.nI[k], 1 << 27))]
-    key_bits = max(x.M.bit_length() for x in insts[:npl])
-    t0 = time.perf_counter()
-    autotune.tune_sort(sides, key_bits=key_bits, device=dev, reps=2)
-    t_tune = time.perf_counter() - t0
-    digit_bits = {n.bit_length(): mitm_gpu2.sort_digit_bits(n) for n in sides if n > 1}
     run_plain(insts[:1], i_limit=1 << 16, device=dev)
     torch.cuda.synchronize(dev)
     t0 = time.perf_counter()
@@ -574,9 +570,7 @@ def measure_portfolio(dev, args, compact: bool = False) -> dict:
         "per_modulus_fused": {"moduli_per_s": len(insts) / t_p, "records_per_s": recs / t_p, "s": t_p,
                               "same_results": same},
         "plain_mitm_gpu2": {"moduli": npl, "moduli_per_s": npl / t_pl, "records_per_s": rec_pl / t_pl, "s": t_pl,
-                            "same_results": same_plain,
-                            "sort_digit_bits": {f"2^{c - 1}..2^{c}": b for c, b in sorted(digit_bits.items())},
-                            "sort_key_bits": key_bits, "sort_tune_s": t_tune},
+                            "same_results": same_plain},
         "batched_over_plain": (len(insts) / t_b) / (npl / t_pl),
         "mitm64_all_cores": cpu,
         "batched_over_mitm64": ((recs / t_b) / cpu["records_per_s"]) if cpu and cpu.get("records_per_s") else None,
