@@ -22,10 +22,10 @@
 //           in x; child x is kept iff A <= H[t][x]  (t = positions left after x)
 //   D side: G[t][x] = ceil(Dmin / (b_x b_{x-1} ... b_{x-t})), non-increasing in
 //           x; child x is kept iff A >= G[t][x]
-// so a level is: count children per node (k_bgen_count), exclusive scan
-// (cf_scan_u64), and write one child per thread (k_bgen_expand), which finds
-// its parent by binary search over the scanned offsets -- every thread does the
-// same work whatever the shape of the tree.  The last level writes the records
+// so a level is: count the children per node and scan the counts (k_bgen_count_scan, blocks of 1,024
+// nodes; block sums scanned and added in further launches), and write a tile of children per CTA
+// (k_bgen_expand), whose parents' offsets are searched by each child in shared memory -- every thread does
+// the same work whatever the shape of the tree.  The last level writes the records
 // (canonical keys) directly, in the reference's order.  The product never
 // overflows: on the I side the host checks that Icap - 1 < 2^128 (A * a_x <= Icap - 1 for every kept
 // child) or, for larger caps (the table then saturates at 2^128 - 1), that r - 1 primes multiply below 2^128;

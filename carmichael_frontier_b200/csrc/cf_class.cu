@@ -571,7 +571,7 @@ __device__ __forceinline__ void cj_probe_range(const CjArgs& a, const u32* s_bm,
 }
 
 // Bound by integer issue: k = 64, r = 5, 5.9e8 I records in 0.60 ms (9.8e11 records/s; the fused
-// probe 3.2 ms), issue slots 68% busy, ALU pipe 62%, the multiplier pipe 57%, shared memory 60%; 24
+// probe 3.2 ms), issue slots 68% busy, ALU pipe 62%, the multiplier pipe 57%, shared memory 55%; 24
 // instructions per 32 records, of which 12 test, the rest survivors, prefixes past their suffix (10 to
 // 30%) and the block set-up.  Survivors wait in a ring per warp until 32 can be looked up at once
 // (pushed as found, with their V from registers: 0.64 ms).  32 warps of 64 registers: more registers

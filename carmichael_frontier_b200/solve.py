@@ -402,7 +402,7 @@ class Solver:
                     if k == self._bufset:
                         t.record_stream(self._torch_stream())
             pshape = self._part_shape(inst, plan)
-            h = self._enqueue_solve(inst, plan, marks) if pshape is None \
+            h = self._enqueue_solve(inst, plan, marks, sh) if pshape is None \
                 else self._enqueue_fused(inst, plan, pshape, marks)
             h["set"] = self._bufset
             self._queued[self._bufset] = h
@@ -433,7 +433,7 @@ class Solver:
         return part_shape(nIt if plan.get("swap") and nIt < nD else nD, plan["bbits"], tu.part_lb, tu.part_sigma,
                           lib.cf_batch_part_max_ranges())
 
-    def _enqueue_solve(self, inst: Instance, plan: dict, marks: list | None):
+    def _enqueue_solve(self, inst: Instance, plan: dict, marks: list | None, sh: int):
         """Class join, or table build in place and generate-and-probe, with tables, check and
         read-back: one cf_solve call.  Table by table from Python, k = 29, r = 2 took 235 us a
         solve against 184, and 24 portfolio moduli (11.0 ms against 8.3)"""
@@ -456,7 +456,6 @@ class Solver:
         # L2-resident while built); larger tables the wide entries
         q.side_format = 1 if q.bbits <= 20 else 0
         tb = lib.cf_solve_table_bytes(len(pD), len(pI), r)
-        sh = self._sh()
         tabs = self._buf("tables", tb)
         stage = self._pinned_buf("stage", tb, tabs, sh)
         if cp:
