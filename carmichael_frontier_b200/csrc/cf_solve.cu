@@ -79,6 +79,10 @@ extern "C" int cf_solve(const CfSolve* s, void* stream) {
     cf_set_error("cf_solve: bad arguments%s", "");
     return CF_EBADARG;
   }
+  if (s->class_plan && ((s->primesD[s->nD - 1] | s->primesI[s->nI - 1]) >> 31)) {   // 32-bit factors in its kernels
+    cf_set_error("cf_solve: the class join takes primes below 2^31%s", "");
+    return CF_EBADARG;
+  }
   const cudaStream_t st = (cudaStream_t)stream;
   const int r = s->r;
   const size_t bD = up256(cf_pool_bytes(s->nD, r)), bI = up256(cf_pool_bytes(s->nI, r));

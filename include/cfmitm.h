@@ -213,7 +213,7 @@ int cf_fused_probe(const void* pool_dev, const void* tail, int n, int r, uint64_
  * first fields are {u64 magic; u32 ok, d, mp, phi; u64 ws_bytes}, and ok = 0 means that the class
  * join does not apply to this instance (join it with the fused probe).  cf_class_join runs it:
  * poolD / poolI are device pool tables (D with a multiplier whose residues mod plan.mp and plan.d
- * are multD_m and multD_d, I with multiplier 1), ws is plan.ws_bytes of 256-byte aligned device
+ * are multD_m and multD_d, I with multiplier 1; every prime below 2^31), ws is plan.ws_bytes of 256-byte aligned device
  * memory, pairs / npairs / err as for cf_fused_probe; CF_ERR_PART_OVERFLOW in *err: a survivor
  * list ran out, join the instance with the fused probe instead.  ev_built: null, or a CUDA event
  * recorded between the filter build and the probe. */

@@ -108,3 +108,22 @@ def test_portfolio_batches_small_probing_sides_where_there_is_a_batch(monkeypatc
         with pytest.raises(Split):
             b.prepare(xs)
         assert len(seen) == 2 * batched
+
+
+def test_cf_solve_refuses_a_class_plan_for_primes_of_2_31_or_more():
+    # refused before anything is prepared or queued: the device addresses are never used
+    import ctypes as C
+    lib = _lib.load()
+    x = instance(64, 150, 4)
+    cp = class_plan(x)
+    for big in ("D", "I"):
+        pD, pI = np.array(x.B0, dtype=np.uint64), np.array(x.INS, dtype=np.uint64)
+        (pD if big == "D" else pI)[-1] = (1 << 31) + 11
+        lb = np.ones(1, dtype=np.uint32)
+        stage = np.zeros(lib.cf_solve_table_bytes(64, 150, 4), dtype=np.uint8)
+        q = _lib.CfSolve(primesD=pD.ctypes.data, primesI=pI.ctypes.data, m=M // (M & -M), multD_odd=1, multD_2=1, n_D=1,
+                         n_I=1, limbsB=lb.ctypes.data, nlimbs=1, lgP0=1.0, lgB=1.0, eps=1e-6, nD=64, nI=150, r=4,
+                         a=6, class_plan=C.cast(C.c_char_p(cp), C.c_void_p), stage=stage.ctypes.data, tables=256, ws=256,
+                         ws_bytes=1 << 62, misc=256)
+        assert lib.cf_solve(C.byref(q), None) == _lib.CF_EBADARG
+        assert b"2^31" in lib.cf_last_error_string() and not stage.any()

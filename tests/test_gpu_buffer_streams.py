@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 
 def busy(torch, stream):
     with torch.cuda.stream(stream):
-        torch.cuda._sleep(200_000_000)             # a tenth of a second
+        torch.cuda._sleep(600_000_000)             # a third of a second
         ev = torch.cuda.Event()
         ev.record(stream)
     return ev

@@ -22,9 +22,9 @@ def summary(r):
 
 
 def busy(torch, stream):
-    """Hold the stream for a tenth of a second; an event after it."""
+    """Hold the stream for a third of a second; an event after it."""
     with torch.cuda.stream(stream):
-        torch.cuda._sleep(200_000_000)
+        torch.cuda._sleep(600_000_000)
         ev = torch.cuda.Event()
         ev.record(stream)
     return ev
