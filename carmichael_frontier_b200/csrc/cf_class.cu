@@ -1013,6 +1013,15 @@ extern "C" int cf_class_plan(u64 m, int nD, int nI, int r, u64 i_lo, u64 i_n, in
   return CF_ENOMEM;
 }
 
+// Whether a plan was made for these sides, this window and a modulus with odd part m.
+bool cf_class_plan_fits(const void* plan, u64 m, int nD, int nI, int r, u64 i_lo, u64 i_n, int swap) {
+  const CfClassPlan* P = (const CfClassPlan*)plan;
+  if (P->magic != kCjMagic || !P->ok || P->r != (u32)r || P->swap != (u32)(swap != 0) || P->i_lo != i_lo || P->i_n != i_n)
+    return false;
+  return P->side[P->swap ? 1 : 0].n == (u32)nD && P->side[P->swap ? 0 : 1].n == (u32)nI && P->mp && P->d && m % P->mp == 0 &&
+         m % P->d == 0;
+}
+
 // Run a planned class join on the stream: equal-residue pairs {D rank, I rank} are appended through
 // *npairs (zeroed by the caller).  poolD, poolI: device pool tables (cf_pool_prepare) of the two
 // sides, D with the multiplier whose residues mod plan->mp and plan->d are multD_m and multD_d, I

@@ -23,6 +23,7 @@ extern "C" int cf_fused_probe3(const void* pool_dev, const void* tail, int n, in
 extern "C" int cf_class_join(const void* plan, const void* poolD, const void* poolI, u32 multD_m, u32 multD_d,
                              void* ws, size_t ws_bytes, void* pairs, u32 max_pairs, u32* npairs, u32* err,
                              void* ev_built, void* stream);
+bool cf_class_plan_fits(const void* plan, u64 m, int nD, int nI, int r, u64 i_lo, u64 i_n, int swap);
 extern "C" size_t cf_pair_result_bytes(void);
 extern "C" int cf_check_pairs(const void* poolD, const void* poolI, const void* screen, int r, const void* pairs,
                               const u32* npairs, u32 max_pairs, void* results, u32* err, void* stream);
@@ -77,6 +78,11 @@ extern "C" int cf_solve(const CfSolve* s, void* stream) {
       (!s->class_plan && (s->tails_bytes < cf_solve_tail_bytes(s->nD, s->nI, s->r) ||
                           s->ws_bytes < cf_dtab_bytes2(s->bbits, s->fbits) || !cf_dtab_bytes2(s->bbits, s->fbits)))) {
     cf_set_error("cf_solve: bad arguments%s", "");
+    return CF_EBADARG;
+  }
+  // a plan of other sides would index the pools past their ends
+  if (s->class_plan && !cf_class_plan_fits(s->class_plan, s->m, s->nD, s->nI, s->r, s->i_lo, s->n_I, s->swap)) {
+    cf_set_error("cf_solve: the class plan is of another instance or window%s", "");
     return CF_EBADARG;
   }
   if (s->class_plan && ((s->primesD[s->nD - 1] | s->primesI[s->nI - 1]) >> 31)) {   // 32-bit factors in its kernels

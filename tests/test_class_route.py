@@ -110,20 +110,51 @@ def test_portfolio_batches_small_probing_sides_where_there_is_a_batch(monkeypatc
         assert len(seen) == 2 * batched
 
 
-def test_cf_solve_refuses_a_class_plan_for_primes_of_2_31_or_more():
-    # refused before anything is prepared or queued: the device addresses are never used
+def solve_status(x, cp, pD=None, pI=None, **other):
+    """(status, error text) of cf_solve with a class plan.  The device addresses are never used by a call that
+    is refused."""
     import ctypes as C
     lib = _lib.load()
+    pD = np.array(x.B0, dtype=np.uint64) if pD is None else pD
+    pI = np.array(x.INS, dtype=np.uint64) if pI is None else pI
+    lb = np.ones(1, dtype=np.uint32)
+    stage = np.zeros(lib.cf_solve_table_bytes(len(pD), len(pI), x.r), dtype=np.uint8)
+    args = dict(primesD=pD.ctypes.data, primesI=pI.ctypes.data, m=M // (M & -M), multD_odd=1, multD_2=1, n_D=1,
+                n_I=math.comb(len(pI), x.r), limbsB=lb.ctypes.data, nlimbs=1, lgP0=1.0, lgB=1.0, eps=1e-6, nD=len(pD),
+                nI=len(pI), r=x.r, a=6, class_plan=C.cast(C.c_char_p(cp), C.c_void_p), stage=stage.ctypes.data, tables=256,
+                ws=256, ws_bytes=1 << 62, misc=256)
+    rc = lib.cf_solve(C.byref(_lib.CfSolve(**{**args, **other})), None)
+    assert not stage.any()
+    return rc, lib.cf_last_error_string()
+
+
+def test_cf_solve_refuses_a_class_plan_for_primes_of_2_31_or_more():
     x = instance(64, 150, 4)
-    cp = class_plan(x)
-    for big in ("D", "I"):
-        pD, pI = np.array(x.B0, dtype=np.uint64), np.array(x.INS, dtype=np.uint64)
-        (pD if big == "D" else pI)[-1] = (1 << 31) + 11
-        lb = np.ones(1, dtype=np.uint32)
-        stage = np.zeros(lib.cf_solve_table_bytes(64, 150, 4), dtype=np.uint8)
-        q = _lib.CfSolve(primesD=pD.ctypes.data, primesI=pI.ctypes.data, m=M // (M & -M), multD_odd=1, multD_2=1, n_D=1,
-                         n_I=1, limbsB=lb.ctypes.data, nlimbs=1, lgP0=1.0, lgB=1.0, eps=1e-6, nD=64, nI=150, r=4,
-                         a=6, class_plan=C.cast(C.c_char_p(cp), C.c_void_p), stage=stage.ctypes.data, tables=256, ws=256,
-                         ws_bytes=1 << 62, misc=256)
-        assert lib.cf_solve(C.byref(q), None) == _lib.CF_EBADARG
-        assert b"2^31" in lib.cf_last_error_string() and not stage.any()
+    for big in (0, 1):
+        sides = [np.array(x.B0, dtype=np.uint64), np.array(x.INS, dtype=np.uint64)]
+        sides[big][-1] = (1 << 31) + 11
+        rc, text = solve_status(x, class_plan(x), *sides)
+        assert rc == _lib.CF_EBADARG and b"2^31" in text
+
+
+@pytest.mark.parametrize("what", ["smaller I pool", "larger D pool", "radius", "window", "start", "swap", "modulus"])
+def test_cf_solve_refuses_the_plan_of_another_instance(what):
+    x = instance(64, 150, 4)
+    cp, y, other = class_plan(x), x, {}
+    if what == "smaller I pool":
+        y = instance(64, 149, 4)
+        other = dict(n_I=math.comb(150, 4))
+    elif what == "larger D pool":
+        y = instance(65, 150, 4)
+    elif what == "radius":
+        other = dict(r=5)
+    elif what == "window":
+        other = dict(n_I=math.comb(150, 4) - 1)
+    elif what == "start":
+        other = dict(i_lo=1)
+    elif what == "swap":
+        other = dict(swap=1)
+    else:
+        other = dict(m=3 ** 3 * 5 ** 2 * 7 * 11 * 13 * 17 * 31)      # without divisors of the plan
+    rc, text = solve_status(y, cp, **other)
+    assert rc == _lib.CF_EBADARG and b"another instance" in text
