@@ -62,12 +62,13 @@ def sort(cuda, k, i):
 @pytest.mark.parametrize("kind,n,held", [
     ("narrow1000", 20_003, True), ("narrow1048576", 1 << 20, True), ("narrow1048576", 7_624_512, True),
     ("narrow16777216", (1 << 24) + 7, True), ("narrow5000000", 4_000_001, True), ("narrow65536", 65_537, True),
-    ("ascending", 20_003, True), ("ascending", 1 << 22, True), ("ascending", 20_000_003, True), ("ascending runs", 1 << 24, True), ("pairs", 5_000_001, True),
+    ("ascending", 20_003, True), ("ascending", 1 << 22, True), ("ascending", 20_000_003, True),
+    ("ascending runs", 1 << 24, True), ("pairs", 5_000_001, True),
     ("products", 7_624_512, True), ("products", 30_000_001, True), ("cut", 1 << 20, True), ("cut", 20_000_001, False),
     ("smooth cut", 1 << 20, True), ("smooth cut", 7_624_512, True), ("smooth cut", 20_000_001, True),
     ("cut", 65_000, True), ("few1000", 1 << 20, False), ("few1000", 7_624_512, False), ("few70000", 7_624_512, False),
-    ("few100", 65_537, True), ("few2000000", 7_624_512, True), ("few400000", 7_624_512, False), ("few3", 20_003, False), ("one", 20_003, True),
-    ("one", 65_536, True), ("one", 65_537, False), ("one", 3_000_000, False)])
+    ("few100", 65_537, True), ("few2000000", 7_624_512, True), ("few400000", 7_624_512, False),
+    ("few3", 20_003, False), ("one", 20_003, True), ("one", 65_536, True), ("one", 65_537, False), ("one", 3_000_000, False)])
 def test_sort_and_its_route(cuda, kind, n, held):
     rng = np.random.default_rng(n)
     k = keys_of(kind, n, rng)
